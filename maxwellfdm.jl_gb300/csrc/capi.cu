@@ -412,14 +412,15 @@ int fdfd_create(const fdfd_desc *d, fdfd_handle **out) {
   const cd w2 = om * om;
   h->w2[0] = w2.real();
   h->w2[1] = w2.imag();
-  // per-axis coefficients, 6 kinds: cm, ce, wm, wp, s∆lₑ, s∆lₘ
+  // per-axis coefficients, 8 kinds: cm, ce, wm, wp, s∆lₑ, s∆lₘ, and the
+  // forward-mean weights of H at its own and at the next index
   const int st = h->N[0] + h->N[1] + h->N[2];
   h->coef_stride = st;
   h->coef_off[0] = 0;
   h->coef_off[1] = h->N[0];
   h->coef_off[2] = h->N[0] + h->N[1];
-  std::vector<double2> c64(6 * (size_t)st);
-  std::vector<float2> c32(6 * (size_t)st);
+  std::vector<double2> c64(8 * (size_t)st);
+  std::vector<float2> c32(8 * (size_t)st);
   for (int w = 0; w < 3; ++w) {
     const int N = h->N[w];
     for (int i = 0; i < N; ++i) {
@@ -431,8 +432,15 @@ int fdfd_create(const fdfd_desc *d, fdfd_handle **out) {
       }
       const int jm = i > 0 ? i - 1 : (h->bloch[w] ? N - 1 : 0);
       const cd smm(d->sdl_m[w][2 * jm], d->sdl_m[w][2 * jm + 1]);
-      const cd vals[6] = {1.0 / sm, 1.0 / se, smm / (2.0 * se), sm / (2.0 * se), se, sm};
-      for (int kd = 0; kd < 6; ++kd) {
+      // the next s∆lₑ; past the end of a symmetry axis H is 0 and takes no weight
+      cd sen(0.0, 0.0);
+      if (i + 1 < N || h->bloch[w]) {
+        const int jp = i + 1 < N ? i + 1 : 0;
+        sen = cd(d->sdl_e[w][2 * jp], d->sdl_e[w][2 * jp + 1]);
+      }
+      const cd vals[8] = {1.0 / sm,        1.0 / se, smm / (2.0 * se), sm / (2.0 * se), se, sm,
+                          se / (2.0 * sm), sen / (2.0 * sm)};
+      for (int kd = 0; kd < 8; ++kd) {
         const size_t idx = (size_t)kd * st + h->coef_off[w] + i;
         c64[idx] = make_double2(vals[kd].real(), vals[kd].imag());
         c32[idx] = make_float2((float)vals[kd].real(), (float)vals[kd].imag());

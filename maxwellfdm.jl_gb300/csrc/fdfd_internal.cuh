@@ -123,7 +123,7 @@ struct fdfd_handle {
   double omega[2] = {0, 0};
   double w2[2] = {0, 0};
   double e_ikl[3][2];
-  // per-axis coefficients: [kind(4)][axis(3)] contiguous, kind = cm, ce, wm, wp
+  // per-axis coefficients: [kind(8)][axis(3)] contiguous, kind = cm, ce, wm, wp, s∆lₑ, s∆lₘ, H mean own, next
   double2 *coef64 = nullptr;
   float2 *coef32 = nullptr;
   long long coef_off[3] = {0, 0, 0};

@@ -16,38 +16,165 @@
 //     H_w[N] = 0 there (normal H on the PEC plane); Bloch axes wrap with the
 //     phase e^{∓ikL}.  These are the same two-point means the ε tensor's
 //     off-diagonal averaging uses.
-// All kernels are grid-stride loops over cells, x fastest (coalesced).
 #include <cuda_runtime.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "operator_common.cuh"
 
 namespace fdfd {
 
-__global__ void k_h_from_e(OpArgs<double> a, Extra<double> ex, const double2 *__restrict__ e,
-                           const double2 *__restrict__ jm, double2 *__restrict__ hout, double2 iow) {
-  const long long nc = a.ncell;
-  for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < nc;
-       cell += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(cell % a.N[0]), j = (int)((cell / a.N[0]) % a.N[1]), k = (int)(cell / ((long long)a.N[0] * a.N[1]));
-    const double2 cmx = a.cm[0][i], cmy = a.cm[1][j], cmz = a.cm[2][k];
-    const double2 ex0 = load_e<double, false>(e, a, ex, i, j, k, 0);
-    const double2 ey0 = load_e<double, false>(e, a, ex, i, j, k, 1);
-    const double2 ez0 = load_e<double, false>(e, a, ex, i, j, k, 2);
-    const double2 exy = load_e<double, false>(e, a, ex, i, j + 1, k, 0);
-    const double2 exz = load_e<double, false>(e, a, ex, i, j, k + 1, 0);
-    const double2 eyx = load_e<double, false>(e, a, ex, i + 1, j, k, 1);
-    const double2 eyz = load_e<double, false>(e, a, ex, i, j, k + 1, 1);
-    const double2 ezx = load_e<double, false>(e, a, ex, i + 1, j, k, 2);
-    const double2 ezy = load_e<double, false>(e, a, ex, i, j + 1, k, 2);
-    double2 h[3];
-    h[0] = csub(cmul(cmy, csub(ezy, ez0)), cmul(cmz, csub(eyz, ey0)));
-    h[1] = csub(cmul(cmz, csub(exz, ex0)), cmul(cmx, csub(ezx, ez0)));
-    h[2] = csub(cmul(cmx, csub(eyx, ey0)), cmul(cmy, csub(exy, ex0)));
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if (jm) h[c] = cadd(h[c], jm[3 * cell + c]);
-      hout[3 * cell + c] = cmul(iow, h[c]);
+// The two kernels below are bound by the FP64 pipe (measured 0.53·10¹² lane
+// FMAs/s on the chip: a warp's FP64 instruction holds its scheduler's pipe
+// for 64 cycles however few lanes are active), so they are laid out to issue
+// few FP64 instructions:
+//   * threads run over the flattened cells of an x-y plane, so ragged Nx
+//     leaves no idle lanes, and march along z keeping what the next plane
+//     needs in registers;
+//   * a coefficient that is real for the whole warp (outside that axis' PML)
+//     multiplies as a real number, axis by axis.
+// 128×128×64, cold: k_h_from_e 192 → 84 µs, each k_corner_mean 271 → 43 µs
+// (HBM alone would take 22 and 15 µs; the FP64 pipe is busy 75-78 % of the
+// launch).
+constexpr int FB = 256;
+
+// acc ± c·d and c·d, with a real c when RC
+template <bool NEG, bool RC>
+__device__ __forceinline__ void axpy_c(double2 &acc, double2 c, double2 d) {
+  const double cx = NEG ? -c.x : c.x;
+  acc.x = fma(cx, d.x, acc.x);
+  acc.y = fma(cx, d.y, acc.y);
+  if (!RC) {
+    const double cy = NEG ? -c.y : c.y;
+    acc.x = fma(-cy, d.y, acc.x);
+    acc.y = fma(cy, d.x, acc.y);
+  }
+}
+template <bool RC>
+__device__ __forceinline__ double2 mul_c(double2 c, double2 d) {
+  double2 r = mk(c.x * d.x, c.x * d.y);
+  if (!RC) {
+    r.x = fma(-c.y, d.y, r.x);
+    r.y = fma(c.y, d.x, r.y);
+  }
+  return r;
+}
+
+// f(XR, YR, ZR) for three warp-uniform flags as compile-time constants: one
+// branch to a body that holds only the FP64 instructions it needs (branches
+// inside the body become predicated instructions, which take the pipe too:
+// 131 µs against 84 for k_h_from_e at 128×128×64).
+template <typename F>
+__device__ __forceinline__ void by_axis(bool xr, bool yr, bool zr, F f) {
+  using T = std::true_type;
+  using N = std::false_type;
+  if (xr) {
+    if (yr) {
+      if (zr) f(T{}, T{}, T{});
+      else f(T{}, T{}, N{});
+    } else {
+      if (zr) f(T{}, N{}, T{});
+      else f(T{}, N{}, N{});
     }
+  } else {
+    if (yr) {
+      if (zr) f(N{}, T{}, T{});
+      else f(N{}, T{}, N{});
+    } else {
+      if (zr) f(N{}, N{}, T{});
+      else f(N{}, N{}, N{});
+    }
+  }
+}
+
+// REALW: ω is real, so i/ω = i·s and s is folded into the curl coefficients.
+// BL: some axis is periodic.
+template <bool REALW, bool BL>
+__global__ void __launch_bounds__(FB) k_h_from_e(OpArgs<double> a, Extra<double> ex, const double2 *__restrict__ e,
+                                                 const double2 *__restrict__ jm, double2 *__restrict__ hout,
+                                                 double2 iow, int kc) {
+  const int plane = a.N[0] * a.N[1];
+  const int p0 = blockIdx.x * FB + threadIdx.x;
+  const bool act = p0 < plane;
+  const int p = act ? p0 : plane - 1;  // idle lanes of the last warp repeat a cell (and store nothing)
+  const int i = p % a.N[0], j = p / a.N[0];
+  const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, a.N[2]);
+  const bool blx = BL && a.bloch[0], bly = BL && a.bloch[1], blz = BL && a.bloch[2];
+  const bool pi = !blx && i == 0, pj = !bly && j == 0;
+  const double sc = REALW ? iow.y : 1.0;
+  const double2 cx = cscale(a.cm[0][i], sc), cy = cscale(a.cm[1][j], sc);
+  const bool xr = __all_sync(0xffffffffu, cx.y == 0.0), yr = __all_sync(0xffffffffu, cy.y == 0.0);
+  // the +x and +y neighbours: offset in cells, factor (1, or the Bloch phase), present or a PEC ghost
+  const bool xin = i + 1 < a.N[0], yin = j + 1 < a.N[1];
+  const bool xok = xin || blx, yok = yin || bly;
+  const long long dx = xin ? 1 : 1 - a.N[0], dy = yin ? a.N[0] : a.N[0] - plane;
+  const double2 zero = czero<double2>();
+  const double2 *c0 = e + 3 * ((long long)plane * k0 + p);
+  double2 v0 = c0[0], v1 = c0[1], v2 = c0[2];
+  for (int k = k0; k < k1; ++k) {
+    const long long cell = (long long)plane * k + p;
+    const double2 *ec = e + 3 * cell;
+    const bool z0 = !blz && k == 0;
+    double2 n0 = zero, n1 = zero, n2 = zero;
+    if (k + 1 < a.N[2]) {
+      const double2 *en = ec + 3ll * plane;
+      n0 = en[0];
+      n1 = en[1];
+      n2 = en[2];
+    } else if (blz) {
+      n0 = cmul(e[3ll * p], ex.ph[2]);
+      n1 = cmul(e[3ll * p + 1], ex.ph[2]);
+    }
+    double2 eyx = zero, ezx = zero, exy = zero, ezy = zero;
+    if (xok) {
+      eyx = ec[3 * dx + 1];
+      ezx = ec[3 * dx + 2];
+      if (BL && !xin) {
+        eyx = cmul(eyx, ex.ph[0]);
+        ezx = cmul(ezx, ex.ph[0]);
+      }
+    }
+    if (yok) {
+      exy = ec[3 * dy];
+      ezy = ec[3 * dy + 2];
+      if (BL && !yin) {
+        exy = cmul(exy, ex.ph[1]);
+        ezy = cmul(ezy, ex.ph[1]);
+      }
+    }
+    // tangential E on the low PEC walls is pinned
+    const double2 ex0 = (pj || z0) ? zero : v0, ey0 = (pi || z0) ? zero : v1, ez0 = (pi || pj) ? zero : v2;
+    if (z0) eyx = exy = zero;
+    if (pj) ezx = zero;
+    if (pi) ezy = zero;
+    const double2 exz = pj ? zero : n0, eyz = pi ? zero : n1;
+    const double2 cz = cscale(a.cm[2][k], sc);
+    const bool zr = cz.y == 0.0;
+    double2 h[3];
+    const double2 dzy = csub(ezy, ez0), dyz = csub(eyz, ey0), dxz = csub(exz, ex0), dzx = csub(ezx, ez0),
+                  dyx = csub(eyx, ey0), dxy = csub(exy, ex0);
+    by_axis(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
+      constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+      h[0] = mul_c<YR>(cy, dzy);
+      axpy_c<true, ZR>(h[0], cz, dyz);
+      h[1] = mul_c<ZR>(cz, dxz);
+      axpy_c<true, XR>(h[1], cx, dzx);
+      h[2] = mul_c<XR>(cx, dyx);
+      axpy_c<true, YR>(h[2], cy, dxy);
+    });
+    if (act) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double2 m = zero;
+        if (jm) m = jm[3 * cell + c];
+        if (REALW) hout[3 * cell + c] = mk(fma(-sc, m.y, -h[c].y), fma(sc, m.x, h[c].x));
+        else hout[3 * cell + c] = cmul(iow, cadd(h[c], m));
+      }
+    }
+    v0 = n0;
+    v1 = n1;
+    v2 = n2;
   }
 }
 
@@ -85,47 +212,75 @@ __global__ void k_e_from_h(OpArgs<double> a, Extra<double> ex, const double2 *__
   }
 }
 
-__global__ void k_corner_mean(OpArgs<double> a, Extra<double> ex, int hfield, const double2 *__restrict__ in,
-                              double2 *__restrict__ out) {
-  const long long nc = a.ncell;
-  for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < nc;
-       cell += (long long)gridDim.x * blockDim.x) {
-    const int g[3] = {(int)(cell % a.N[0]), (int)((cell / a.N[0]) % a.N[1]), (int)(cell / ((long long)a.N[0] * a.N[1]))};
-#pragma unroll
-    for (int w = 0; w < 3; ++w) {
-      const long long stride = (w == 0) ? 1 : (w == 1) ? a.N[0] : (long long)a.N[0] * a.N[1];
-      const int n = a.N[w], t = g[w];
-      const double2 self = in[3 * cell + w];
-      double2 r;
-      if (!hfield) {
-        // backward mean of E_w onto the primal corner t
-        double2 nb, wnb;
-        if (t > 0) {
-          nb = in[3 * (cell - stride) + w];
-          wnb = ex.sdlm[w][t - 1];
-        } else if (a.bloch[w]) {
-          nb = cmul(in[3 * (cell + (long long)(n - 1) * stride) + w], ex.phinv[w]);
-          wnb = ex.sdlm[w][n - 1];
-        } else {
-          nb = self;
-          wnb = ex.sdlm[w][0];
-        }
-        r = cadd(cmul(wnb, nb), cmul(ex.sdlm[w][t], self));
-        r = cmul(r, cinv(cscale(ex.sdle[w][t], 2.0)));
-      } else {
-        // forward mean of H_w onto the dual corner t
-        double2 nb = czero<double2>(), wnb = czero<double2>();
-        if (t + 1 < n) {
-          nb = in[3 * (cell + stride) + w];
-          wnb = ex.sdle[w][t + 1];
-        } else if (a.bloch[w]) {
-          nb = cmul(in[3 * (cell - (long long)(n - 1) * stride) + w], ex.ph[w]);
-          wnb = ex.sdle[w][0];
-        }
-        r = cadd(cmul(ex.sdle[w][t], self), cmul(wnb, nb));
-        r = cmul(r, cinv(cscale(ex.sdlm[w][t], 2.0)));
-      }
-      out[3 * cell + w] = r;
+// Weights of a two-point mean along each axis, per index t: own[w][t] of the
+// value at t and nb[w][t] of its neighbour (t − 1 for E, t + 1 for H).
+struct MeanW {
+  const double2 *own[3], *nb[3];
+};
+
+template <bool HF, bool BL>
+__global__ void __launch_bounds__(FB) k_corner_mean(OpArgs<double> a, Extra<double> ex, MeanW wt,
+                                                    const double2 *__restrict__ in, double2 *__restrict__ out, int kc) {
+  const int plane = a.N[0] * a.N[1];
+  const int p0 = blockIdx.x * FB + threadIdx.x;
+  const bool act = p0 < plane;
+  const int p = act ? p0 : plane - 1;
+  const int i = p % a.N[0], j = p / a.N[0];
+  const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, a.N[2]);
+  const double2 ox = wt.own[0][i], nx = wt.nb[0][i], oy = wt.own[1][j], ny = wt.nb[1][j];
+  const bool xr = __all_sync(0xffffffffu, ox.y == 0.0 && nx.y == 0.0);
+  const bool yr = __all_sync(0xffffffffu, oy.y == 0.0 && ny.y == 0.0);
+  // neighbour along x and y: in the grid, wrapped with the Bloch phase, or a
+  // symmetry wall (E mirrors its own value, H is 0)
+  const bool xin = HF ? i + 1 < a.N[0] : i > 0, yin = HF ? j + 1 < a.N[1] : j > 0;
+  const long long dx = HF ? (xin ? 1 : 1 - a.N[0]) : (xin ? -1 : a.N[0] - 1);
+  const long long dy = HF ? (yin ? a.N[0] : a.N[0] - plane) : (yin ? -a.N[0] : plane - a.N[0]);
+  const double2 zero = czero<double2>();
+  const double2 phx = HF ? ex.ph[0] : ex.phinv[0], phy = HF ? ex.ph[1] : ex.phinv[1];
+  // z: the value at k carried from plane to plane (E: the previous one, H: the next)
+  const bool blx = BL && a.bloch[0], bly = BL && a.bloch[1], blz = BL && a.bloch[2];
+  double2 carry = zero;
+  if (HF) carry = in[3 * ((long long)plane * k0 + p) + 2];
+  else if (k0 > 0) carry = in[3 * ((long long)plane * (k0 - 1) + p) + 2];
+  for (int k = k0; k < k1; ++k) {
+    const long long cell = (long long)plane * k + p;
+    const double2 *ic = in + 3 * cell;
+    const double2 s0 = ic[0], s1 = ic[1];
+    double2 b0 = HF ? zero : s0, b1 = HF ? zero : s1;
+    if (xin || blx) b0 = ic[3 * dx];
+    if (yin || bly) b1 = ic[3 * dy + 1];
+    if (BL) {
+      if (!xin && blx) b0 = cmul(b0, phx);
+      if (!yin && bly) b1 = cmul(b1, phy);
+    }
+    double2 s2, b2;
+    if (HF) {
+      s2 = carry;
+      b2 = zero;
+      if (k + 1 < a.N[2]) b2 = carry = ic[3ll * plane + 2];
+      else if (blz) b2 = cmul(in[3ll * p + 2], ex.ph[2]);
+    } else {
+      s2 = ic[2];
+      b2 = carry;
+      if (k == 0) b2 = blz ? cmul(in[3 * ((long long)plane * (a.N[2] - 1) + p) + 2], ex.phinv[2]) : s2;
+      carry = s2;
+    }
+    const double2 oz = wt.own[2][k], nz = wt.nb[2][k];
+    const bool zr = oz.y == 0.0 && nz.y == 0.0;
+    double2 r0, r1, r2;
+    by_axis(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
+      constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+      r0 = mul_c<XR>(ox, s0);
+      r1 = mul_c<YR>(oy, s1);
+      r2 = mul_c<ZR>(oz, s2);
+      axpy_c<false, XR>(r0, nx, b0);
+      axpy_c<false, YR>(r1, ny, b1);
+      axpy_c<false, ZR>(r2, nz, b2);
+    });
+    if (act) {
+      out[3 * cell] = r0;
+      out[3 * cell + 1] = r1;
+      out[3 * cell + 2] = r2;
     }
   }
 }
@@ -231,6 +386,18 @@ int d2h_real(fdfd_handle *h, const double *src, double *dst, int mask) {
                     "D2H values");
 }
 
+// Grid of a z-marching plane kernel: blocks over the flattened plane, and
+// chunks of kc planes short enough to give the chip about eight blocks per
+// SM (a chunk re-reads one plane, so at most 16 planes gain nothing more).
+static dim3 plane_grid(const fdfd_handle *h, int *kc) {
+  const long long bx = ((long long)h->N[0] * h->N[1] + FB - 1) / FB;
+  const long long k = bx * h->N[2] / (152 * 8);
+  *kc = (int)std::max(1ll, std::min(16ll, k));
+  // blockIdx.y is limited to 65535 chunks
+  *kc = std::max(*kc, (h->N[2] + 65534) / 65535);
+  return dim3((unsigned)bx, (unsigned)((h->N[2] + *kc - 1) / *kc), 1);
+}
+
 int h_from_e_dev_impl(fdfd_handle *h, const double2 *e, const double2 *jm, double2 *hout) {
   const OpArgs<double> a = op_args<double>(h);
   const Extra<double> ex = make_extra<double>(h);
@@ -238,7 +405,12 @@ int h_from_e_dev_impl(fdfd_handle *h, const double2 *e, const double2 *jm, doubl
   const double wr = h->omega[0], wi = h->omega[1], d = wr * wr + wi * wi;
   if (!(d > 0.0)) return set_error(h, FDFD_ERR_ARG, "h_from_e needs ω ≠ 0");
   const double2 iow = make_double2(wi / d, wr / d);
-  k_h_from_e<<<152 * 8, 256, 0, h->stream>>>(a, ex, e, jm, hout, iow);
+  int kc;
+  const dim3 grid = plane_grid(h, &kc);
+  const bool bl = h->bloch[0] || h->bloch[1] || h->bloch[2];
+  const auto kern = iow.x == 0.0 ? (bl ? k_h_from_e<true, true> : k_h_from_e<true, false>)
+                                 : (bl ? k_h_from_e<false, true> : k_h_from_e<false, false>);
+  kern<<<grid, FB, 0, h->stream>>>(a, ex, e, jm, hout, iow, kc);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "k_h_from_e");
 }
@@ -260,7 +432,18 @@ int e_from_h_dev_impl(fdfd_handle *h, const double2 *hin, const double2 *je, dou
 int corner_mean_dev_impl(fdfd_handle *h, int hfield, const double2 *in, double2 *out) {
   const OpArgs<double> a = op_args<double>(h);
   const Extra<double> ex = make_extra<double>(h);
-  k_corner_mean<<<152 * 8, 256, 0, h->stream>>>(a, ex, hfield, in, out);
+  // weights: E backward mean wp (own), wm; H forward mean kinds 6 (own) and 7
+  MeanW wt;
+  for (int w = 0; w < 3; ++w) {
+    wt.own[w] = hfield ? h->coef64 + 6 * h->coef_stride + h->coef_off[w] : a.wp[w];
+    wt.nb[w] = hfield ? h->coef64 + 7 * h->coef_stride + h->coef_off[w] : a.wm[w];
+  }
+  int kc;
+  const dim3 grid = plane_grid(h, &kc);
+  const bool bl = h->bloch[0] || h->bloch[1] || h->bloch[2];
+  const auto kern = hfield ? (bl ? k_corner_mean<true, true> : k_corner_mean<true, false>)
+                           : (bl ? k_corner_mean<false, true> : k_corner_mean<false, false>);
+  kern<<<grid, FB, 0, h->stream>>>(a, ex, wt, in, out, kc);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "k_corner_mean");
 }

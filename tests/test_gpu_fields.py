@@ -87,3 +87,32 @@ def test_e_from_h(pkg, oracle, bloch, kb):
     with pytest.raises(pkg.FDFDError):
         A.e_from_h(h)
     A.close()
+
+
+@pytest.mark.parametrize("bloch", [(False, False, False), (True, False, False), (False, True, False),
+                                   (False, False, True), (True, True, True)])
+@pytest.mark.parametrize("N", [(2, 2, 2), (3, 43, 2), (64, 4, 5), (129, 2, 35)])
+def test_field_kernels_plane_edges(pkg, oracle, bloch, N):
+    """h_from_e and the corner means where their kernels can go wrong: planes
+    of one cell more or less than the 256-thread block, of several blocks,
+    one-plane and several-plane z-chunks, each axis periodic in turn, and
+    real and complex ω (the factor i/ω folded into the curl or not).  The
+    bound is that of the other tests here (FP64 on both sides)."""
+    O = oracle
+    rng = np.random.default_rng(41)
+    lp = tuple(np.concatenate([[0.0], np.cumsum(rng.uniform(0.6, 1.4, n))]) for n in N)
+    g = O.Grid(lp, bloch)
+    kb = tuple(0.17 if b else 0.0 for b in bloch)
+    npml = tuple(0 if bloch[w] or N[w] < 8 else 3 for w in range(3))
+    for om in (2 * np.pi / 6.5, 0.9 + 0.2j):
+        sdl_e, sdl_m = O.stretched_dl(g, 2 * np.pi / 6.5, (npml, npml))
+        Ce, _ = O.create_curls(g, sdl_e, sdl_m, kb)
+        Mce, Mcm = O.create_Mcs(g, sdl_e, sdl_m, kb)
+        A = pkg.FDFDOperator(g.N, om, sdl_e, sdl_m, bloch, [np.exp(-1j * kb[w] * g.L[w]) for w in range(3)])
+        n = 3 * g.ncell
+        v = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        jm = rng.standard_normal(n) + 1j * rng.standard_normal(n)
+        for got, ref in ((A.h_from_e(v, jm), O.h_from_e(v, om, Ce, jm)), (A.h_from_e(v), O.h_from_e(v, om, Ce, None)),
+                         (A.corner_mean(v, "E"), Mce @ v), (A.corner_mean(v, "H"), Mcm @ v)):
+            assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+        A.close()
