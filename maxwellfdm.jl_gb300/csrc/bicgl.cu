@@ -30,6 +30,7 @@
 // (complex128), in a fixed order.
 // The grid-stride vector kernels run one full wave (SM count × the
 // kernel's resident blocks per SM), so none ends on a partial wave.
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
 
@@ -157,69 +158,6 @@ __global__ void __launch_bounds__(VB) k_bl_r(VSet<typename CT<R>::C> r, VSet<typ
 
 constexpr int pow2_at_least(int k) { return k <= 1 ? 1 : 2 * pow2_at_least((k + 1) / 2); }
 
-// Sum NV complex FP64 values over the block (complex128 kernels), write the
-// block's partials, and return true in the block that arrives last (which
-// then holds the grid sums, in block order, in `tot`).
-template <int NV>
-__device__ bool block_sums_last(double2 (&v)[NV], RedBuf red, double2 (&tot)[NV]) {
-  __shared__ double2 wred[VB / 32][NV];
-  __shared__ bool last;
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      v[q].x += __shfl_xor_sync(0xffffffffu, v[q].x, o);
-      v[q].y += __shfl_xor_sync(0xffffffffu, v[q].y, o);
-    }
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NV; ++q) wred[wid][q] = v[q];
-  __syncthreads();
-  if (tid < NV) {
-    double2 s = make_double2(0, 0);
-    for (int w = 0; w < VB / 32; ++w) s = addd(s, wred[w][tid]);
-    red.part[(long long)NV * blockIdx.x + tid] = s;
-  }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(red.count, 1u);
-    last = prev == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  // every thread sums a fixed subset of the blocks, then a fixed tree:
-  // deterministic for a given launch shape
-  double2 s[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) s[q] = make_double2(0, 0);
-  for (unsigned b = tid; b < gridDim.x; b += VB)
-#pragma unroll
-    for (int q = 0; q < NV; ++q) s[q] = addd(s[q], __ldcg(&red.part[(long long)NV * b + q]));
-#pragma unroll
-  for (int q = 0; q < NV; ++q)
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      s[q].x += __shfl_xor_sync(0xffffffffu, s[q].x, o);
-      s[q].y += __shfl_xor_sync(0xffffffffu, s[q].y, o);
-    }
-  __syncthreads();
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NV; ++q) wred[wid][q] = s[q];
-  __syncthreads();
-  if (tid < NV) {
-    double2 t = make_double2(0, 0);
-    for (int w = 0; w < VB / 32; ++w) t = addd(t, wred[w][tid]);
-    tot[tid] = t;  // tot lives in shared memory of the caller
-  }
-  __syncthreads();
-  if (tid == 0) *red.count = 0u;
-  return true;
-}
-
 // Gram matrix of r_0 … r_L — (r_i, r_j) for 1 ≤ i ≤ j ≤ L, then (r_i, r_0)
 // for 1 ≤ i ≤ L — into sc->gram (last block).  The stored r_i (i < L−1)
 // still lack the last BiCG step's −α u_{i+1}; it is applied in registers.
@@ -296,12 +234,18 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
     if (!df_block_sums_last<VB, K, 2 * NV>(v, red, tot)) return;
     if (threadIdx.x < NV) sc->gram[threadIdx.x] = make_double2(tot[2 * threadIdx.x], tot[2 * threadIdx.x + 1]);
   } else {
-    double2 acc[NV];
+    constexpr int K = pow2_at_least(2 * NV);
+    double v[K];
 #pragma unroll
-    for (int q = 0; q < NV; ++q) acc[q] = make_double2((double)ar[q], (double)ai[q]);
-    __shared__ double2 tot[NV];
-    if (!block_sums_last<NV>(acc, red, tot)) return;
-    if (threadIdx.x < NV) sc->gram[threadIdx.x] = tot[threadIdx.x];
+    for (int q = 0; q < K; ++q) v[q] = 0.0;
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+      v[2 * q] = (double)ar[q];
+      v[2 * q + 1] = (double)ai[q];
+    }
+    __shared__ double tot[2 * NV];
+    if (!d_block_sums_last<VB, K, 2 * NV>(v, red, tot)) return;
+    if (threadIdx.x < NV) sc->gram[threadIdx.x] = make_double2(tot[2 * threadIdx.x], tot[2 * threadIdx.x + 1]);
   }
 }
 
@@ -533,6 +477,16 @@ static int wave_blocks(const void *kern, int cap) {
   return std::min(b, cap);
 }
 
+// Blocks for a reducing kernel over n elements: at most RED_BLOCKS, and at
+// least two element pairs per thread down to one block per SM — below that
+// the block and grid sums cost more than the elements (a warp's share of the
+// Gram matrix's sums is 31 additions; at n = 98304 the FP64 Gram kernel took
+// 68 µs on two blocks per SM with butterfly sums).
+static int red_cap(long long n) {
+  const long long b = (n / 2 + 2 * VB - 1) / (2 * VB);
+  return (int)std::min<long long>(RED_BLOCKS, std::max<long long>(b, 152));
+}
+
 // Launch a grid-stride vector kernel on one full wave.
 template <typename... P, typename... A>
 static void launch_wave(fdfd_handle *h, void (*kern)(P...), int cap, A... args) {
@@ -569,12 +523,12 @@ static int bl_cycle_t(fdfd_handle *h, typename CT<R>::C *x, typename CT<R>::C *c
   // the reducing kernels keep ≤ RED_BLOCKS blocks: 8·RED_BLOCKS partial
   // slots hold the Gram matrix's L(L+1)/2 + L ≤ 14 values per block
   if ((rc = ensure_red(h, 8 * RED_BLOCKS))) return rc;
-  launch_wave(h, k_bl_gram<R, L>, RED_BLOCKS, rs, us, n, h->red, sc);
+  launch_wave(h, k_bl_gram<R, L>, red_cap(n), rs, us, n, h->red, sc);
   if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_gram"))) return rc;
   k_bl_mr<L><<<1, 32, 0, h->stream>>>(sc);
   h->launches++;
   if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_mr"))) return rc;
-  launch_wave(h, k_bl_fin<R, L>, RED_BLOCKS, rs, us, x, n, h->red, sc);
+  launch_wave(h, k_bl_fin<R, L>, red_cap(n), rs, us, x, n, h->red, sc);
   return cuda_check(h, cudaGetLastError(), "k_bl_fin");
 }
 

@@ -26,9 +26,15 @@ enum FinMode : int {
   FIN_BL_REDO = 9,   // after a replaced residual: ρ₁ = (r̂, r₀) against the stored −ω ρ₀
 };
 
+// a / b, called by a converged warp: a warp's FP64 instruction takes 64
+// cycles of its scheduler's pipe for one lane as for 32, so lane 1 divides
+// the imaginary part in the same instructions as the other lanes the real one.
 __device__ __forceinline__ double2 dcdiv(double2 a, double2 b) {
-  double d = b.x * b.x + b.y * b.y;
-  return make_double2((a.x * b.x + a.y * b.y) / d, (a.y * b.x - a.x * b.y) / d);
+  const bool im = (threadIdx.x & 31) == 1;
+  const double d = b.x * b.x + b.y * b.y;
+  const double p = im ? a.y : a.x, q = im ? -a.x : a.y;
+  const double v = (p * b.x + q * b.y) / d;
+  return make_double2(__shfl_sync(0xffffffffu, v, 0), __shfl_sync(0xffffffffu, v, 1));
 }
 __device__ __forceinline__ double2 dcmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -44,60 +50,83 @@ __device__ __forceinline__ void stop_tests(KScalars *sc, double rr) {
   if (rr <= sc->upd2 * sc->rr_max) { sc->done = 1; sc->reason = 2; return; }
 }
 
+// The scalar step of a reduction, run by the first warp of the last block
+// (all lanes hold the same sums; lane 0 stores).
 __device__ inline void finalise(int mode, KScalars *sc, double2 d0, double2 d1) {
-  sc->dot0 = d0;
-  sc->dot1 = d1;
+  const bool w = (threadIdx.x & 31) == 0;
+  const double2 rho = sc->rho, alpha = sc->alpha, omega = sc->omega, rho_pre = sc->rho_pre;
+  __syncwarp();  // every lane has read the old scalars
+  if (w) {
+    sc->dot0 = d0;
+    sc->dot1 = d1;
+  }
+  auto stop = [&](int reason) {
+    if (w) {
+      sc->done = 1;
+      sc->reason = reason;
+    }
+  };
+  // the stop tests of an iteration's end; a vanished scalar is a breakdown
+  // unless they already stop the iteration
+  auto broken = [&](bool tests) {
+    if (!w) return;
+    if (tests) stop_tests(sc, d1.x);
+    if (!sc->done) {
+      sc->done = 1;
+      sc->reason = 3;
+    }
+  };
+  auto zero = [](double2 v) { return v.x == 0.0 && v.y == 0.0; };
   switch (mode) {
-    case FIN_ALPHA: {
-      if (!dfinite(d0)) { sc->done = 1; sc->reason = 4; break; }
-      if (d0.x == 0.0 && d0.y == 0.0) { sc->done = 1; sc->reason = 3; break; }
-      sc->alpha = dcdiv(sc->rho, d0);
+    case FIN_ALPHA:
+    case FIN_COCG_A: {
+      if (!dfinite(d0)) { stop(4); break; }
+      if (zero(d0)) { stop(3); break; }
+      const double2 al = dcdiv(rho, d0);
+      if (w) sc->alpha = al;
       break;
     }
     case FIN_OMEGA: {
-      if (!dfinite(d0) || !isfinite(d1.x)) { sc->done = 1; sc->reason = 4; break; }
-      sc->omega = d1.x > 0.0 ? make_double2(d0.x / d1.x, d0.y / d1.x) : make_double2(0.0, 0.0);
+      if (!dfinite(d0) || !isfinite(d1.x)) { stop(4); break; }
+      if (w) sc->omega = d1.x > 0.0 ? make_double2(d0.x / d1.x, d0.y / d1.x) : make_double2(0.0, 0.0);
       break;
     }
     case FIN_XR: {
-      double2 rho_new = d0;
-      double2 om = sc->omega;
-      if (om.x == 0.0 && om.y == 0.0) { stop_tests(sc, d1.x); if (!sc->done) { sc->done = 1; sc->reason = 3; } break; }
-      if (rho_new.x == 0.0 && rho_new.y == 0.0) { stop_tests(sc, d1.x); if (!sc->done) { sc->done = 1; sc->reason = 3; } break; }
-      sc->beta = dcmul(dcdiv(rho_new, sc->rho), dcdiv(sc->alpha, om));
-      sc->rho = rho_new;
-      stop_tests(sc, d1.x);
-      break;
-    }
-    case FIN_COCG_A: {
-      if (!dfinite(d0)) { sc->done = 1; sc->reason = 4; break; }
-      if (d0.x == 0.0 && d0.y == 0.0) { sc->done = 1; sc->reason = 3; break; }
-      sc->alpha = dcdiv(sc->rho, d0);
+      if (zero(omega) || zero(d0)) { broken(true); break; }
+      const double2 be = dcmul(dcdiv(d0, rho), dcdiv(alpha, omega));
+      if (w) {
+        sc->beta = be;
+        sc->rho = d0;
+        stop_tests(sc, d1.x);
+      }
       break;
     }
     case FIN_BL_RHO:
     case FIN_BL_REDO:
     case FIN_BL_CYCLE: {
-      if (mode == FIN_BL_CYCLE) sc->rho_pre = make_double2(-(sc->omega.x * sc->rho.x - sc->omega.y * sc->rho.y),
-                                                          -(sc->omega.x * sc->rho.y + sc->omega.y * sc->rho.x));
-      const double2 rho0 = mode == FIN_BL_RHO ? sc->rho : sc->rho_pre;
-      if (!dfinite(d0)) { sc->done = 1; sc->reason = 4; break; }
-      if (rho0.x == 0.0 && rho0.y == 0.0) {
-        if (mode == FIN_BL_CYCLE) stop_tests(sc, d1.x);
-        if (!sc->done) { sc->done = 1; sc->reason = 3; }
-        break;
+      double2 rho0 = mode == FIN_BL_RHO ? rho : rho_pre;
+      if (mode == FIN_BL_CYCLE) {
+        rho0 = make_double2(-(omega.x * rho.x - omega.y * rho.y), -(omega.x * rho.y + omega.y * rho.x));
+        if (w) sc->rho_pre = rho0;
       }
-      sc->beta = dcmul(sc->alpha, dcdiv(d0, rho0));
-      sc->rho = d0;
-      if (mode == FIN_BL_CYCLE) stop_tests(sc, d1.x);
+      if (!dfinite(d0)) { stop(4); break; }
+      if (zero(rho0)) { broken(mode == FIN_BL_CYCLE); break; }
+      const double2 be = dcmul(alpha, dcdiv(d0, rho0));
+      if (w) {
+        sc->beta = be;
+        sc->rho = d0;
+        if (mode == FIN_BL_CYCLE) stop_tests(sc, d1.x);
+      }
       break;
     }
     case FIN_COCG_R: {
-      double2 rho_new = d0;
-      if (sc->rho.x == 0.0 && sc->rho.y == 0.0) { sc->done = 1; sc->reason = 3; break; }
-      sc->beta = dcdiv(rho_new, sc->rho);
-      sc->rho = rho_new;
-      stop_tests(sc, d1.x);
+      if (zero(rho)) { stop(3); break; }
+      const double2 be = dcdiv(d0, rho);
+      if (w) {
+        sc->beta = be;
+        sc->rho = d0;
+        stop_tests(sc, d1.x);
+      }
       break;
     }
     default:
@@ -133,8 +162,11 @@ __device__ __forceinline__ typename CT<R>::C shadow(long long dof) {
                                  __uint_as_float(0x4B000000u | ((hsh >> 16) ^ 0x8000u)));
     return __ffma2_rn(b, make_float2(1.0f / 32768.0f, 1.0f / 32768.0f), make_float2(-257.0f, -257.0f));
   } else {
-    const int re = (int)(int16_t)(hsh & 0xffffu), im = (int)(int16_t)(hsh >> 16);
-    return mk(R(re) * R(1.0 / 32768.0), R(im) * R(1.0 / 32768.0));
+    // the double with high word 0x42400000 and low word v is 2³⁷ + v·2⁻¹⁵
+    // exactly: one FP64 instruction per value (a conversion and a product
+    // would be two)
+    return mk(__hiloint2double(0x42400000, (int)((hsh & 0xffffu) ^ 0x8000u)) - 137438953473.0,
+              __hiloint2double(0x42400000, (int)((hsh >> 16) ^ 0x8000u)) - 137438953473.0);
   }
 }
 
@@ -279,73 +311,95 @@ __device__ inline void block_reduce_finalise_df(DF a0r, DF a0i, DF a1r, DF a1i, 
   __shared__ double tot[4];
   DF v[4] = {a0r, a0i, a1r, a1i};
   if (!df_block_sums_last<NT, 4, 4>(v, red, tot)) return;
-  if (threadIdx.x + threadIdx.y + threadIdx.z == 0 && sc)
+  if (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z) < 32 && sc)
     finalise(mode, sc, make_double2(tot[0], tot[1]), make_double2(tot[2], tot[3]));
 }
 
-// Block-level reduction of two complex FP64 values (complex128 kernels),
-// then the grid-level last-block finalisation.  Must be called by every
-// thread of the block.
-template <int NT>
-__device__ inline void block_reduce_finalise(double2 a0, double2 a1, RedBuf red, int mode, KScalars *sc) {
-  __shared__ double2 wred[NT / 32][2];
-  __shared__ bool last;
+// The FP64 counterparts for complex128 kernels.  The reduce-scatter matters
+// more here: a butterfly on each of the Gram matrix's 28 sums is 140 FP64
+// instructions of 64 cycles per warp, the scatter 31.
+template <int M, int O>
+struct DScatter {
+  static __device__ __forceinline__ void run(double *v, int lane) {
+    if constexpr (M > 1) {
+      const bool up = (lane & O) != 0;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0.x += __shfl_xor_sync(0xffffffffu, a0.x, o);
-    a0.y += __shfl_xor_sync(0xffffffffu, a0.y, o);
-    a1.x += __shfl_xor_sync(0xffffffffu, a1.x, o);
-    a1.y += __shfl_xor_sync(0xffffffffu, a1.y, o);
+      for (int i = 0; i < M / 2; ++i) {
+        const double keep = up ? v[M / 2 + i] : v[i];
+        const double send = up ? v[i] : v[M / 2 + i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, O);
+      }
+      DScatter<M / 2, O / 2>::run(v, lane);
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], O);
+      DScatter<1, O / 2>::run(v, lane);
+    }
   }
+};
+template <int M>
+struct DScatter<M, 0> {
+  static __device__ __forceinline__ void run(double *, int) {}
+};
+
+// Block and grid sums of KR FP64 values per thread, as df_block_sums_last
+// (KR doubles of red.part per block); tot holds the grid sums in the last
+// block, which sums the blocks' partials with all its warps.
+template <int NT, int K, int KR>
+__device__ bool d_block_sums_last(double (&v)[K], RedBuf red, double *tot) {
+  static_assert((K & (K - 1)) == 0 && K <= 32 && KR <= K && (KR % 2) == 0, "FP64 block sums");
+  constexpr int NW = NT / 32;
+  constexpr int G = KR <= NW ? NW / KR : 1;  // warps that share one value's partials
+  __shared__ double wred[NW][K];
+  __shared__ bool last;
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int lane = tid & 31, wid = tid >> 5;
-  if (lane == 0) { wred[wid][0] = a0; wred[wid][1] = a1; }
+  DScatter<K, 16>::run(v, lane);
+  if ((lane & ((1 << df_shift<K>()) - 1)) == 0) wred[wid][lane >> df_shift<K>()] = v[0];
   __syncthreads();
   const unsigned nblk = gridDim.x * gridDim.y * gridDim.z;
   const unsigned bid = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-  if (tid == 0) {
-    double2 s0 = make_double2(0, 0), s1 = make_double2(0, 0);
-    for (int w = 0; w < NT / 32; ++w) {
-      s0.x += wred[w][0].x; s0.y += wred[w][0].y;
-      s1.x += wred[w][1].x; s1.y += wred[w][1].y;
-    }
-    red.part[2 * bid] = s0;
-    red.part[2 * bid + 1] = s1;
-    __threadfence();
-    unsigned prev = atomicAdd(red.count, 1u);
-    last = (prev == nblk - 1);
-  }
-  __syncthreads();
-  if (!last) return;
-  // last block: deterministic sum of all partials in block order
-  __threadfence();
-  double2 s0 = make_double2(0, 0), s1 = make_double2(0, 0);
-  for (unsigned b = tid; b < nblk; b += NT) {
-    double2 p0 = __ldcg(&red.part[2 * b]);
-    double2 p1 = __ldcg(&red.part[2 * b + 1]);
-    s0.x += p0.x; s0.y += p0.y;
-    s1.x += p1.x; s1.y += p1.y;
-  }
-  // fixed-order tree over the block (deterministic for a fixed launch shape)
+  double *part = reinterpret_cast<double *>(red.part);
+  if (tid < KR) {
+    double s = wred[0][tid];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s0.x += __shfl_xor_sync(0xffffffffu, s0.x, o);
-    s0.y += __shfl_xor_sync(0xffffffffu, s0.y, o);
-    s1.x += __shfl_xor_sync(0xffffffffu, s1.x, o);
-    s1.y += __shfl_xor_sync(0xffffffffu, s1.y, o);
+    for (int w = 1; w < NW; ++w) s += wred[w][tid];
+    part[(long long)KR * bid + tid] = s;
+    __threadfence();
   }
   __syncthreads();
-  if (lane == 0) { wred[wid][0] = s0; wred[wid][1] = s1; }
+  if (tid == 0) last = atomicAdd(red.count, 1u) == nblk - 1;
   __syncthreads();
-  if (tid == 0) {
-    double2 t0 = make_double2(0, 0), t1 = make_double2(0, 0);
-    for (int w = 0; w < NT / 32; ++w) {
-      t0.x += wred[w][0].x; t0.y += wred[w][0].y;
-      t1.x += wred[w][1].x; t1.y += wred[w][1].y;
-    }
-    *red.count = 0u;
-    if (sc) finalise(mode, sc, t0, t1);
+  if (!last) return false;
+  __threadfence();
+  for (int q = wid; q < KR * G; q += NW) {
+    const int val = q % KR, g = q / KR;
+    double s = 0.0;
+    for (unsigned b = lane + 32 * g; b < nblk; b += 32 * G) s += __ldcg(&part[(long long)KR * b + val]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) wred[g][val] = s;
   }
+  __syncthreads();
+  if (tid < KR) {
+    double s = wred[0][tid];
+#pragma unroll
+    for (int g = 1; g < G; ++g) s += wred[g][tid];
+    tot[tid] = s;
+  }
+  __syncthreads();
+  if (tid == 0) *red.count = 0u;
+  return true;
+}
+
+// complex128 kernels: grid sums of the complex a0 and a1, then finalise in
+// the last block.  Must be called by every thread of the block.
+template <int NT>
+__device__ inline void block_reduce_finalise(double2 a0, double2 a1, RedBuf red, int mode, KScalars *sc) {
+  __shared__ double tot[4];
+  double v[4] = {a0.x, a0.y, a1.x, a1.y};
+  if (!d_block_sums_last<NT, 4, 4>(v, red, tot)) return;
+  if (threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z) < 32 && sc)
+    finalise(mode, sc, make_double2(tot[0], tot[1]), make_double2(tot[2], tot[3]));
 }
 
 // Per-thread accumulator: FP64 for double kernels; for float kernels a

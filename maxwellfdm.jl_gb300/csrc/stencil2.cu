@@ -153,8 +153,11 @@ __device__ __forceinline__ float2 pdot3(float2 a0, float2 b0, float2 a1, float2 
   t = __ffma2_rn(f2(a2.x), b2, t);
   return __ffma2_rn(make_float2(a2.y, -a2.y), make_float2(b2.y, b2.x), t);
 }
-__device__ __forceinline__ double2 pdot3(double2 a0, double2 b0, double2 a1, double2 b1, double2 a2, double2 b2) {
-  return cadd(cadd(cdotc(a0, b0), cdotc(a1, b1)), cdotc(a2, b2));
+// (re, im) += conj(a)·b
+template <typename R, typename C>
+__device__ __forceinline__ void dot_into(R &re, R &im, C a, C b) {
+  re = fma(a.y, b.y, fma(a.x, b.x, re));
+  im = fma(-a.y, b.x, fma(a.x, b.y, im));
 }
 // a·u + b·v for coefficients a, b that are real when RC (corner averaging)
 template <bool RC>
@@ -679,9 +682,16 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
             acc.i0.add(q0.y + q1.y + q2.y);
             acc.r1.add(yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
           } else if (EPI == EPI_DOT_SHD) {
-            const C q = pdot3(shadow<R>(3ll * ce), yx, shadow<R>(3ll * ce + 1), yy, shadow<R>(3ll * ce + 2), yz);
-            acc.r0.add(q.x);
-            acc.i0.add(q.y);
+            const C s0 = shadow<R>(3ll * ce), s1 = shadow<R>(3ll * ce + 1), s2 = shadow<R>(3ll * ce + 2);
+            if constexpr (sizeof(R) == 8) {  // straight into the sums: 12 FP64 instructions
+              dot_into(acc.r0.s, acc.i0.s, s0, yx);
+              dot_into(acc.r0.s, acc.i0.s, s1, yy);
+              dot_into(acc.r0.s, acc.i0.s, s2, yz);
+            } else {
+              const C q = pdot3(s0, yx, s1, yy, s2, yz);
+              acc.r0.add(q.x);
+              acc.i0.add(q.y);
+            }
           }
           C *yo = y + 3 * ce;
           yo[0] = yx;

@@ -121,3 +121,41 @@ def test_bicgstabl_degrees(pkg, sysx, ell):
         assert rel <= 1e-8 * 1.01, (ell, tr, rel, st)
         assert st[0]["matvecs"] >= 2 * ell
     A.close()
+
+
+@pytest.mark.parametrize("ell", [1, 2, 3, 4])
+@pytest.mark.parametrize("N", [(4, 3, 2), (33, 9, 7), (40, 24, 26)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_reductions_of_every_ell(pkg, oracle, N, ell, precision):
+    """The Gram matrix, the closing update and the dot products of
+    BiCGStab(1 … 4) on systems of 72 to 75 k unknowns — fewer element pairs
+    than one block's threads, an odd count, and several blocks: the true
+    residual, recomputed with the oracle's matrix, meets the tolerance."""
+    S = _system(oracle, N, spheres=False) if min(N) > 6 else None
+    if S is None:
+        g = oracle.uniform_grid(N)
+        S = oracle.System(g, 2 * np.pi / 7.0, ((0, 0, 0), (0, 0, 0)), [])
+    A = _op(pkg, S)
+    rng = np.random.default_rng(5)
+    b = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    x, st = A.solve(b, tol=1e-8, precision=precision, ell=ell)
+    rel = np.linalg.norm(b - S.A @ x) / np.linalg.norm(b)
+    assert rel <= 1e-8 * 1.01, (rel, st)
+    A.close()
+
+
+@pytest.mark.parametrize("N", [(2, 2, 2), (31, 9, 2), (64, 40, 70)])
+def test_residual_norm(pkg, oracle, N):
+    """‖b − A x‖² of fdfd_residual_dev (the FP64 block and grid sums) against
+    numpy: one block, a partial block, many blocks."""
+    torch = pytest.importorskip("torch")
+    g = oracle.uniform_grid(N)
+    S = oracle.System(g, 2 * np.pi / 7.0, ((0, 0, 0), (0, 0, 0)), [])
+    A = _op(pkg, S)
+    rng = np.random.default_rng(6)
+    v = [torch.from_numpy(rng.standard_normal((A.n, 2))).cuda() for _ in range(2)]
+    r = torch.empty_like(v[0])
+    rr = A.residual_dev(v[0].data_ptr(), v[1].data_ptr(), r.data_ptr())
+    ref = np.linalg.norm(r.cpu().numpy()) ** 2
+    assert abs(rr - ref) <= 1e-13 * ref
+    A.close()
