@@ -5,7 +5,7 @@
 // degree-ℓ one does not; it needs markedly fewer operator applications in
 // both precisions, for about 1.3× the vector traffic per application.
 //
-// One cycle = 4ℓ + 3 kernels, all reading their scalars from device memory
+// One cycle = 4ℓ + 2 kernels, all reading their scalars from device memory
 // (so a batch of cycles replays as one CUDA graph):
 //   for j = 0 … ℓ−1:
 //     u_i = r_i − β u_i (i ≤ j)                      k_bl_u (+ the deferred
@@ -17,9 +17,8 @@
 //     r_{j+1} = A r_j [, ρ₁ = (r̂, r_{j+1}), β]       operator, EPI_DOT_SHD + FIN_BL_RHO
 // r̂ is the generated shadow vector (shadow() in krylov_fin.cuh): no
 // memory traffic for it.
-//   Gram matrix of r_0 … r_ℓ                                  k_bl_gram
-//   minimal-residual coefficients (modified Gram–Schmidt
-//   carried out on the Gram matrix, one thread)               k_bl_mr
+//   Gram matrix of r_0 … r_ℓ and, in its last block, the
+//   minimal-residual coefficients γ from it                   k_bl_gram
 //   x, r_0, u_0 closing update, (r̂, r_0), ‖r_0‖², stop tests  k_bl_fin + FIN_BL_CYCLE
 // The last BiCG step's updates r_i −= α u_{i+1} (i < ℓ−1) and x += α u_0
 // are never stored: k_bl_gram and k_bl_fin read r_i and u_{i+1} anyway and
@@ -74,13 +73,19 @@ __device__ __forceinline__ void stp(double2 *p, long long q, Pair<double2> v) {
   p[2 * q + 1] = v.b;
 }
 
-// Grid-stride visit of element pairs (n is even: 3·Ncell with Ncell ≥ 2 …
-// an odd tail element is still handled, by block 0 thread 0).
-template <typename F2, typename F1>
-__device__ __forceinline__ void pairs(long long n, F2 f2, F1 f1) {
-  const long long np = n >> 1;
-  for (long long q = blockIdx.x * (long long)VB + threadIdx.x; q < np; q += (long long)gridDim.x * VB) f2(q);
-  if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) f1(n - 1);
+// Grid-stride visit of the n elements: complex64 in pairs (an odd tail
+// element by block 0 thread 0), complex128 — 16 bytes each, and bound by the
+// FP64 pipe on small systems, where pairs leave some threads one pair more
+// than others — singly.
+template <typename R, typename F2, typename F1>
+__device__ __forceinline__ void visit(long long n, F2 f2, F1 f1) {
+  if constexpr (sizeof(R) == 8) {
+    for (long long e = blockIdx.x * (long long)VB + threadIdx.x; e < n; e += (long long)gridDim.x * VB) f1(e);
+  } else {
+    const long long np = n >> 1;
+    for (long long q = blockIdx.x * (long long)VB + threadIdx.x; q < np; q += (long long)gridDim.x * VB) f2(q);
+    if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) f1(n - 1);
+  }
 }
 
 // BiCG step J of a cycle, first half: u_i = r_i − β u_i for i = 0 … J.
@@ -96,7 +101,7 @@ __global__ void __launch_bounds__(VB) k_bl_u(VSet<typename CT<R>::C> r, VSet<typ
   C ba[2];
   scalars<R>([&](int i) { return i == 0 ? sc->beta : sc->alpha; }, ba);
   const C be = ba[0], al = ba[1];
-  pairs(
+  visit<R>(
       n,
       [&](long long q) {
         Pair<C> rv[J + 1], uv[J + 1];
@@ -147,7 +152,7 @@ __global__ void __launch_bounds__(VB) k_bl_r(VSet<typename CT<R>::C> r, VSet<typ
   C a1[1];
   scalars<R>([&](int) { return sc->alpha; }, a1);
   const C al = a1[0];
-  pairs(
+  visit<R>(
       n,
       [&](long long q) {
         const Pair<C> rv = ldp(r.v[J], q), uv = ldp(u.v[J + 1], q);
@@ -158,9 +163,80 @@ __global__ void __launch_bounds__(VB) k_bl_r(VSet<typename CT<R>::C> r, VSet<typ
 
 constexpr int pow2_at_least(int k) { return k <= 1 ? 1 : 2 * pow2_at_least((k + 1) / 2); }
 
+// The minimal-residual step of a cycle from the Gram sums (gram: (r_i, r_j),
+// 1 ≤ i ≤ j ≤ L, then (r_i, r_0), as (re, im) pairs): γ = argmin
+// ‖r_0 − Σ γ_k r_k‖ by G = Tᴴ D T (T unit upper triangular — the modified
+// Gram–Schmidt coefficients), T γ = D⁻¹ T⁻ᴴ g.  Written with the original
+// r_k, the cycle's closing update is x += Σ γ_k r_{k−1}, r_0 −= Σ γ_k r_k,
+// u_0 −= Σ γ_k u_k.  One warp, an entry (a, b) of the factorisation per
+// lane: every FP64 instruction costs its 64 cycles for all entries at once
+// (one thread working through them took 13.5 µs and a launch of its own: with it a
+// BiCGStab(4) cycle of the 32³ box in FP64 took 36 µs more).
+template <int L>
+__device__ __forceinline__ void bl_mr(const double *gram, KScalars *sc) {
+  const int lane = threadIdx.x & 31;
+  // lane (a, b), 0 ≤ a < L, a ≤ b ≤ L (column L: the right-hand side);
+  // lanes beyond hold a copy of entry (L−1, L)
+  constexpr int NE = L * (L + 1) / 2 + L;
+  int la = L - 1, lb = L;
+  {
+    int e = 0;
+#pragma unroll
+    for (int a = 0; a < L; ++a)
+#pragma unroll
+      for (int b = a; b <= L; ++b, ++e)
+        if (lane == e) {
+          la = a;
+          lb = b;
+        }
+  }
+  auto lane_of = [](int a, int b) { return a * (L + 1) - a * (a - 1) / 2 + (b - a); };
+  double2 v;
+  {
+    const int q = lb < L ? lb * (lb + 1) / 2 + la : L * (L + 1) / 2 + la;
+    v = make_double2(gram[2 * q], gram[2 * q + 1]);
+  }
+  auto from = [&](double2 t, int src) {
+    return make_double2(__shfl_sync(0xffffffffu, t.x, src), __shfl_sync(0xffffffffu, t.y, src));
+  };
+  double2 tau = make_double2(0.0, 0.0);  // row a scaled: τ_ab, and γ' in column L
+#pragma unroll
+  for (int p = 0; p < L; ++p) {
+    const double s = __shfl_sync(0xffffffffu, v.x, lane_of(p, p));
+    if (!(s > 0.0) || !isfinite(s)) {
+      if (lane == 0) {
+        sc->done = 1;
+        sc->reason = isfinite(s) ? 3 : 4;
+      }
+      return;
+    }
+    const double inv = 1.0 / s;
+    if (la == p) tau = scd(v, inv);
+    if (p + 1 < L) {
+      // v_ab −= conj(v_pa) τ_pb for the rows below
+      const double2 va = from(v, lane_of(p, la > p ? la : p));
+      const double2 tb = from(tau, lane_of(p, lb > p ? lb : p));
+      if (la > p) v = subd(v, dcmul(conjd(va), tb));
+    }
+  }
+  // back substitution: γ_a = γ'_a − Σ_{b>a} τ_ab γ_b, kept in column L
+  double2 gam = from(tau, lane_of(la, L));
+#pragma unroll
+  for (int p = L - 1; p >= 1; --p) {
+    const double2 gp = from(gam, lane_of(p, L));
+    const double2 t = from(tau, lane_of(la, la < p ? p : L));
+    if (la < p) gam = subd(gam, dcmul(t, gp));
+  }
+  if (lb == L && lane < NE) {
+    sc->gam[la] = gam;
+    if (la == L - 1) sc->omega = gam;
+  }
+}
+
 // Gram matrix of r_0 … r_L — (r_i, r_j) for 1 ≤ i ≤ j ≤ L, then (r_i, r_0)
-// for 1 ≤ i ≤ L — into sc->gram (last block).  The stored r_i (i < L−1)
-// still lack the last BiCG step's −α u_{i+1}; it is applied in registers.
+// for 1 ≤ i ≤ L — and, in the last block, the minimal-residual coefficients
+// from it.  The stored r_i (i < L−1) still lack the last BiCG step's
+// −α u_{i+1}; it is applied in registers.
 template <typename R, int L>
 __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u, long long n,
                                                    RedBuf red, KScalars *sc) {
@@ -191,7 +267,7 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
       ai[q] += d.y;
     }
   };
-  pairs(
+  visit<R>(
       n,
       [&](long long q) {
         C va[L + 1], vb[L + 1];
@@ -232,7 +308,7 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
     }
     __shared__ double tot[2 * NV];
     if (!df_block_sums_last<VB, K, 2 * NV>(v, red, tot)) return;
-    if (threadIdx.x < NV) sc->gram[threadIdx.x] = make_double2(tot[2 * threadIdx.x], tot[2 * threadIdx.x + 1]);
+    if (threadIdx.x < 32) bl_mr<L>(tot, sc);
   } else {
     constexpr int K = pow2_at_least(2 * NV);
     double v[K];
@@ -245,103 +321,11 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
     }
     __shared__ double tot[2 * NV];
     if (!d_block_sums_last<VB, K, 2 * NV>(v, red, tot)) return;
-    if (threadIdx.x < NV) sc->gram[threadIdx.x] = make_double2(tot[2 * threadIdx.x], tot[2 * threadIdx.x + 1]);
+    if (threadIdx.x < 32) bl_mr<L>(tot, sc);
   }
 }
 
-// The minimal-residual step of the cycle from the Gram matrix (one thread;
-// its own launch so the arrays stay in registers): modified Gram–Schmidt on
-// r_1 … r_ℓ carried out on the Gram matrix — r̂_j = Σ_k Lc[j][k] r_k —
-// then the closing coefficients in terms of the original r_k.
-template <int L>
-__global__ void k_bl_mr(KScalars *sc) {
-  if (threadIdx.x != 0 || sc->done) return;
-  double2 G[L + 1][L + 1], g0[L + 1];
-  {
-    int q = 0;
-#pragma unroll
-    for (int j = 1; j <= L; ++j)
-#pragma unroll
-      for (int i = 1; i <= j; ++i, ++q) {
-        G[i][j] = sc->gram[q];
-        G[j][i] = conjd(sc->gram[q]);
-      }
-#pragma unroll
-    for (int i = 1; i <= L; ++i, ++q) g0[i] = sc->gram[q];
-  }
-  double2 Lc[L + 1][L + 1], tau[L + 1][L + 1], gp[L + 1], gam[L + 1], gpp[L + 1];
-  double isig[L + 1];
-#pragma unroll
-  for (int a = 0; a <= L; ++a)
-#pragma unroll
-    for (int b = 0; b <= L; ++b) Lc[a][b] = tau[a][b] = make_double2(0, 0);
-  double2 gr0[L + 1];  // (r̂_i, r_0)
-#pragma unroll
-  for (int j = 1; j <= L; ++j) {
-    Lc[j][j] = make_double2(1, 0);
-    double2 dij[L + 1];  // (r̂_i, r_j)
-#pragma unroll
-    for (int i = 1; i < j; ++i) {
-      double2 d = make_double2(0, 0);
-#pragma unroll
-      for (int k = 1; k <= i; ++k) d = addd(d, dcmul(conjd(Lc[i][k]), G[k][j]));
-      dij[i] = d;
-      tau[i][j] = scd(d, isig[i]);
-#pragma unroll
-      for (int k = 1; k <= i; ++k) Lc[j][k] = subd(Lc[j][k], dcmul(tau[i][j], Lc[i][k]));
-    }
-    // with r̂_j = r_j − Σ_{i<j} τ_ij r̂_i and the r̂_i orthogonal:
-    //   (r̂_j, r̂_j) = (r_j, r_j) − Σ_i |(r̂_i, r_j)|²/σ_i
-    //   (r̂_j, r_0)  = (r_j, r_0) − Σ_i conj(τ_ij) (r̂_i, r_0)
-    double s = G[j][j].x;
-    double2 g = g0[j];
-#pragma unroll
-    for (int i = 1; i < j; ++i) {
-      s -= (dij[i].x * dij[i].x + dij[i].y * dij[i].y) * isig[i];
-      g = subd(g, dcmul(conjd(tau[i][j]), gr0[i]));
-    }
-    if (!(s > 0.0) || !isfinite(s)) {
-      sc->done = 1;
-      sc->reason = isfinite(s) ? 3 : 4;
-      return;
-    }
-    isig[j] = 1.0 / s;
-    gr0[j] = g;
-    gp[j] = scd(g, isig[j]);
-  }
-  gam[L] = gp[L];
-#pragma unroll
-  for (int j = L - 1; j >= 1; --j) {
-    double2 t = gp[j];
-#pragma unroll
-    for (int i = j + 1; i <= L; ++i) t = subd(t, dcmul(tau[j][i], gam[i]));
-    gam[j] = t;
-  }
-#pragma unroll
-  for (int j = 1; j < L; ++j) {
-    double2 t = gam[j + 1];
-#pragma unroll
-    for (int i = j + 1; i < L; ++i) t = addd(t, dcmul(tau[j][i], gam[i + 1]));
-    gpp[j] = t;
-  }
-#pragma unroll
-  for (int k = 0; k <= LMAX; ++k) sc->cx[k] = sc->cr[k] = sc->cu[k] = make_double2(0, 0);
-  sc->cx[0] = gam[1];
-#pragma unroll
-  for (int k = 1; k <= L; ++k) {
-    double2 cx = make_double2(0, 0), cr = make_double2(0, 0);
-#pragma unroll
-    for (int j = k; j < L; ++j) cx = addd(cx, dcmul(gpp[j], Lc[j][k]));
-#pragma unroll
-    for (int j = k; j <= L; ++j) cr = subd(cr, dcmul(gp[j], Lc[j][k]));
-    sc->cx[k] = cx;
-    sc->cr[k] = cr;
-    sc->cu[k] = make_double2(-gam[k].x, -gam[k].y);
-  }
-  sc->omega = gam[L];
-}
-
-// x += α u_0 + Σ cx_k r_k ; r_0 += Σ cr_k r_k ; u_0 += Σ cu_k u_k ; then
+// x += α u_0 + Σ γ_k r_{k−1} ; r_0 −= Σ γ_k r_k ; u_0 −= Σ γ_k u_k ; then
 // (r̂, r_0) and ‖r_0‖² → FIN_BL_CYCLE.  α u_0 and the r_i −= α u_{i+1}
 // (i < L−1) are the last BiCG step's deferred updates (α of that step:
 // nothing writes sc->alpha between it and this kernel).
@@ -350,16 +334,11 @@ __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<type
                                                   typename CT<R>::C *x, long long n, RedBuf red, KScalars *sc) {
   using C = typename CT<R>::C;
   if (sc->done) return;
-  C cs[3 * (L + 1) + 1];
-  scalars<R>(
-      [&](int i) {
-        return i <= L ? sc->cx[i] : i <= 2 * L + 1 ? sc->cr[i - (L + 1)] : i <= 3 * L + 2 ? sc->cu[i - 2 * (L + 1)] : sc->alpha;
-      },
-      cs);
-  const C *cx = cs, *cr = cs + (L + 1), *cu = cs + 2 * (L + 1);
-  const C al = cs[3 * (L + 1)];
+  C cs[L + 1];
+  scalars<R>([&](int i) { return i < L ? sc->gam[i] : sc->alpha; }, cs);
+  const C al = cs[L];
   Acc<R> a0r, a0i, a1;
-  pairs(
+  visit<R>(
       n,
       [&](long long q) {
         C ra[L + 1], rb[L + 1], ua[L + 1], ub[L + 1];
@@ -382,16 +361,13 @@ __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<type
         xv.b = cadd(xv.b, cmul(al, ub[0]));
         C r0a = ra[0], r0b = rb[0], u0a = ua[0], u0b = ub[0];
 #pragma unroll
-        for (int k = 0; k <= L; ++k) {
-          xv.a = cadd(xv.a, cmul(cx[k], ra[k]));
-          xv.b = cadd(xv.b, cmul(cx[k], rb[k]));
-        }
-#pragma unroll
         for (int k = 1; k <= L; ++k) {
-          r0a = cadd(r0a, cmul(cr[k], ra[k]));
-          r0b = cadd(r0b, cmul(cr[k], rb[k]));
-          u0a = cadd(u0a, cmul(cu[k], ua[k]));
-          u0b = cadd(u0b, cmul(cu[k], ub[k]));
+          xv.a = cadd(xv.a, cmul(cs[k - 1], ra[k - 1]));
+          xv.b = cadd(xv.b, cmul(cs[k - 1], rb[k - 1]));
+          r0a = csub(r0a, cmul(cs[k - 1], ra[k]));
+          r0b = csub(r0b, cmul(cs[k - 1], rb[k]));
+          u0a = csub(u0a, cmul(cs[k - 1], ua[k]));
+          u0b = csub(u0b, cmul(cs[k - 1], ub[k]));
         }
         stp(x, q, xv);
         stp(r.v[0], q, Pair<C>{r0a, r0b});
@@ -412,11 +388,10 @@ __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<type
         for (int k = 0; k + 1 < L; ++k) rk[k] = csub(rk[k], cmul(al, uk[k + 1]));
         C xe = cadd(x[e], cmul(al, uk[0])), r0 = rk[0], u0 = uk[0];
 #pragma unroll
-        for (int k = 0; k <= L; ++k) xe = cadd(xe, cmul(cx[k], rk[k]));
-#pragma unroll
         for (int k = 1; k <= L; ++k) {
-          r0 = cadd(r0, cmul(cr[k], rk[k]));
-          u0 = cadd(u0, cmul(cu[k], uk[k]));
+          xe = cadd(xe, cmul(cs[k - 1], rk[k - 1]));
+          r0 = csub(r0, cmul(cs[k - 1], rk[k]));
+          u0 = csub(u0, cmul(cs[k - 1], uk[k]));
         }
         x[e] = xe;
         r.v[0][e] = r0;
@@ -525,9 +500,6 @@ static int bl_cycle_t(fdfd_handle *h, typename CT<R>::C *x, typename CT<R>::C *c
   if ((rc = ensure_red(h, 8 * RED_BLOCKS))) return rc;
   launch_wave(h, k_bl_gram<R, L>, red_cap(n), rs, us, n, h->red, sc);
   if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_gram"))) return rc;
-  k_bl_mr<L><<<1, 32, 0, h->stream>>>(sc);
-  h->launches++;
-  if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_mr"))) return rc;
   launch_wave(h, k_bl_fin<R, L>, red_cap(n), rs, us, x, n, h->red, sc);
   return cuda_check(h, cudaGetLastError(), "k_bl_fin");
 }

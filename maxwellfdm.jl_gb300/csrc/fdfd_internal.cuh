@@ -103,11 +103,11 @@ struct KScalars {
   int done;              // 1: later kernels of the batch are no-ops
   int reason;            // 1 recursive converged, 2 reliable update due, 3 breakdown, 4 nonfinite
   long long iter;
-  // BiCGStab(ℓ), ℓ ≤ 4: −ω·ρ of the last cycle end, and the coefficients of
-  // the cycle's closing update x += Σ cx_k r_k, r₀ += Σ cr_k r_k, u₀ += Σ cu_k u_k
+  // BiCGStab(ℓ), ℓ ≤ 4: −ω·ρ of the last cycle end, and the minimal-residual
+  // coefficients γ_1 … γ_ℓ of the cycle's closing update
+  // x += Σ γ_k r_{k−1}, r₀ −= Σ γ_k r_k, u₀ −= Σ γ_k u_k
   double2 rho_pre;
-  double2 cx[5], cr[5], cu[5];
-  double2 gram[14];  // (r_i, r_j), 1 ≤ i ≤ j ≤ ℓ, then (r_i, r_0)
+  double2 gam[4];
 };
 
 struct Workspace;  // solver vectors (solver.cu)
