@@ -8,22 +8,25 @@
 // One cycle = 4ℓ + 2 kernels, all reading their scalars from device memory
 // (so a batch of cycles replays as one CUDA graph):
 //   for j = 0 … ℓ−1:
-//     u_i = r_i − β u_i (i ≤ j)                      k_bl_u (+ the deferred
-//                                                    updates of step j−1)
+//     u_j = r_j − β u_j                              k_bl_step
 //     u_{j+1} = A u_j, γ = (r̂, u_{j+1}), α = ρ/γ     operator, EPI_DOT_SHD + FIN_ALPHA
-//     r_j −= α u_{j+1}; the other r_i and x are      k_bl_r
-//     updated by the next k_bl_u (last step: by
-//     k_bl_gram and k_bl_fin, on the fly)
+//     r_j −= α u_{j+1}                               k_bl_step
 //     r_{j+1} = A r_j [, ρ₁ = (r̂, r_{j+1}), β]       operator, EPI_DOT_SHD + FIN_BL_RHO
 // r̂ is the generated shadow vector (shadow() in krylov_fin.cuh): no
 // memory traffic for it.
 //   Gram matrix of r_0 … r_ℓ and, in its last block, the
 //   minimal-residual coefficients γ from it                   k_bl_gram
 //   x, r_0, u_0 closing update, (r̂, r_0), ‖r_0‖², stop tests  k_bl_fin + FIN_BL_CYCLE
-// The last BiCG step's updates r_i −= α u_{i+1} (i < ℓ−1) and x += α u_0
-// are never stored: k_bl_gram and k_bl_fin read r_i and u_{i+1} anyway and
-// apply them in registers (only r_0, u_0 and x outlive the cycle), which
-// saves nine vector passes per cycle.
+// Only the operator's inputs u_j and r_j are updated as the cycle goes.  The
+// lower vectors' updates of step j — u_i = r_i − β_j u_i, x += α_j u_0,
+// r_i −= α_j u_{i+1} for i < j — are never stored: k_bl_gram and k_bl_fin
+// read those vectors anyway and replay the steps in registers from the saved
+// α_j and β_j (Replay below; only r_0, u_0 and x outlive the cycle).  A
+// cycle of ℓ = 4 makes 46 vector passes instead of the 73 that storing them
+// took (96³ complex64: the solve 1.29× faster).  In complex128 a complex
+// product costs more than three vector passes (FP64 pipe), so there k_bl_gram
+// stores the replayed vectors and x, and k_bl_fin does not replay them again:
+// 55 passes.
 // Vectors and products are in the solve's inner precision; every sum
 // across threads and blocks is double-float FP32 (complex64) or FP64
 // (complex128), in a fixed order.
@@ -49,7 +52,6 @@ struct VSet {
 };
 
 __device__ __forceinline__ double2 conjd(double2 a) { return make_double2(a.x, -a.y); }
-__device__ __forceinline__ double2 addd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
 __device__ __forceinline__ double2 subd(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
 __device__ __forceinline__ double2 scd(double2 a, double s) { return make_double2(a.x * s, a.y * s); }
 
@@ -88,77 +90,54 @@ __device__ __forceinline__ void visit(long long n, F2 f2, F1 f1) {
   }
 }
 
-// BiCG step J of a cycle, first half: u_i = r_i − β u_i for i = 0 … J.
-// For J ≥ 1 it first completes the previous step's updates that the
-// operator did not need (step J−1 updated only r_{J−1}):
-//   r_i −= α u_{i+1} (i < J−1) and x += α u_0, with α of step J−1 —
-// one pass over those vectors instead of two.
-template <typename R, int J>
-__global__ void __launch_bounds__(VB) k_bl_u(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u,
-                                             typename CT<R>::C *x, long long n, const KScalars *sc) {
+// v −= s·w, the form of both BiCG updates: u_j = r_j − β u_j (out = u_j)
+// and r_j −= α u_{j+1} (out = r_j).  Bound by HBM (3 vectors); saves the
+// scalar for the cycle's end.
+template <typename R>
+__global__ void __launch_bounds__(VB) k_bl_step(const typename CT<R>::C *v, const typename CT<R>::C *w,
+                                                typename CT<R>::C *out, long long n, int beta, int j, KScalars *sc) {
   using C = typename CT<R>::C;
   if (sc->done) return;
-  C ba[2];
-  scalars<R>([&](int i) { return i == 0 ? sc->beta : sc->alpha; }, ba);
-  const C be = ba[0], al = ba[1];
+  C s1[1];
+  scalars<R>([&](int) { return beta ? sc->beta : sc->alpha; }, s1);
+  const C s = s1[0];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    (beta ? sc->beta_j : sc->alpha_j)[j] = beta ? sc->beta : sc->alpha;
+    sc->bl_steps = beta ? j : j + 1;
+  }
   visit<R>(
       n,
       [&](long long q) {
-        Pair<C> rv[J + 1], uv[J + 1];
-#pragma unroll
-        for (int i = 0; i <= J; ++i) {
-          rv[i] = ldp(r.v[i], q);
-          uv[i] = ldp(u.v[i], q);
-        }
-        if (J >= 1) {
-#pragma unroll
-          for (int i = 0; i + 1 < J; ++i) {
-            rv[i] = Pair<C>{csub(rv[i].a, cmul(al, uv[i + 1].a)), csub(rv[i].b, cmul(al, uv[i + 1].b))};
-            stp(r.v[i], q, rv[i]);
-          }
-          const Pair<C> xv = ldp(x, q);
-          stp(x, q, Pair<C>{cadd(xv.a, cmul(al, uv[0].a)), cadd(xv.b, cmul(al, uv[0].b))});
-        }
-#pragma unroll
-        for (int i = 0; i <= J; ++i)
-          stp(u.v[i], q, Pair<C>{csub(rv[i].a, cmul(be, uv[i].a)), csub(rv[i].b, cmul(be, uv[i].b))});
+        const Pair<C> a = ldp(v, q), b = ldp(w, q);
+        stp(out, q, Pair<C>{csub(a.a, cmul(s, b.a)), csub(a.b, cmul(s, b.b))});
       },
-      [&](long long e) {
-        C rv[J + 1], uv[J + 1];
-#pragma unroll
-        for (int i = 0; i <= J; ++i) {
-          rv[i] = r.v[i][e];
-          uv[i] = u.v[i][e];
-        }
-        if (J >= 1) {
-#pragma unroll
-          for (int i = 0; i + 1 < J; ++i) {
-            rv[i] = csub(rv[i], cmul(al, uv[i + 1]));
-            r.v[i][e] = rv[i];
-          }
-          x[e] = cadd(x[e], cmul(al, uv[0]));
-        }
-#pragma unroll
-        for (int i = 0; i <= J; ++i) u.v[i][e] = csub(rv[i], cmul(be, uv[i]));
-      });
+      [&](long long e) { out[e] = csub(v[e], cmul(s, w[e])); });
 }
 
-// BiCG step J, second half: r_J −= α u_{J+1} (the operator's next input).
-template <typename R, int J>
-__global__ void __launch_bounds__(VB) k_bl_r(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u, long long n,
-                                             const KScalars *sc) {
-  using C = typename CT<R>::C;
-  if (sc->done) return;
-  C a1[1];
-  scalars<R>([&](int) { return sc->alpha; }, a1);
-  const C al = a1[0];
-  visit<R>(
-      n,
-      [&](long long q) {
-        const Pair<C> rv = ldp(r.v[J], q), uv = ldp(u.v[J + 1], q);
-        stp(r.v[J], q, Pair<C>{csub(rv.a, cmul(al, uv.a)), csub(rv.b, cmul(al, uv.b))});
-      },
-      [&](long long e) { r.v[J][e] = csub(r.v[J][e], cmul(al, u.v[J + 1][e])); });
+// α_1 … α_{L−1} (index 0 … L−2), β_1 … β_{L−1}, then α_0, in one array
+template <int L>
+struct Hist {
+  static constexpr int N = 2 * (L - 1) + 1;
+  static __device__ __forceinline__ double2 at(const KScalars *sc, int i) {
+    return i < L - 1 ? sc->alpha_j[i + 1] : i < 2 * (L - 1) ? sc->beta_j[i - (L - 1) + 1] : sc->alpha_j[0];
+  }
+};
+
+// The steps j = 1 … L−1 of one element: r[0 … L−1] and u[0 … L−1] hold each
+// vector as the operator read it (r_j, u_j of step j) and end as they stand
+// after step L−1.  With X also x += Σ_j α_j u_0; without it u_0 is not used.
+template <int L, bool X, typename C>
+__device__ __forceinline__ void replay(C *r, C *u, C &x, const C *hist) {
+  if (X) x = cadd(x, cmul(hist[2 * (L - 1)], u[0]));
+#pragma unroll
+  for (int j = 1; j < L; ++j) {
+    const C al = hist[j - 1], be = hist[L - 1 + j - 1];
+#pragma unroll
+    for (int i = X ? 0 : 1; i < j; ++i) u[i] = csub(r[i], cmul(be, u[i]));
+    if (X) x = cadd(x, cmul(al, u[0]));
+#pragma unroll
+    for (int i = 0; i < j; ++i) r[i] = csub(r[i], cmul(al, u[i + 1]));
+  }
 }
 
 constexpr int pow2_at_least(int k) { return k <= 1 ? 1 : 2 * pow2_at_least((k + 1) / 2); }
@@ -235,18 +214,16 @@ __device__ __forceinline__ void bl_mr(const double *gram, KScalars *sc) {
 
 // Gram matrix of r_0 … r_L — (r_i, r_j) for 1 ≤ i ≤ j ≤ L, then (r_i, r_0)
 // for 1 ≤ i ≤ L — and, in the last block, the minimal-residual coefficients
-// from it.  The stored r_i (i < L−1) still lack the last BiCG step's
-// −α u_{i+1}; it is applied in registers.
+// from it.
 template <typename R, int L>
-__global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u, long long n,
-                                                   RedBuf red, KScalars *sc) {
+__global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u,
+                                                   typename CT<R>::C *x, long long n, RedBuf red, KScalars *sc) {
+  constexpr bool KEEP = sizeof(R) == 8;  // complex128: the replayed vectors are stored
   using C = typename CT<R>::C;
   constexpr int NV = L * (L + 1) / 2 + L;
-  constexpr int ND = L > 1 ? L - 1 : 1;  // deferred corrections (L − 1 of them)
   if (sc->done) return;
-  C a1[1];
-  scalars<R>([&](int) { return sc->alpha; }, a1);
-  const C al = a1[0];
+  C hist[Hist<L>::N];
+  scalars<R>([&](int i) { return Hist<L>::at(sc, i); }, hist);
   R ar[NV], ai[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) ar[q] = ai[q] = R(0);
@@ -270,8 +247,7 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
   visit<R>(
       n,
       [&](long long q) {
-        C va[L + 1], vb[L + 1];
-        Pair<C> ud[ND];
+        C va[L + 1], vb[L + 1], ua[L], ub[L];
 #pragma unroll
         for (int i = 0; i <= L; ++i) {
           const Pair<C> p = ldp(r.v[i], q);
@@ -279,23 +255,36 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
           vb[i] = p.b;
         }
 #pragma unroll
-        for (int i = 0; i + 1 < L; ++i) ud[i] = ldp(u.v[i + 1], q);
-#pragma unroll
-        for (int i = 0; i + 1 < L; ++i) {
-          va[i] = csub(va[i], cmul(al, ud[i].a));
-          vb[i] = csub(vb[i], cmul(al, ud[i].b));
+        for (int i = 1; i < L; ++i) {
+          const Pair<C> p = ldp(u.v[i], q);
+          ua[i] = p.a;
+          ub[i] = p.b;
         }
+        C none = czero<C>();
+        replay<L, false>(va, ua, none, hist);
+        replay<L, false>(vb, ub, none, hist);
         one(va);
         one(vb);
       },
       [&](long long e) {
-        C v[L + 1];
+        C v[L + 1], ue[L], xe = czero<C>();
+        if (KEEP) xe = x[e];
 #pragma unroll
         for (int i = 0; i <= L; ++i) v[i] = r.v[i][e];
 #pragma unroll
-        for (int i = 0; i + 1 < L; ++i) v[i] = csub(v[i], cmul(al, u.v[i + 1][e]));
+        for (int i = KEEP ? 0 : 1; i < L; ++i) ue[i] = u.v[i][e];
+        replay<L, KEEP>(v, ue, xe, hist);
+        if (KEEP) {
+          x[e] = xe;
+#pragma unroll
+          for (int i = 0; i + 1 < L; ++i) {
+            r.v[i][e] = v[i];
+            u.v[i][e] = ue[i];
+          }
+        }
         one(v);
       });
+  if (KEEP && blockIdx.x == 0 && threadIdx.x == 0) sc->bl_steps = 0;  // x holds this cycle's steps
   if constexpr (sizeof(R) == 4) {
     constexpr int K = pow2_at_least(2 * NV);
     DF v[K];
@@ -325,18 +314,17 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
   }
 }
 
-// x += α u_0 + Σ γ_k r_{k−1} ; r_0 −= Σ γ_k r_k ; u_0 −= Σ γ_k u_k ; then
-// (r̂, r_0) and ‖r_0‖² → FIN_BL_CYCLE.  α u_0 and the r_i −= α u_{i+1}
-// (i < L−1) are the last BiCG step's deferred updates (α of that step:
-// nothing writes sc->alpha between it and this kernel).
+// The replayed steps (complex64; k_bl_gram has stored them in complex128),
+// then x += Σ γ_k r_{k−1} ; r_0 −= Σ γ_k r_k ;
+// u_0 −= Σ γ_k u_k ; then (r̂, r_0) and ‖r_0‖² → FIN_BL_CYCLE.
 template <typename R, int L>
 __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u,
                                                   typename CT<R>::C *x, long long n, RedBuf red, KScalars *sc) {
   using C = typename CT<R>::C;
   if (sc->done) return;
-  C cs[L + 1];
-  scalars<R>([&](int i) { return i < L ? sc->gam[i] : sc->alpha; }, cs);
-  const C al = cs[L];
+  C cs[L + Hist<L>::N];
+  scalars<R>([&](int i) { return i < L ? sc->gam[i] : Hist<L>::at(sc, i - L); }, cs);
+  const C *hist = cs + L;
   Acc<R> a0r, a0i, a1;
   visit<R>(
       n,
@@ -352,13 +340,10 @@ __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<type
         }
         Pair<C> xv = ldp(x, q);
         const Pair<C> hv{shadow<R>(2 * q), shadow<R>(2 * q + 1)};
-#pragma unroll
-        for (int k = 0; k + 1 < L; ++k) {
-          ra[k] = csub(ra[k], cmul(al, ua[k + 1]));
-          rb[k] = csub(rb[k], cmul(al, ub[k + 1]));
+        if (sizeof(R) == 4) {
+          replay<L, true>(ra, ua, xv.a, hist);
+          replay<L, true>(rb, ub, xv.b, hist);
         }
-        xv.a = cadd(xv.a, cmul(al, ua[0]));
-        xv.b = cadd(xv.b, cmul(al, ub[0]));
         C r0a = ra[0], r0b = rb[0], u0a = ua[0], u0b = ub[0];
 #pragma unroll
         for (int k = 1; k <= L; ++k) {
@@ -384,9 +369,9 @@ __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<type
           rk[k] = r.v[k][e];
           uk[k] = u.v[k][e];
         }
-#pragma unroll
-        for (int k = 0; k + 1 < L; ++k) rk[k] = csub(rk[k], cmul(al, uk[k + 1]));
-        C xe = cadd(x[e], cmul(al, uk[0])), r0 = rk[0], u0 = uk[0];
+        C xe = x[e];
+        if (sizeof(R) == 4) replay<L, true>(rk, uk, xe, hist);
+        C r0 = rk[0], u0 = uk[0];
 #pragma unroll
         for (int k = 1; k <= L; ++k) {
           xe = cadd(xe, cmul(cs[k - 1], rk[k - 1]));
@@ -402,6 +387,35 @@ __global__ void __launch_bounds__(VB, sizeof(R) == 4 ? 3 : 2) k_bl_fin(VSet<type
         a1.add(r0.x * r0.x + r0.y * r0.y);
       });
   sum_finalise<VB>(a0r, a0i, a1, red, FIN_BL_CYCLE, sc);
+}
+
+// A cycle that broke down after `steps` completed BiCG steps: x += Σ α_j u_0
+// over them (replay() cut short), so that the restart keeps their progress.
+template <typename R>
+__global__ void __launch_bounds__(VB) k_bl_fold(VSet<typename CT<R>::C> r, VSet<typename CT<R>::C> u,
+                                                typename CT<R>::C *x, long long n, int steps, const KScalars *sc) {
+  using C = typename CT<R>::C;
+  for (long long e = blockIdx.x * (long long)VB + threadIdx.x; e < n; e += (long long)gridDim.x * VB) {
+    C rv[LMAX], uv[LMAX];
+#pragma unroll
+    for (int i = 0; i < LMAX; ++i)
+      if (i < steps) {
+        rv[i] = r.v[i][e];
+        uv[i] = u.v[i][e];
+      }
+    C xe = cadd(x[e], cmul(tocr<R>(sc->alpha_j[0]), uv[0]));
+#pragma unroll
+    for (int j = 1; j < LMAX; ++j)
+      if (j < steps) {
+        const C al = tocr<R>(sc->alpha_j[j]), be = tocr<R>(sc->beta_j[j]);
+#pragma unroll
+        for (int i = 0; i < j; ++i) uv[i] = csub(rv[i], cmul(be, uv[i]));
+        xe = cadd(xe, cmul(al, uv[0]));
+#pragma unroll
+        for (int i = 0; i < j; ++i) rv[i] = csub(rv[i], cmul(al, uv[i + 1]));
+      }
+    x[e] = xe;
+  }
 }
 
 // (r̂, r_0) with the generated shadow vector: FIN_BL_REDO after a replaced
@@ -476,21 +490,11 @@ static int bl_cycle_t(fdfd_handle *h, typename CT<R>::C *x, typename CT<R>::C *c
   constexpr int NOCAP = 1 << 30;
   int rc;
   for (int j = 0; j < L; ++j) {
-    switch (j) {
-      case 0: launch_wave(h, k_bl_u<R, 0>, NOCAP, rs, us, x, n, (const KScalars *)sc); break;
-      case 1: launch_wave(h, k_bl_u<R, 1>, NOCAP, rs, us, x, n, (const KScalars *)sc); break;
-      case 2: launch_wave(h, k_bl_u<R, 2>, NOCAP, rs, us, x, n, (const KScalars *)sc); break;
-      default: launch_wave(h, k_bl_u<R, 3>, NOCAP, rs, us, x, n, (const KScalars *)sc); break;
-    }
-    if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_u"))) return rc;
+    launch_wave(h, k_bl_step<R>, NOCAP, (const typename CT<R>::C *)r[j], (const typename CT<R>::C *)u[j], u[j], n, 1, j, sc);
+    if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_step"))) return rc;
     if ((rc = launch_apply_fin<R>(h, u[j], u[j + 1], EPI_DOT_SHD, nullptr, FIN_ALPHA, sc, tr))) return rc;
-    switch (j) {
-      case 0: launch_wave(h, k_bl_r<R, 0>, NOCAP, rs, us, n, (const KScalars *)sc); break;
-      case 1: launch_wave(h, k_bl_r<R, 1>, NOCAP, rs, us, n, (const KScalars *)sc); break;
-      case 2: launch_wave(h, k_bl_r<R, 2>, NOCAP, rs, us, n, (const KScalars *)sc); break;
-      default: launch_wave(h, k_bl_r<R, 3>, NOCAP, rs, us, n, (const KScalars *)sc); break;
-    }
-    if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_r"))) return rc;
+    launch_wave(h, k_bl_step<R>, NOCAP, (const typename CT<R>::C *)r[j], (const typename CT<R>::C *)u[j + 1], r[j], n, 0, j, sc);
+    if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_step"))) return rc;
     if (j + 1 < L) rc = launch_apply_fin<R>(h, r[j], r[j + 1], EPI_DOT_SHD, nullptr, FIN_BL_RHO, sc, tr);
     else rc = launch_apply_fin<R>(h, r[j], r[j + 1], EPI_STORE, nullptr, FIN_NONE, sc, tr);
     if (rc) return rc;
@@ -498,7 +502,7 @@ static int bl_cycle_t(fdfd_handle *h, typename CT<R>::C *x, typename CT<R>::C *c
   // the reducing kernels keep ≤ RED_BLOCKS blocks: 8·RED_BLOCKS partial
   // slots hold the Gram matrix's L(L+1)/2 + L ≤ 14 values per block
   if ((rc = ensure_red(h, 8 * RED_BLOCKS))) return rc;
-  launch_wave(h, k_bl_gram<R, L>, red_cap(n), rs, us, n, h->red, sc);
+  launch_wave(h, k_bl_gram<R, L>, red_cap(n), rs, us, x, n, h->red, sc);
   if ((rc = cuda_check(h, cudaGetLastError(), "k_bl_gram"))) return rc;
   launch_wave(h, k_bl_fin<R, L>, red_cap(n), rs, us, x, n, h->red, sc);
   return cuda_check(h, cudaGetLastError(), "k_bl_fin");
@@ -517,6 +521,17 @@ int bl_cycle(fdfd_handle *h, typename CT<R>::C *x, typename CT<R>::C *const *r, 
   return set_error(h, FDFD_ERR_ARG, "BiCGStab(l) needs 1 <= l <= 4");
 }
 
+// Fold the completed steps of a broken-down cycle into x (see k_bl_fold).
+template <typename R>
+int bl_fold(fdfd_handle *h, typename CT<R>::C *x, typename CT<R>::C *const *r, typename CT<R>::C *const *u, long long n,
+            int ell, int steps, KScalars *sc) {
+  if (steps < 1) return FDFD_OK;
+  steps = std::min(steps, ell);
+  k_bl_fold<R><<<RED_BLOCKS, VB, 0, h->stream>>>(vset<R>(r, ell + 1), vset<R>(u, ell + 1), x, n, steps, sc);
+  h->launches++;
+  return cuda_check(h, cudaGetLastError(), "k_bl_fold");
+}
+
 template <typename R>
 int bl_redo(fdfd_handle *h, const typename CT<R>::C *r0, long long n, int fin, KScalars *sc) {
   int rc = ensure_red(h, RED_BLOCKS);
@@ -530,6 +545,9 @@ template int bl_cycle<float>(fdfd_handle *, float2 *, float2 *const *, float2 *c
                              bool);
 template int bl_cycle<double>(fdfd_handle *, double2 *, double2 *const *, double2 *const *, long long, int,
                               KScalars *, bool);
+template int bl_fold<float>(fdfd_handle *, float2 *, float2 *const *, float2 *const *, long long, int, int, KScalars *);
+template int bl_fold<double>(fdfd_handle *, double2 *, double2 *const *, double2 *const *, long long, int, int,
+                             KScalars *);
 template int bl_redo<float>(fdfd_handle *, const float2 *, long long, int, KScalars *);
 template int bl_redo<double>(fdfd_handle *, const double2 *, long long, int, KScalars *);
 

@@ -108,6 +108,8 @@ struct KScalars {
   // x += Σ γ_k r_{k−1}, r₀ −= Σ γ_k r_k, u₀ −= Σ γ_k u_k
   double2 rho_pre;
   double2 gam[4];
+  double2 alpha_j[4], beta_j[4];  // α and β of the current cycle's steps
+  int bl_steps;                   // steps of the current cycle whose α is applied
 };
 
 struct Workspace;  // solver vectors (solver.cu)

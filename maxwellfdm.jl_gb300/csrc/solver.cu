@@ -58,6 +58,9 @@ int bl_cycle(fdfd_handle *, typename CT<R>::C *, typename CT<R>::C *const *, typ
              int, KScalars *, bool);
 template <typename R>
 int bl_redo(fdfd_handle *, const typename CT<R>::C *, long long, int, KScalars *);
+template <typename R>
+int bl_fold(fdfd_handle *, typename CT<R>::C *, typename CT<R>::C *const *, typename CT<R>::C *const *, long long, int,
+            int, KScalars *);
 
 #define TRY(x)              \
   do {                      \
@@ -241,16 +244,21 @@ static int cocg_iter(fdfd_handle *h, Workspace *ws, bool tr) {
   return FDFD_OK;
 }
 
-// One BiCGStab(ℓ) cycle.  Vectors: 0 x (correction), 2 … 2+ℓ r_0 … r_ℓ,
-// 3+ℓ … 3+2ℓ u_0 … u_ℓ (slot 1 unused: r̂ is generated).
+// BiCGStab(ℓ) vectors: 0 x (correction), 2 … 2+ℓ r_0 … r_ℓ, 3+ℓ … 3+2ℓ
+// u_0 … u_ℓ (slot 1 unused: r̂ is generated).
 template <typename R>
-static int bl_iter(fdfd_handle *h, Workspace *ws, int ell, bool tr) {
-  using C = typename CT<R>::C;
-  C *r[5], *u[5];
+static void bl_vecs(Workspace *ws, int ell, typename CT<R>::C **r, typename CT<R>::C **u) {
   for (int i = 0; i <= ell; ++i) {
     r[i] = vec<R>(ws, 2 + i);
     u[i] = vec<R>(ws, 3 + ell + i);
   }
+}
+
+// One BiCGStab(ℓ) cycle.
+template <typename R>
+static int bl_iter(fdfd_handle *h, Workspace *ws, int ell, bool tr) {
+  typename CT<R>::C *r[5], *u[5];
+  bl_vecs<R>(ws, ell, r, u);
   return bl_cycle<R>(h, vec<R>(ws, 0), r, u, ws->n, ell, ws->sc, tr);
 }
 
@@ -482,6 +490,12 @@ struct Solve {
         status = FDFD_ERR_NONFINITE;
         done = true;
         return FDFD_OK;
+      }
+      // a cycle of BiCGStab(ℓ) that broke down: its completed steps' x updates
+      if (hs.reason == 3 && o.method == FDFD_BICGSTABL) {
+        typename CT<R>::C *rv[5], *uv[5];
+        bl_vecs<R>(ws, ell, rv, uv);
+        TRY(bl_fold<R>(h, vec<R>(ws, 0), rv, uv, n, ell, hs.bl_steps, ws->sc));
       }
       // fold the correction into x64 and recompute the true residual
       if constexpr (sizeof(R) == 4) TRY(accum(h, ws->x64, vec<R>(ws, 0), n));

@@ -159,3 +159,20 @@ def test_residual_norm(pkg, oracle, N):
     ref = np.linalg.norm(r.cpu().numpy()) ** 2
     assert abs(rr - ref) <= 1e-13 * ref
     A.close()
+
+
+@pytest.mark.parametrize("ell", [1, 2, 4])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_exact_after_one_step(pkg, oracle, precision, ell):
+    """A right-hand side on a pinned wall DOF only (its row of A is
+    −ω²ε alone): the first BiCG step solves it exactly and the second breaks
+    down (A u = 0); the completed step's update of x must survive that."""
+    g = oracle.uniform_grid((6, 5, 4))
+    om = 0.5  # −ω² = −1/4: every product of the step is exact
+    S = oracle.System(g, om, ((0, 0, 0), (0, 0, 0)), [])
+    A = _op(pkg, S)
+    b = np.zeros(A.n, complex)
+    b[1 + 3 * (0 + 6 * (2 + 5 * 1))] = 1.0  # E_y at i = 0
+    x, st = A.solve(b, tol=1e-10, precision=precision, ell=ell)
+    assert np.linalg.norm(b - S.A @ x) <= 1e-10, st
+    A.close()
