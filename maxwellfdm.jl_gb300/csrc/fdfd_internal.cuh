@@ -209,7 +209,7 @@ int launch_apply_fin(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>:
 // does not serve the call (the caller then uses the first one)
 template <typename R>
 int launch_apply_v2(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y, int epi,
-                    const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc);
+                    const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc, bool tma);
 // number of blocks launch_apply uses (reduction buffer sizing)
 int apply_blocks(const fdfd_handle *h);
 // pick the z-chunk length per precision by timing (stencil.cu)

@@ -30,9 +30,10 @@
 //   * off-diagonal ε (only where the 32×8 tile-plane flag is set): each
 //     thread forms the corner terms at its own corner from registers and
 //     shuffles and averages the two corners around each output.
-// It serves the forward operator on PEC walls with 16-byte aligned inputs;
+// It serves the forward operator; where TMA cannot (odd Nx in complex64,
+// periodic axes) k_apply_cp runs the same march on a ring filled by cp.async;
 // the first TMA kernel (stencil.cu) keeps the S-weighted COCG epilogue and
-// the plain-load kernel Bloch phases and Aᵀ.
+// the plain-load kernel Aᵀ.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -48,7 +49,7 @@ namespace fdfd {
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_encode_fn();
 
-template <typename R, int RW, int NS, bool EDR = true>
+template <typename R, int RW, int NS, bool EDR = true, bool EOR = true>
 struct V2 {
   using C = typename CT<R>::C;
   static constexpr int NW = 8;          // warps per CTA, RW rows each
@@ -75,7 +76,7 @@ struct V2 {
   // i0 … i0+EOX−1, j0 … j0+TYT, laid out [pair][jj][ii] (EOX·4 bytes a
   // multiple of 16); complex128 reads them from global memory
   static constexpr int EOX = TX + 4, EOY = TYT + 1;
-  static constexpr int EO_BYTES = sizeof(R) == 4 ? EOX * EOY * 3 * (int)sizeof(R) : 0;
+  static constexpr int EO_BYTES = (EOR && sizeof(R) == 4) ? EOX * EOY * 3 * (int)sizeof(R) : 0;
   static constexpr int EO_SLOT = (EO_BYTES + 127) / 128 * 128;
   static constexpr int EO_OFF = NS * SLOT;
   // complex64: a ring slot per plane for the ε diagonal of the tile's cells,
@@ -184,20 +185,31 @@ struct Accs2 {
   ShortAcc<R> r0, i0, r1;
 };
 
-template <typename R>
+template <typename R, bool BL>
 __device__ __forceinline__ R eoff_at(const OpArgs<R> &a, int p, int gi, int gj, int gk) {
-  // off-diagonal pair p at corner (gi, gj, gk); PEC ghost corners (index N) are 0
+  // off-diagonal pair p at corner (gi, gj, gk); PEC ghost corners (index N)
+  // are 0, ghosts of a periodic axis its corner 0
+  if (BL) {
+    if (gi == a.N[0] && a.bloch[0]) gi = 0;
+    if (gj == a.N[1] && a.bloch[1]) gj = 0;
+    if (gk == a.N[2] && a.bloch[2]) gk = 0;
+  }
   if (gi >= a.N[0] || gj >= a.N[1] || gk >= a.N[2]) return R(0);
   return __ldg(&a.eoff[(long long)p * a.ncell + gi + (long long)a.N[0] * (gj + (long long)a.N[1] * gk)]);
 }
 
-template <typename R, int EPI, int RW, int NS, int MB, bool EDR>
-__global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
-    k_apply_v2(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap emap,
-               const __grid_constant__ CUtensorMap dmap, OpArgs<R> a,
-               Extra<R> ex, const typename CT<R>::C *__restrict__ x, typename CT<R>::C *__restrict__ y,
-               const typename CT<R>::C *__restrict__ aux0, RedBuf red, int fin, KScalars *sc, int *errflag) {
-  using G = V2<R, RW, NS, EDR>;
+// The kernel's body.  CPA = false: the ring is filled by TMA (tmap, emap,
+// dmap) on PEC walls.  CPA = true: by cp.async from every thread, one group
+// per plane, which serves what TMA cannot — an x pitch that is no multiple
+// of 16 bytes (complex64 with odd Nx) and periodic axes, whose ghost cells
+// are the wrapped ones times the Bloch phase.
+template <typename R, int EPI, int RW, int NS, bool EDR, bool CPA>
+__device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensorMap &emap, const CUtensorMap &dmap,
+                                         const OpArgs<R> &a, const Extra<R> &ex,
+                                         const typename CT<R>::C *__restrict__ x, typename CT<R>::C *__restrict__ y,
+                                         const typename CT<R>::C *__restrict__ aux0, RedBuf red, int fin, KScalars *sc,
+                                         int *errflag) {
+  using G = V2<R, RW, NS, EDR, !CPA>;
   using C = typename CT<R>::C;
   using X = typename G::Exch;
   constexpr int NW = G::NW, TYT = G::TYT, KC2 = G::KC2;
@@ -233,16 +245,18 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
   const int cx = 6 * (i0 - G::XOFF), cy = j0 - 1;
   const int jw = RW * w;  // the warp's first tile row
   const int tiles_yr = (a.N[1] + RW - 1) / RW;
+  // periodic axes (only the cp.async ring serves them)
+  const bool bx_ = CPA && a.bloch[0], by_ = CPA && a.bloch[1], bz_ = CPA && a.bloch[2];
   const bool ering = G::EO_SLOT > 0 && ex.eoff_tma != 0;
   const bool edr = G::ED_SLOT > 0 && ex.ediag_tma != 0;
 
   // TMA destinations need 128-byte alignment; the declared alignment gives
   // it, checked here once (every thread returns together, before any copy)
-  if ((smem_u32(sm) & 127u) != 0u) {
+  if (!CPA && (smem_u32(sm) & 127u) != 0u) {
     if (tid == 0) atomicExch(errflag, 2);
     return;
   }
-  if (tid == 0) {
+  if (!CPA && tid == 0) {
     for (int s = 0; s < NS; ++s) mbar_init(smem_u32(&bars[s]), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmap)) : "memory");
@@ -251,10 +265,93 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
   }
   pdl_wait();
   if (sc != nullptr && sc->done) return;  // every thread, before any copy is issued
+  // cp.async ring: the warp's rows of a plane's box (rows j0−1 … j0+TYT; the
+  // warps 0-3 carry the halo jobs below, so the rows left over go to the
+  // last warps).  A complex64 row whose pitch is a multiple of 16 bytes goes
+  // in 16-byte copies from column i0−2 on, any other row element by element
+  // from column i0−1; cof: per copy of the lane, its offset in the row
+  // (wrapped on a periodic axis), or −1 outside the grid (filled with 0).
+  constexpr int NCOPY = 4;
+  const bool vec = CPA && sizeof(C) == 8 && (a.N[0] & 1) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const int row3 = 3 * a.N[0];
+  int cof[NCOPY];
+  // Bloch phases other than 1, applied to the wrapped cells once landed
+  bool phx = false, phy = false, phz = false;
+  if constexpr (CPA) {
+#pragma unroll
+    for (int n = 0; n < NCOPY; ++n) {
+      const int t = lane + 32 * n;
+      int off = vec ? 3 * (i0 - 2) + 2 * t : 3 * (i0 - 1) + t;
+      if (off < 0) off = bx_ ? off + row3 : -1;
+      else if (off >= row3) off = (bx_ && off < row3 + 3) ? off - row3 : -1;
+      if (off < 0 || off >= row3 || t >= (vec ? 3 * (TX + 4) / 2 : 3 * (TX + 2))) off = -1;
+      cof[n] = off;
+    }
+    phx = bx_ && (ex.ph[0].x != R(1) || ex.ph[0].y != R(0));
+    phy = by_ && (ex.ph[1].x != R(1) || ex.ph[1].y != R(0));
+    phz = bz_ && (ex.ph[2].x != R(1) || ex.ph[2].y != R(0));
+  }
+  auto copy_plane = [&](int q, int s) {
+    const bool zout = q < 0 || q >= a.N[2];
+    const int gq = q < 0 ? q + a.N[2] : q >= a.N[2] ? q - a.N[2] : q;
+    for (int r = NW - 1 - w; r < G::BY; r += NW) {
+      int gj = j0 + r - 1;
+      bool ok = !zout || bz_;
+      if (gj < 0) {
+        ok = ok && by_;
+        gj += a.N[1];
+      } else if (gj >= a.N[1]) {
+        ok = ok && by_ && gj == a.N[1];
+        gj -= a.N[1];
+      }
+      const C *src = x + (ok ? row3 * (gj + a.N[1] * gq) : 0);
+      const uint32_t dst = smem_u32(sm + s * G::SLOT) + r * (G::XW * 3 * (int)sizeof(C));
+      if (vec) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          const bool in = ok && cof[n] >= 0;
+          if (lane + 32 * n < 3 * (TX + 4) / 2) cp_async<16>(dst + (lane + 32 * n) * 16, src + (in ? cof[n] : 0), in);
+        }
+      } else {
+#pragma unroll
+        for (int n = 0; n < NCOPY; ++n) {
+          const bool in = ok && cof[n] >= 0;
+          if (lane + 32 * n < 3 * (TX + 2))
+            cp_async<sizeof(C)>(dst + ((G::XOFF - 1) * 3 + lane + 32 * n) * (int)sizeof(C), src + (in ? cof[n] : 0), in);
+        }
+      }
+    }
+  };
+  // multiply the wrapped cells of a landed plane by their Bloch phases (the
+  // warp's own rows, so only the warp has to have seen its copies land)
+  auto phase_plane = [&](int q, int s) {
+    __syncwarp();
+    const bool zw = phz && (q < 0 || q >= a.N[2]);
+    for (int r = NW - 1 - w; r < G::BY; r += NW) {
+      const int gj = j0 + r - 1;
+      const bool yw = phy && (gj < 0 || gj >= a.N[1]);
+      C *row = reinterpret_cast<C *>(sm + s * G::SLOT) + (r * G::XW + G::XOFF - 1) * 3;
+      if (zw || yw) {
+        C p = zw ? (q < 0 ? ex.phinv[2] : ex.ph[2]) : mk(R(1), R(0));
+        if (yw) p = cmul(p, gj < 0 ? ex.phinv[1] : ex.ph[1]);
+        for (int e = lane; e < 3 * (TX + 2); e += 32) row[e] = cmul(row[e], p);
+        __syncwarp();
+      }
+      if (phx && lane < 6) {  // column −1 of the first tile, column N_x of the last
+        const int e = lane < 3 ? lane : 3 * (a.N[0] - i0 + 1) + lane - 3;
+        if (lane < 3 ? i0 == 0 : e < 3 * (TX + 2)) row[e] = cmul(row[e], lane < 3 ? ex.phinv[0] : ex.ph[0]);
+      }
+    }
+  };
   // the first planes' E tiles go out now, so their latency overlaps the
   // coefficient tables below; each slot's single arrival (and its ε tiles,
   // which need the off-diagonal flags) follows once the tables are in place
-  if (tid == 0) {
+  if constexpr (CPA) {
+    for (int p = 0; p < NS; ++p) {
+      if (kfirst + p <= k1) copy_plane(kfirst + p, p);
+      cp_async_commit();
+    }
+  } else if (tid == 0) {
     for (int p = 0; p < NS; ++p) {
       const int q = kfirst + p;
       if (q <= k1) {
@@ -294,7 +391,10 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
       unsigned char any = 0;
 #pragma unroll
       for (int s = 0; s < NW; ++s) {
-        const int tr = j0 / RW + s;
+        int tr = j0 / RW + s;
+        // periodic y: the strip past the last row forms the corner terms of
+        // row N_y (corner row 0) for the last strip's outputs
+        if (CPA && by_ && tr * RW == a.N[1]) --tr;
         unsigned char f = 0;
         if (a.eoff != nullptr && q >= 0 && q < a.N[2] && tr < tiles_yr) {
           if (ex.oflag_w != nullptr) f = ex.oflag_w[(bx + (long long)tiles_x * tr) * a.N[2] + q];
@@ -332,7 +432,7 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
     if (edr) tma_copy4d(smem_u32(sm + G::ED_OFF + s * G::ED_SLOT), &dmap, i0, j0, q, 0, bar);
     mbar_arrive(bar);
   };
-  if (tid == 0) {
+  if (!CPA && tid == 0) {
     for (int p = 0; p < NS; ++p) {
       const int q = kfirst + p;
       if (q <= k1) issue(q, p, false);
@@ -342,7 +442,7 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
   // (plane gk): the ε ring, or global memory
   auto eps_off = [&](int s, int p, int jj, int ii, int gk) -> R {
     if (ering) return reinterpret_cast<const R *>(sm + G::EO_OFF + s * G::EO_SLOT)[(p * G::EOY + jj) * G::EOX + ii];
-    return eoff_at(a, p, i0 + ii, j0 + jj, gk);
+    return eoff_at<R, CPA>(a, p, i0 + ii, j0 + jj, gk);
   };
 
   Accs2<R> acc;
@@ -356,9 +456,18 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
   // run without the pin selects.
   auto march = [&](auto wall_tag) {
     constexpr bool WALL = decltype(wall_tag)::value;
-    bool ok = mbar_wait_sleep(smem_u32(&bars[0]), 0, ex.wait_limit, 100000u);
-    ok = ok && mbar_wait_sleep(smem_u32(&bars[1]), 0, ex.wait_limit, 100000u);
-    const bool pin_i = WALL && gi == 0;  // PEC x wall: E_y, E_z at i = 0 are pinned
+    bool ok = true;
+    if constexpr (CPA) {
+      // planes k0−1 … k0+1 have landed (the newest group may be in flight)
+      cp_async_wait<1>();
+      if (phx || phy || phz)
+        for (int p = 0; p < 3; ++p) phase_plane(kfirst + p, p);
+      __syncthreads();
+    } else {
+      ok = mbar_wait_sleep(smem_u32(&bars[0]), 0, ex.wait_limit, 100000u);
+      ok = ok && mbar_wait_sleep(smem_u32(&bars[1]), 0, ex.wait_limit, 100000u);
+    }
+    const bool pin_i = WALL && gi == 0 && !bx_;  // PEC x wall: E_y, E_z at i = 0 are pinned
     C eo[RW][3];         // E(k), pinned DOFs zeroed
     C od[RW][3];         // off-diagonal ε terms of plane k (½ of each corner around an output)
     C hxp[RW], hyp[RW];  // H_x, H_y at k−1
@@ -370,13 +479,13 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
 #pragma unroll
     for (int r = 0; r < RW; ++r) {
       const int gj = j0 + jw + r;
-      pin_j[r] = WALL && gj == 0;
+      pin_j[r] = WALL && gj == 0 && !by_;
       act[r] = gi < a.N[0] && gj < a.N[1];
       cell[r] = gi + a.N[0] * gj + plane * k0;
       zcn[r] = czero<C>();
     }
     {
-      const bool zpin0 = WALL && k0 == 0, zpinm = WALL && kfirst == 0;
+      const bool zpin0 = WALL && k0 == 0 && !bz_, zpinm = WALL && kfirst == 0 && !bz_;
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
         const int jj = jw + r;
@@ -401,7 +510,7 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
         ezp[r] = mz;
       }
     }
-    run = !__syncthreads_or(!ok);
+    if (!CPA) run = !__syncthreads_or(!ok);
 
     // ring slots of planes k−1, k, k+1 and the phase parity expected next in
     // each slot, advanced without divisions
@@ -410,7 +519,7 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
     for (int k = k0; run && k < k1; ++k) {
       const int p0 = k - kfirst;
       X &xc_ = xch[k & 1];
-      const bool z0 = WALL && k == 0;
+      const bool z0 = WALL && k == 0 && !bz_;
       // diagonal ε (when it does not come through the ring) and the epilogue
       // operand at plane k: their latency overlaps this plane's curls
       R epk[RW][3];
@@ -433,8 +542,10 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
           }
         }
       }
-      ok = mbar_wait_sleep(smem_u32(&bars[s1]), (phase >> s1) & 1u, ex.wait_limit, 100000u);
-      phase ^= 1u << s1;
+      if (!CPA) {
+        ok = mbar_wait_sleep(smem_u32(&bars[s1]), (phase >> s1) & 1u, ex.wait_limit, 100000u);
+        phase ^= 1u << s1;
+      }
       const C cmz = zt[p0], cez = zt[KC2 + p0];
       const bool rc = rx && ry && k >= a.rlo[2] && k <= a.rhi[2];
       // E(k+1) at the thread's cells (true values; the curls take the pinned
@@ -488,7 +599,7 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
       } else if (w == 1 && lane < TYT) {
         // column i0−1, tile row `lane` (reaches only pinned outputs when i0 = 0)
         const int jj = lane;
-        const bool pj = WALL && j0 + jj == 0, pi0 = WALL && i0 == 0;
+        const bool pj = WALL && j0 + jj == 0 && !by_, pi0 = WALL && i0 == 0 && !bx_;
         const C cmy = yt[jj + 1], cmh = xt[0];
         const C ex_k = zif(pj || z0, ev2<R, RW, NS>(sm, s0, 0, jj, -1));
         const C ex_k1 = zif(pj, ev2<R, RW, NS>(sm, s1, 0, jj, -1));
@@ -567,7 +678,7 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
       if (w == 2 && lane < TYT && zf[p0 * NW + lane / RW]) {
         // x-directed corner terms at column i0+32, tile row `lane`
         const int jj = lane;
-        const bool pj = WALL && j0 + jj == 0;
+        const bool pj = WALL && j0 + jj == 0 && !by_;
         const C wmy = yt[2 * (TYT + 2) + jj + 1], wpy = yt[3 * (TYT + 2) + jj + 1];
         const C eym = zif(z0, ev2<R, RW, NS>(sm, s0, 1, jj - 1, TX));
         const C ey0 = zif(z0, ev2<R, RW, NS>(sm, s0, 1, jj, TX));
@@ -589,13 +700,19 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
       }
       // ---- all H(k) and corner terms written; planes k and k+1 no longer
       // read after this plane, plane k−1 not at all
-      if (__syncthreads_or(!ok)) {
+      if constexpr (CPA) {
+        cp_async_wait<0>();  // plane k+2 has landed; every thread sees it after the barrier
+        if ((phx || phy || phz) && k + 2 <= k1) phase_plane(k + 2, s1 + 1 == NS ? 0 : s1 + 1);
+        __syncthreads();
+        if (k - 1 + NS <= k1) copy_plane(k - 1 + NS, sm1);
+        cp_async_commit();
+      } else if (__syncthreads_or(!ok)) {
         run = false;
         kstop = k;
         break;
       }
       // the refill goes out from the last warp, which has no halo job
-      if (tid == G::NT - 32) {
+      if (!CPA && tid == G::NT - 32) {
         const int q = k - 1 + NS;  // the plane that takes plane k−1's slot
         if (q <= k1) {
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -719,7 +836,8 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
   if (i0 == 0 || j0 == 0 || k0 <= 1) march(std::true_type{});
   else march(std::false_type{});
 
-  if (!run) {
+  if (CPA) cp_async_wait<0>();
+  if (!CPA && !run) {
     // a bounded wait gave up: report it and wait (with the full limit) for
     // the last copy issued into each slot — planes up to min(k1, kstop+NS−2),
     // plane q in slot (q − kfirst) mod NS as phase (q − kfirst) / NS — so no
@@ -733,6 +851,23 @@ __global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
   }
   __syncthreads();
   if (EPI != EPI_STORE) sum_finalise<G::NT>(acc.r0, acc.i0, acc.r1, red, fin, sc);
+}
+
+template <typename R, int EPI, int RW, int NS, int MB, bool EDR>
+__global__ void __launch_bounds__(V2<R, RW, NS, EDR>::NT, MB)
+    k_apply_v2(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap emap,
+               const __grid_constant__ CUtensorMap dmap, OpArgs<R> a,
+               Extra<R> ex, const typename CT<R>::C *__restrict__ x, typename CT<R>::C *__restrict__ y,
+               const typename CT<R>::C *__restrict__ aux0, RedBuf red, int fin, KScalars *sc, int *errflag) {
+  apply_v2<R, EPI, RW, NS, EDR, false>(tmap, emap, dmap, a, ex, x, y, aux0, red, fin, sc, errflag);
+}
+
+template <typename R, int EPI, int RW, int NS, int MB>
+__global__ void __launch_bounds__(V2<R, RW, NS, false, false>::NT, MB)
+    k_apply_cp(OpArgs<R> a, Extra<R> ex, const typename CT<R>::C *__restrict__ x, typename CT<R>::C *__restrict__ y,
+               const typename CT<R>::C *__restrict__ aux0, RedBuf red, int fin, KScalars *sc) {
+  apply_v2<R, EPI, RW, NS, false, true>(CUtensorMap{}, CUtensorMap{}, CUtensorMap{}, a, ex, x, y, aux0, red, fin, sc,
+                                        nullptr);
 }
 
 // ------------------------------------------------------------------ host
@@ -827,6 +962,52 @@ static int launch_v2_t(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R
   return cuda_check(h, e, "k_apply_v2 launch");
 }
 
+// The cp.async form, for any Nx, alignment of x and periodic axes.
+template <typename R, int EPI, int RW, int NS, int MB>
+static int launch_cp_t(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y,
+                       const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc) {
+  using G = V2<R, RW, NS, false, false>;
+  Extra<R> ex = make_extra<R>(h);
+  ex.kchunk = kc;
+  dim3 grid((h->N[0] + TX - 1) / TX, (h->N[1] + G::TYT - 1) / G::TYT, (h->N[2] + kc - 1) / kc);
+  const int p = sizeof(R) == 4 ? 1 : 0;
+  if (h->nwork[p] > 0) {
+    ex.work = h->work[p];
+    grid = dim3((unsigned)h->nwork[p], 1, 1);
+  }
+  if (EPI != EPI_STORE) {
+    int rc = ensure_red(h, (int)(grid.x * grid.y * grid.z));
+    if (rc) return rc;
+  }
+  static DevFlags attr;
+  if (!attr.done(h->dev)) {
+    cudaError_t e = cudaFuncSetAttribute(k_apply_cp<R, EPI, RW, NS, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         G::SMEM);
+    if (e != cudaSuccess) return cuda_check(h, e, "cudaFuncSetAttribute(k_apply_cp)");
+    e = cudaFuncSetAttribute(k_apply_cp<R, EPI, RW, NS, MB>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                             cudaSharedmemCarveoutMaxShared);
+    if (e != cudaSuccess) return cuda_check(h, e, "cudaFuncSetAttribute(carveout)");
+    attr.set(h->dev);
+  }
+  ex.oflag_w = h->has_off ? h->oflag_rows[RW - 1] : nullptr;
+  const OpArgs<R> a = op_args<R>(h);
+  const cudaError_t e = launch_k(h, k_apply_cp<R, EPI, RW, NS, MB>, grid, dim3(G::NT, 1, 1), (size_t)G::SMEM, a, ex, x,
+                                 y, aux0, h->red, fin, sc);
+  h->launches++;
+  return cuda_check(h, e, "k_apply_cp launch");
+}
+
+template <typename R, int EPI>
+static int launch_cp_e(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y,
+                       const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc) {
+  if constexpr (sizeof(R) == 8) {
+    return launch_cp_t<R, EPI, 1, 4, 2>(h, x, y, aux0, fin, sc, kc);
+  } else {
+    if (h->op_variant == 1 || h->op_variant == 3) return launch_cp_t<R, EPI, 1, 4, 2>(h, x, y, aux0, fin, sc, kc);
+    return launch_cp_t<R, EPI, 2, 4, 2>(h, x, y, aux0, fin, sc, kc);
+  }
+}
+
 template <typename R, int EPI>
 static int launch_v2_e(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y,
                        const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc) {
@@ -842,24 +1023,33 @@ static int launch_v2_e(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R
   }
 }
 
-// Launch through the second TMA kernel when it serves the call; returns
-// FDFD_ERR_UNSUPPORTED (without touching the error string) when it does not.
+template <typename R, int EPI>
+static int launch_any_e(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y,
+                        const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc, bool tma) {
+  return tma ? launch_v2_e<R, EPI>(h, x, y, aux0, fin, sc, kc) : launch_cp_e<R, EPI>(h, x, y, aux0, fin, sc, kc);
+}
+
+// Launch through the second operator kernel when it serves the call (tma:
+// in its TMA form, which needs PEC walls and 16-byte pitches; else with the
+// cp.async ring); returns FDFD_ERR_UNSUPPORTED (without touching the error
+// string) when it does not.
 template <typename R>
 int launch_apply_v2(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y, int epi,
-                    const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc) {
+                    const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc, bool tma) {
   // cell offsets are 32-bit in the kernel
   if (h->op_variant == 0 || 3 * h->ncell >= (1ll << 31)) return FDFD_ERR_UNSUPPORTED;
   switch (epi) {
-    case EPI_STORE: return launch_v2_e<R, EPI_STORE>(h, x, y, aux0, fin, sc, kc);
-    case EPI_RESID: return launch_v2_e<R, EPI_RESID>(h, x, y, aux0, fin, sc, kc);
-    case EPI_DOT_AUX: return launch_v2_e<R, EPI_DOT_AUX>(h, x, y, aux0, fin, sc, kc);
-    case EPI_DOT_TS: return launch_v2_e<R, EPI_DOT_TS>(h, x, y, aux0, fin, sc, kc);
-    case EPI_DOT_SHD: return launch_v2_e<R, EPI_DOT_SHD>(h, x, y, aux0, fin, sc, kc);
+    case EPI_STORE: return launch_any_e<R, EPI_STORE>(h, x, y, aux0, fin, sc, kc, tma);
+    case EPI_RESID: return launch_any_e<R, EPI_RESID>(h, x, y, aux0, fin, sc, kc, tma);
+    case EPI_DOT_AUX: return launch_any_e<R, EPI_DOT_AUX>(h, x, y, aux0, fin, sc, kc, tma);
+    case EPI_DOT_TS: return launch_any_e<R, EPI_DOT_TS>(h, x, y, aux0, fin, sc, kc, tma);
+    case EPI_DOT_SHD: return launch_any_e<R, EPI_DOT_SHD>(h, x, y, aux0, fin, sc, kc, tma);
   }
   return FDFD_ERR_UNSUPPORTED;
 }
-template int launch_apply_v2<float>(fdfd_handle *, const float2 *, float2 *, int, const float2 *, int, KScalars *, int);
+template int launch_apply_v2<float>(fdfd_handle *, const float2 *, float2 *, int, const float2 *, int, KScalars *, int,
+                                    bool);
 template int launch_apply_v2<double>(fdfd_handle *, const double2 *, double2 *, int, const double2 *, int, KScalars *,
-                                     int);
+                                     int, bool);
 
 }  // namespace fdfd

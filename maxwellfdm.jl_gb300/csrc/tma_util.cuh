@@ -41,6 +41,21 @@ __device__ __forceinline__ void tma_copy4d(uint32_t dst, const CUtensorMap *map,
       "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(bar)
       : "memory");
 }
+// Asynchronous 8- or 16-byte copy to shared memory (zeros when !in), and the
+// thread's groups of them.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(uint32_t dst, const void *src, bool in) {
+  const int n = in ? BYTES : 0;
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %3, %2;" ::"r"(dst), "l"(src), "r"(n), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 // Bounded wait on an mbarrier phase: gives up after `limit` SM clocks
 // (WAIT_LIMIT ≈ 2^31, about one second) and reports false instead of
 // spinning forever.  limit = 0 tests the phase once without waiting.

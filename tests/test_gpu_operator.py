@@ -243,3 +243,41 @@ def test_balanced_schedules(pkg, oracle, monkeypatch, waves, kernel):
     assert st[0]["status"] == 0
     assert np.linalg.norm(b - S.A @ xs) / np.linalg.norm(b) <= 1.02e-7
     A.close()
+
+
+@pytest.mark.parametrize("kc", [0, 1, 2, 5])
+@pytest.mark.parametrize("bloch", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 1)])
+@pytest.mark.parametrize("N", [(3, 2, 2), (33, 17, 9), (64, 31, 6), (31, 48, 7), (7, 5, 1)])
+def test_cp_async_ring(pkg, oracle, monkeypatch, N, bloch, kc):
+    """The operator kernel fed by cp.async — odd Nx in complex64, periodic
+    axes in both precisions with a Bloch phase on one of them (phase 1 on
+    the others) — on tiles of one column, row or plane more or less than
+    whole ones, with ε random on every cell and corner (ghost corners of the
+    periodic axes included), at forced z-chunks and the tuner's choice."""
+    if N[2] == 1 and not bloch[2]:
+        pytest.skip("a symmetry axis has at least two cells")
+    if kc:
+        monkeypatch.setenv("FDFD_KCHUNK", str(kc))
+    O = oracle
+    isb = tuple(bool(b) for b in bloch)
+    g = O.Grid(_nonuniform(N, 2), isb)
+    kb = [0.0, 0.0, 0.0]
+    for w in range(3):
+        if isb[w]:
+            kb[w] = 0.23
+            break
+    om = 2 * np.pi / 6
+    npml = tuple(0 if isb[w] or N[w] < 6 else 2 for w in range(3))
+    sdl_e, sdl_m = O.stretched_dl(g, om, (npml, npml))
+    rng = np.random.default_rng(3)
+    ed = rng.uniform(1.0, 12.0, N + (3,))
+    eo = rng.uniform(-2.0, 2.0, N + (3,))
+    Ce, Cm = O.create_curls(g, sdl_e, sdl_m, tuple(kb))
+    Aref = O.create_A(om, O.create_paramop(g, ed, eo, sdl_e, sdl_m, tuple(kb)), Ce, Cm)
+    A = pkg.FDFDOperator(g.N, om, sdl_e, sdl_m, isb, [np.exp(-1j * kb[w] * g.L[w]) for w in range(3)])
+    A.set_eps(ed, eo)
+    x = _rand(A.n, 9)
+    ref = Aref @ x
+    assert np.linalg.norm(A.matvec(x, "c128") - ref) <= TOL64 * np.linalg.norm(ref)
+    assert np.linalg.norm(A.matvec(x, "c64") - ref) <= TOL32 * np.linalg.norm(ref)
+    A.close()
