@@ -88,8 +88,10 @@ __device__ __forceinline__ typename CT<R>::C own_e(const typename CT<R>::C *__re
 template <typename R>
 __device__ __forceinline__ int cidx(const OpArgs<R> &a, int v, int g) {
   // coefficient index for a (possibly ghost) H/E position along axis v
+  // (positions further out than one cell, which tiles wider than the grid
+  // ask for, are never used: any index in range)
   if (g < 0) return a.bloch[v] ? a.N[v] - 1 : 0;
-  if (g >= a.N[v]) return a.bloch[v] ? g - a.N[v] : a.N[v] - 1;
+  if (g >= a.N[v]) return a.bloch[v] && g == a.N[v] ? 0 : a.N[v] - 1;
   return g;
 }
 

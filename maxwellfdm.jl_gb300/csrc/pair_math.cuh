@@ -1,0 +1,85 @@
+// Complex arithmetic of the z-marching operator kernels (stencil2.cu, hh.cu):
+// paired FP32 instructions for complex64, scalar FP64 for complex128, and
+// neighbour exchange within a warp.
+#pragma once
+
+#include "operator_common.cuh"
+
+namespace fdfd {
+
+template <typename C>
+__device__ __forceinline__ C zif(bool z, C v) {
+  return z ? czero<C>() : v;
+}
+
+template <typename C>
+__device__ __forceinline__ C shfl_up1(C v) {
+  return mk(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
+}
+template <typename C>
+__device__ __forceinline__ C shfl_down1(C v) {
+  return mk(__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1));
+}
+
+// Complex64 arithmetic of the curls and the diagonal term on the paired FP32
+// instructions of sm_100 and later (__fadd2_rn, __fmul2_rn, __ffma2_rn:
+// both lanes rounded to nearest, as the scalar forms are), half the
+// instructions of the scalar forms; complex128 keeps the scalar forms.
+__device__ __forceinline__ float2 f2(float s) { return make_float2(s, s); }
+__device__ __forceinline__ float2 psub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+__device__ __forceinline__ double2 psub(double2 a, double2 b) { return csub(a, b); }
+// a·s + b for real s
+__device__ __forceinline__ float2 pfma(float2 a, float s, float2 b) { return __ffma2_rn(a, f2(s), b); }
+__device__ __forceinline__ double2 pfma(double2 a, double s, double2 b) { return cadd(cscale(a, s), b); }
+// a·u − b·v for coefficients a, b that are real when RC
+template <bool RC>
+__device__ __forceinline__ float2 pdiff(float2 a, float2 u, float2 b, float2 v) {
+  if constexpr (RC) {
+    return __ffma2_rn(f2(a.x), u, __fmul2_rn(f2(-b.x), v));
+  } else {
+    float2 t = __fmul2_rn(make_float2(b.y, -b.y), make_float2(v.y, v.x));  // −b·v
+    t = __ffma2_rn(f2(-b.x), v, t);
+    t = __ffma2_rn(make_float2(-a.y, a.y), make_float2(u.y, u.x), t);     // + a·u
+    return __ffma2_rn(f2(a.x), u, t);
+  }
+}
+template <bool RC>
+__device__ __forceinline__ double2 pdiff(double2 a, double2 u, double2 b, double2 v) {
+  return csub(mulc<RC>(a, u), mulc<RC>(b, v));
+}
+// conj(a0)·b0 + conj(a1)·b1 + conj(a2)·b2
+__device__ __forceinline__ float2 pdot3(float2 a0, float2 b0, float2 a1, float2 b1, float2 a2, float2 b2) {
+  float2 t = __fmul2_rn(f2(a0.x), b0);
+  t = __ffma2_rn(make_float2(a0.y, -a0.y), make_float2(b0.y, b0.x), t);
+  t = __ffma2_rn(f2(a1.x), b1, t);
+  t = __ffma2_rn(make_float2(a1.y, -a1.y), make_float2(b1.y, b1.x), t);
+  t = __ffma2_rn(f2(a2.x), b2, t);
+  return __ffma2_rn(make_float2(a2.y, -a2.y), make_float2(b2.y, b2.x), t);
+}
+// (re, im) += conj(a)·b
+template <typename R, typename C>
+__device__ __forceinline__ void dot_into(R &re, R &im, C a, C b) {
+  re = fma(a.y, b.y, fma(a.x, b.x, re));
+  im = fma(-a.y, b.x, fma(a.x, b.y, im));
+}
+// a·u + b·v for coefficients a, b that are real when RC (corner averaging)
+template <bool RC>
+__device__ __forceinline__ float2 wsum(float2 a, float2 u, float2 b, float2 v) {
+  return cadd(mulc<RC>(a, u), mulc<RC>(b, v));
+}
+template <bool RC>
+__device__ __forceinline__ double2 wsum(double2 a, double2 u, double2 b, double2 v) {
+  return cadd(mulc<RC>(a, u), mulc<RC>(b, v));
+}
+// u·s + v·t for real s, t
+__device__ __forceinline__ float2 pmix(float2 u, float s, float2 v, float t) {
+  return __ffma2_rn(u, f2(s), __fmul2_rn(v, f2(t)));
+}
+__device__ __forceinline__ double2 pmix(double2 u, double s, double2 v, double t) {
+  return cadd(cscale(u, s), cscale(v, t));
+}
+// (u + v)·s for real s
+__device__ __forceinline__ float2 psums(float2 u, float2 v, float s) { return __fmul2_rn(__fadd2_rn(u, v), f2(s)); }
+__device__ __forceinline__ double2 psums(double2 u, double2 v, double s) { return cscale(cadd(u, v), s); }
+
+}  // namespace fdfd

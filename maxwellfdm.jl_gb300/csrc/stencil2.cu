@@ -41,8 +41,10 @@
 #include <cstdlib>
 #include <type_traits>
 
+#include "cp_ring.cuh"
 #include "krylov_fin.cuh"
 #include "operator_common.cuh"
+#include "pair_math.cuh"
 #include "tma_util.cuh"
 
 namespace fdfd {
@@ -103,82 +105,6 @@ __device__ __forceinline__ typename CT<R>::C ev2(const unsigned char *sm, int s,
   using G = V2<R, RW, NS>;
   return reinterpret_cast<const typename CT<R>::C *>(sm + s * G::SLOT)[((jj + 1) * G::XW + ii + G::XOFF) * 3 + c];
 }
-
-template <typename C>
-__device__ __forceinline__ C zif(bool z, C v) {
-  return z ? czero<C>() : v;
-}
-
-template <typename C>
-__device__ __forceinline__ C shfl_up1(C v) {
-  return mk(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1));
-}
-template <typename C>
-__device__ __forceinline__ C shfl_down1(C v) {
-  return mk(__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1));
-}
-
-
-// Complex64 arithmetic of the curls and the diagonal term on the paired FP32
-// instructions of sm_100 and later (__fadd2_rn, __fmul2_rn, __ffma2_rn:
-// both lanes rounded to nearest, as the scalar forms are), half the
-// instructions of the scalar forms; complex128 keeps the scalar forms.
-__device__ __forceinline__ float2 f2(float s) { return make_float2(s, s); }
-__device__ __forceinline__ float2 psub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ double2 psub(double2 a, double2 b) { return csub(a, b); }
-// a·s + b for real s
-__device__ __forceinline__ float2 pfma(float2 a, float s, float2 b) { return __ffma2_rn(a, f2(s), b); }
-__device__ __forceinline__ double2 pfma(double2 a, double s, double2 b) { return cadd(cscale(a, s), b); }
-// a·u − b·v for coefficients a, b that are real when RC
-template <bool RC>
-__device__ __forceinline__ float2 pdiff(float2 a, float2 u, float2 b, float2 v) {
-  if constexpr (RC) {
-    return __ffma2_rn(f2(a.x), u, __fmul2_rn(f2(-b.x), v));
-  } else {
-    float2 t = __fmul2_rn(make_float2(b.y, -b.y), make_float2(v.y, v.x));  // −b·v
-    t = __ffma2_rn(f2(-b.x), v, t);
-    t = __ffma2_rn(make_float2(-a.y, a.y), make_float2(u.y, u.x), t);     // + a·u
-    return __ffma2_rn(f2(a.x), u, t);
-  }
-}
-template <bool RC>
-__device__ __forceinline__ double2 pdiff(double2 a, double2 u, double2 b, double2 v) {
-  return csub(mulc<RC>(a, u), mulc<RC>(b, v));
-}
-// conj(a0)·b0 + conj(a1)·b1 + conj(a2)·b2
-__device__ __forceinline__ float2 pdot3(float2 a0, float2 b0, float2 a1, float2 b1, float2 a2, float2 b2) {
-  float2 t = __fmul2_rn(f2(a0.x), b0);
-  t = __ffma2_rn(make_float2(a0.y, -a0.y), make_float2(b0.y, b0.x), t);
-  t = __ffma2_rn(f2(a1.x), b1, t);
-  t = __ffma2_rn(make_float2(a1.y, -a1.y), make_float2(b1.y, b1.x), t);
-  t = __ffma2_rn(f2(a2.x), b2, t);
-  return __ffma2_rn(make_float2(a2.y, -a2.y), make_float2(b2.y, b2.x), t);
-}
-// (re, im) += conj(a)·b
-template <typename R, typename C>
-__device__ __forceinline__ void dot_into(R &re, R &im, C a, C b) {
-  re = fma(a.y, b.y, fma(a.x, b.x, re));
-  im = fma(-a.y, b.x, fma(a.x, b.y, im));
-}
-// a·u + b·v for coefficients a, b that are real when RC (corner averaging)
-template <bool RC>
-__device__ __forceinline__ float2 wsum(float2 a, float2 u, float2 b, float2 v) {
-  return cadd(mulc<RC>(a, u), mulc<RC>(b, v));
-}
-template <bool RC>
-__device__ __forceinline__ double2 wsum(double2 a, double2 u, double2 b, double2 v) {
-  return cadd(mulc<RC>(a, u), mulc<RC>(b, v));
-}
-// u·s + v·t for real s, t
-__device__ __forceinline__ float2 pmix(float2 u, float s, float2 v, float t) {
-  return __ffma2_rn(u, f2(s), __fmul2_rn(v, f2(t)));
-}
-__device__ __forceinline__ double2 pmix(double2 u, double s, double2 v, double t) {
-  return cadd(cscale(u, s), cscale(v, t));
-}
-// (u + v)·s for real s
-__device__ __forceinline__ float2 psums(float2 u, float2 v, float s) { return __fmul2_rn(__fadd2_rn(u, v), f2(s)); }
-__device__ __forceinline__ double2 psums(double2 u, double2 v, double s) { return cscale(cadd(u, v), s); }
 
 template <typename R>
 struct Accs2 {
@@ -265,90 +191,14 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   }
   pdl_wait();
   if (sc != nullptr && sc->done) return;  // every thread, before any copy is issued
-  // cp.async ring: the warp's rows of a plane's box (rows j0−1 … j0+TYT; the
-  // warps 0-3 carry the halo jobs below, so the rows left over go to the
-  // last warps).  A complex64 row whose pitch is a multiple of 16 bytes goes
-  // in 16-byte copies from column i0−2 on, any other row element by element
-  // from column i0−1; cof: per copy of the lane, its offset in the row
-  // (wrapped on a periodic axis), or −1 outside the grid (filled with 0).
-  constexpr int NCOPY = 4;
-  const bool vec = CPA && sizeof(C) == 8 && (a.N[0] & 1) == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-  const int row3 = 3 * a.N[0];
-  int cof[NCOPY];
-  // Bloch phases other than 1, applied to the wrapped cells once landed
-  bool phx = false, phy = false, phz = false;
-  if constexpr (CPA) {
-#pragma unroll
-    for (int n = 0; n < NCOPY; ++n) {
-      const int t = lane + 32 * n;
-      int off = vec ? 3 * (i0 - 2) + 2 * t : 3 * (i0 - 1) + t;
-      if (off < 0) off = bx_ ? off + row3 : -1;
-      else if (off >= row3) off = (bx_ && off < row3 + 3) ? off - row3 : -1;
-      if (off < 0 || off >= row3 || t >= (vec ? 3 * (TX + 4) / 2 : 3 * (TX + 2))) off = -1;
-      cof[n] = off;
-    }
-    phx = bx_ && (ex.ph[0].x != R(1) || ex.ph[0].y != R(0));
-    phy = by_ && (ex.ph[1].x != R(1) || ex.ph[1].y != R(0));
-    phz = bz_ && (ex.ph[2].x != R(1) || ex.ph[2].y != R(0));
-  }
-  auto copy_plane = [&](int q, int s) {
-    const bool zout = q < 0 || q >= a.N[2];
-    const int gq = q < 0 ? q + a.N[2] : q >= a.N[2] ? q - a.N[2] : q;
-    for (int r = NW - 1 - w; r < G::BY; r += NW) {
-      int gj = j0 + r - 1;
-      bool ok = !zout || bz_;
-      if (gj < 0) {
-        ok = ok && by_;
-        gj += a.N[1];
-      } else if (gj >= a.N[1]) {
-        ok = ok && by_ && gj == a.N[1];
-        gj -= a.N[1];
-      }
-      const C *src = x + (ok ? row3 * (gj + a.N[1] * gq) : 0);
-      const uint32_t dst = smem_u32(sm + s * G::SLOT) + r * (G::XW * 3 * (int)sizeof(C));
-      if (vec) {
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          const bool in = ok && cof[n] >= 0;
-          if (lane + 32 * n < 3 * (TX + 4) / 2) cp_async<16>(dst + (lane + 32 * n) * 16, src + (in ? cof[n] : 0), in);
-        }
-      } else {
-#pragma unroll
-        for (int n = 0; n < NCOPY; ++n) {
-          const bool in = ok && cof[n] >= 0;
-          if (lane + 32 * n < 3 * (TX + 2))
-            cp_async<sizeof(C)>(dst + ((G::XOFF - 1) * 3 + lane + 32 * n) * (int)sizeof(C), src + (in ? cof[n] : 0), in);
-        }
-      }
-    }
-  };
-  // multiply the wrapped cells of a landed plane by their Bloch phases (the
-  // warp's own rows, so only the warp has to have seen its copies land)
-  auto phase_plane = [&](int q, int s) {
-    __syncwarp();
-    const bool zw = phz && (q < 0 || q >= a.N[2]);
-    for (int r = NW - 1 - w; r < G::BY; r += NW) {
-      const int gj = j0 + r - 1;
-      const bool yw = phy && (gj < 0 || gj >= a.N[1]);
-      C *row = reinterpret_cast<C *>(sm + s * G::SLOT) + (r * G::XW + G::XOFF - 1) * 3;
-      if (zw || yw) {
-        C p = zw ? (q < 0 ? ex.phinv[2] : ex.ph[2]) : mk(R(1), R(0));
-        if (yw) p = cmul(p, gj < 0 ? ex.phinv[1] : ex.ph[1]);
-        for (int e = lane; e < 3 * (TX + 2); e += 32) row[e] = cmul(row[e], p);
-        __syncwarp();
-      }
-      if (phx && lane < 6) {  // column −1 of the first tile, column N_x of the last
-        const int e = lane < 3 ? lane : 3 * (a.N[0] - i0 + 1) + lane - 3;
-        if (lane < 3 ? i0 == 0 : e < 3 * (TX + 2)) row[e] = cmul(row[e], lane < 3 ? ex.phinv[0] : ex.ph[0]);
-      }
-    }
-  };
+  CpRing<R, NW, G::BY, G::XW, G::XOFF> ring;
+  if constexpr (CPA) ring.init(a, ex, x, i0, j0, w, lane);
   // the first planes' E tiles go out now, so their latency overlaps the
   // coefficient tables below; each slot's single arrival (and its ε tiles,
   // which need the off-diagonal flags) follows once the tables are in place
   if constexpr (CPA) {
     for (int p = 0; p < NS; ++p) {
-      if (kfirst + p <= k1) copy_plane(kfirst + p, p);
+      if (kfirst + p <= k1) ring.copy(a, sm + p * G::SLOT, kfirst + p);
       cp_async_commit();
     }
   } else if (tid == 0) {
@@ -460,8 +310,8 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
     if constexpr (CPA) {
       // planes k0−1 … k0+1 have landed (the newest group may be in flight)
       cp_async_wait<1>();
-      if (phx || phy || phz)
-        for (int p = 0; p < 3; ++p) phase_plane(kfirst + p, p);
+      if (ring.phased())
+        for (int p = 0; p < 3; ++p) ring.phase(a, ex, sm + p * G::SLOT, kfirst + p);
       __syncthreads();
     } else {
       ok = mbar_wait_sleep(smem_u32(&bars[0]), 0, ex.wait_limit, 100000u);
@@ -702,9 +552,9 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
       // read after this plane, plane k−1 not at all
       if constexpr (CPA) {
         cp_async_wait<0>();  // plane k+2 has landed; every thread sees it after the barrier
-        if ((phx || phy || phz) && k + 2 <= k1) phase_plane(k + 2, s1 + 1 == NS ? 0 : s1 + 1);
+        if (ring.phased() && k + 2 <= k1) ring.phase(a, ex, sm + (s1 + 1 == NS ? 0 : s1 + 1) * G::SLOT, k + 2);
         __syncthreads();
-        if (k - 1 + NS <= k1) copy_plane(k - 1 + NS, sm1);
+        if (k - 1 + NS <= k1) ring.copy(a, sm + sm1 * G::SLOT, k - 1 + NS);
         cp_async_commit();
       } else if (__syncthreads_or(!ok)) {
         run = false;
@@ -989,7 +839,12 @@ static int launch_cp_t(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R
     if (e != cudaSuccess) return cuda_check(h, e, "cudaFuncSetAttribute(carveout)");
     attr.set(h->dev);
   }
-  ex.oflag_w = h->has_off ? h->oflag_rows[RW - 1] : nullptr;
+  // periodic grids take the flags of the 32×8 tiles, as the plain kernel
+  // does: neither set of flags follows the wrap of an axis (a corner on plane
+  // 0 that the last cells read), and with the same ones both kernels include
+  // the same corner terms
+  const bool periodic = h->bloch[0] || h->bloch[1] || h->bloch[2];
+  ex.oflag_w = h->has_off && !periodic ? h->oflag_rows[RW - 1] : nullptr;
   const OpArgs<R> a = op_args<R>(h);
   const cudaError_t e = launch_k(h, k_apply_cp<R, EPI, RW, NS, MB>, grid, dim3(G::NT, 1, 1), (size_t)G::SMEM, a, ex, x,
                                  y, aux0, h->red, fin, sc);

@@ -74,3 +74,43 @@ def test_hh_rejects_offdiagonal(pkg, oracle):
     with pytest.raises(pkg.FDFDError):
         A.set_field_type("H")
     A.close()
+
+
+@pytest.mark.parametrize("kc", [0, 1, 2, 5])
+@pytest.mark.parametrize("bloch", [(0, 0, 0), (1, 0, 0), (0, 1, 0), (0, 0, 1), (1, 1, 1)])
+@pytest.mark.parametrize("N", [(3, 2, 2), (33, 17, 9), (64, 32, 6), (31, 49, 7), (7, 5, 1)])
+def test_hh_matvec_tile_edges(pkg, oracle, monkeypatch, N, bloch, kc):
+    """The H operator on tiles of one column, row or plane more or less than
+    whole ones, each axis periodic in turn with a Bloch phase on one of them,
+    ε random at every sample (walls included), forced z-chunks, real and
+    complex ω: ≤ 1e-12 (complex128), ≤ 1e-5 (complex64) of the oracle's matrix,
+    as in the operator tests."""
+    if N[2] == 1 and not bloch[2]:
+        pytest.skip("a symmetry axis has at least two cells")
+    if kc:
+        monkeypatch.setenv("FDFD_KCHUNK", str(kc))
+    O = oracle
+    rng = np.random.default_rng(51)
+    lp = tuple(np.concatenate([[0.0], np.cumsum(rng.uniform(0.6, 1.4, n))]) for n in N)
+    isb = tuple(bool(b) for b in bloch)
+    g = O.Grid(lp, isb)
+    kb = [0.0, 0.0, 0.0]
+    for w in range(3):
+        if isb[w]:
+            kb[w] = 0.23
+            break
+    npml = tuple(0 if isb[w] or N[w] < 6 else 2 for w in range(3))
+    ed = rng.uniform(1.0, 12.0, N + (3,))
+    ed[..., N[2] // 2:, :] = 3.0  # planes without a change of ε along z
+    for om in (2 * np.pi / 6, 1.1 + 0.1j):
+        sdl_e, sdl_m = O.stretched_dl(g, 2 * np.pi / 6, (npml, npml))
+        Ce, Cm = O.create_curls(g, sdl_e, sdl_m, tuple(kb))
+        A = pkg.FDFDOperator(N, om, sdl_e, sdl_m, isb, [np.exp(-1j * kb[w] * g.L[w]) for w in range(3)])
+        A.set_eps(ed)
+        A.set_field_type("H")
+        x = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+        inv = 1.0 / O.field_to_vec(ed)
+        ref = Ce @ (inv * (Cm @ x)) - om ** 2 * x
+        assert np.linalg.norm(A.matvec(x, "c128") - ref) <= 1e-12 * np.linalg.norm(ref)
+        assert np.linalg.norm(A.matvec(x, "c64") - ref) <= 1e-5 * np.linalg.norm(ref)
+        A.close()
