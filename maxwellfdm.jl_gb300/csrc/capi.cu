@@ -183,32 +183,35 @@ __global__ void k_oflags_rows(const double *eoff, long long ncell, int N0, int N
   }
 }
 
-int build_oflags(fdfd_handle *h) {
-  if (!h->has_off) return FDFD_OK;
-  const int tiles_x = (h->N[0] + TX - 1) / TX, tiles_y = (h->N[1] + TY - 1) / TY;
-  const size_t nflag = (size_t)tiles_x * tiles_y * h->N[2];
-  if (!h->oflag) {
-    if (dev_malloc(&h->oflag, nflag) != cudaSuccess) {
+// Allocate (once) and clear the off-diagonal flags of all group sizes.
+int ensure_oflags(fdfd_handle *h) {
+  const int tiles_x = (h->N[0] + TX - 1) / TX;
+  uint8_t **f[3] = {&h->oflag, &h->oflag_rows[0], &h->oflag_rows[1]};
+  const int rows[3] = {TY, 1, 2};
+  for (int q = 0; q < 3; ++q) {
+    const size_t nf = (size_t)tiles_x * ((h->N[1] + rows[q] - 1) / rows[q]) * h->N[2];
+    if (!*f[q] && dev_malloc(f[q], nf) != cudaSuccess) {
       cudaGetLastError();
+      *f[q] = nullptr;
       return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(oflag) failed");
     }
+    const int rc = cuda_check(h, cudaMemsetAsync(*f[q], 0, nf, h->stream), "memset oflag");
+    if (rc) return rc;
   }
-  int rc = cuda_check(h, cudaMemsetAsync(h->oflag, 0, nflag, h->stream), "memset oflag");
+  return FDFD_OK;
+}
+
+int build_oflags(fdfd_handle *h) {
+  if (!h->has_off) return FDFD_OK;
+  const int tiles_x = (h->N[0] + TX - 1) / TX;
+  int rc = ensure_oflags(h);
   if (rc) return rc;
   k_oflags<<<152 * 4, 256, 0, h->stream>>>(h->eoff64, h->ncell, h->N[0], h->N[1], h->N[2], tiles_x, h->oflag);
   if ((rc = cuda_check(h, cudaGetLastError(), "k_oflags"))) return rc;
-  // per groups of 1 and 2 rows (the second TMA kernel's warp strips)
+  // per groups of 1 and 2 rows (the second kernel's warp strips)
   for (int g = 1; g <= 2; ++g) {
-    const size_t nf = (size_t)tiles_x * ((h->N[1] + g - 1) / g) * h->N[2];
-    uint8_t *&f = h->oflag_rows[g - 1];
-    if (!f) {
-      if (dev_malloc(&f, nf) != cudaSuccess) {
-        cudaGetLastError();
-        return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(oflag rows) failed");
-      }
-    }
-    if ((rc = cuda_check(h, cudaMemsetAsync(f, 0, nf, h->stream), "memset oflag rows"))) return rc;
-    k_oflags_rows<<<152 * 4, 256, 0, h->stream>>>(h->eoff64, h->ncell, h->N[0], h->N[1], h->N[2], tiles_x, g, f);
+    k_oflags_rows<<<152 * 4, 256, 0, h->stream>>>(h->eoff64, h->ncell, h->N[0], h->N[1], h->N[2], tiles_x, g,
+                                                  h->oflag_rows[g - 1]);
     if ((rc = cuda_check(h, cudaGetLastError(), "k_oflags_rows"))) return rc;
   }
   return FDFD_OK;
@@ -238,13 +241,17 @@ static int ensure_eps_buffers(fdfd_handle *h, bool off) {
   return FDFD_OK;
 }
 
-// Refresh the FP32 copies from the FP64 masters and rebuild the flags.
-int finish_eps(fdfd_handle *h) {
+// After new ε data: refresh the FP32 copies from the FP64 masters and rebuild
+// the flags (refresh = false where the caller wrote them itself), retune
+// where the off-diagonal tensor came or went.
+int finish_eps(fdfd_handle *h, bool refresh) {
   const long long n = 3 * h->ncell;
-  k_to_f32<<<152 * 4, 256, 0, h->stream>>>(h->eps32, h->eps64, n);
-  int rc = cuda_check(h, cudaGetLastError(), "k_to_f32");
-  if (rc) return rc;
-  if (h->has_off) {
+  int rc = FDFD_OK;
+  if (refresh) {
+    k_to_f32<<<152 * 4, 256, 0, h->stream>>>(h->eps32, h->eps64, n);
+    if ((rc = cuda_check(h, cudaGetLastError(), "k_to_f32"))) return rc;
+  }
+  if (refresh && h->has_off) {
     k_to_f32<<<152 * 4, 256, 0, h->stream>>>(h->eoff32, h->eoff64, n);
     rc = cuda_check(h, cudaGetLastError(), "k_to_f32");
     if (rc) return rc;
@@ -286,7 +293,7 @@ int upload_eps(fdfd_handle *h, const double *eps_diag_aos, const double *eps_off
                     "upload eps off");
     if (rc) return rc;
   }
-  return finish_eps(h);
+  return finish_eps(h, true);
 }
 
 static int ensure_scratch(fdfd_handle *h, bool c64) {
@@ -477,7 +484,7 @@ int fdfd_create(const fdfd_desc *d, fdfd_handle **out) {
     std::vector<double> ones(3 * (size_t)h->ncell, 1.0);
     cudaMemcpy(h->eps64, ones.data(), ones.size() * sizeof(double), cudaMemcpyHostToDevice);
   }
-  if ((rc = finish_eps(h))) { fdfd_destroy(h); return rc; }
+  if ((rc = finish_eps(h, true))) { fdfd_destroy(h); return rc; }
   if (dev_malloc(&h->util_sc, sizeof(KScalars)) != cudaSuccess) {
     cudaGetLastError();
     fdfd_destroy(h);
@@ -527,6 +534,7 @@ void fdfd_destroy(fdfd_handle *h) {
     cudaFree(h->oflag_rows[0]);
     cudaFree(h->oflag_rows[1]);
     cudaFree(h->smask);
+    cudaFree(h->setup_scratch);
     cudaFree(h->work[0]);
     cudaFree(h->work[1]);
   }

@@ -138,6 +138,8 @@ struct fdfd_handle {
   uint8_t *oflag = nullptr;
   uint8_t *oflag_rows[2] = {nullptr, nullptr};  // the same per x tile, group of 1 / 2 rows and plane
   bool has_off = false;
+  void *setup_scratch = nullptr;  // kept between fdfd_smooth_objects calls (at most 64 MiB)
+  size_t setup_bytes = 0;
   uint8_t *smask = nullptr;  // 4*ncell smoothing mask (from fdfd_smooth_objects)
   bool has_design = false;   // a design region was applied by fdfd_smooth_objects
   int design_lo[3] = {0, 0, 0}, design_hi[3] = {0, 0, 0};

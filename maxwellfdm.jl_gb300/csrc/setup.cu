@@ -24,13 +24,15 @@
 // This file is compiled with --fmad=false: every product and sum rounds
 // exactly as in the oracle, so object indices and masks are bit-identical.
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "fdfd_internal.cuh"
 
 namespace fdfd {
 
-int finish_eps(fdfd_handle *h);
+int finish_eps(fdfd_handle *h, bool refresh);
+int ensure_oflags(fdfd_handle *h);
 
 struct DevObj {
   int kind;
@@ -56,34 +58,38 @@ __device__ __forceinline__ bool inside(const DevObj &o, double x, double y, doub
   return x >= o.p[0] && x <= o.p[3] && y >= o.p[1] && y <= o.p[4] && z >= o.p[2] && z <= o.p[5];
 }
 
-// oind over index boxes: blockIdx.y = object, threads stride over its box
-__global__ void k_assign(int *oind, Axes ax, const DevObj *objs, const int *boxes) {
-  const int q = blockIdx.y;
+// The seven sample sets whose object indices are needed: E_w (0-2, the N³
+// samples), H_w (3-5) and cell centres (6), both extended by a ghost sample
+// per axis ((N+1)³).
+constexpr int NSETS = 7;
+struct SampleSets {
+  int *o[NSETS];
+  Axes ax[NSETS];
+};
+
+// Object indices of every set: blockIdx.y = object, blockIdx.z = set, threads
+// stride over the object's index box.
+__global__ void k_assign(SampleSets S, const DevObj *objs, const int *boxes) {
+  const int q = blockIdx.y, set = blockIdx.z;
   const DevObj o = objs[q];
-  const int *b = boxes + 6 * q;  // lo0, lo1, lo2, hi0, hi1, hi2 (inclusive lo, exclusive hi)
+  const Axes &ax = S.ax[set];
+  int *oind = S.o[set];
+  const int *b = boxes + 6 * ((long long)set * gridDim.y + q);  // lo0, lo1, lo2, hi0, hi1, hi2 (inclusive lo, exclusive hi)
   const int e0 = b[3] - b[0], e1 = b[4] - b[1], e2 = b[5] - b[2];
   if (e0 <= 0 || e1 <= 0 || e2 <= 0) return;
-  const long long vol = (long long)e0 * e1 * e2;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < vol;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int i = b[0] + (int)(t % e0), j = b[1] + (int)((t / e0) % e1), k = b[2] + (int)(t / ((long long)e0 * e1));
-    if (inside(o, ax.pos[0][i], ax.pos[1][j], ax.pos[2][k])) {
+  auto put = [&](int i, int j, int k) {
+    if (inside(o, ax.pos[0][i], ax.pos[1][j], ax.pos[2][k]))
       atomicMax(&oind[i + (long long)ax.n[0] * (j + (long long)ax.n[1] * k)], q + 1);
+  };
+  const long long vol = (long long)e0 * e1 * e2;
+  if (vol < (1ll << 30)) {  // 32-bit index arithmetic
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < (unsigned)vol; t += gridDim.x * blockDim.x) {
+      const unsigned u = t / (unsigned)e0;
+      put(b[0] + (int)(t % (unsigned)e0), b[1] + (int)(u % (unsigned)e1), b[2] + (int)(u / (unsigned)e1));
     }
-  }
-}
-
-// copy plane src → dst along axis w of an (n0,n1,n2) int array
-__global__ void k_copy_plane(int *a, int n0, int n1, int n2, int w, int dst, int src) {
-  const int m0 = (w == 0) ? n1 : n0, m1 = (w == 2) ? n1 : n2;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < (long long)m0 * m1;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int u = (int)(t % m0), v = (int)(t / m0);
-    int id[3], is[3];
-    if (w == 0) { id[0] = dst; is[0] = src; id[1] = is[1] = u; id[2] = is[2] = v; }
-    else if (w == 1) { id[1] = dst; is[1] = src; id[0] = is[0] = u; id[2] = is[2] = v; }
-    else { id[2] = dst; is[2] = src; id[0] = is[0] = u; id[1] = is[1] = v; }
-    a[id[0] + (long long)n0 * (id[1] + (long long)n1 * id[2])] = a[is[0] + (long long)n0 * (is[1] + (long long)n1 * is[2])];
+  } else {
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < vol; t += (long long)gridDim.x * blockDim.x)
+      put(b[0] + (int)(t % e0), b[1] + (int)((t / e0) % e1), b[2] + (int)(t / ((long long)e0 * e1)));
   }
 }
 
@@ -178,104 +184,194 @@ __device__ __forceinline__ double obj_eps(const DevObj *objs, double eps_bg, int
   return q == 0 ? eps_bg : objs[q - 1].eps;
 }
 
-// Kottke tensor of a voxel [lo, hi] whose 8 corner indices are c[]; returns
-// the number of distinct objects (1, 2 or more) and fills T (row-major 3×3).
-__device__ int smoothed_tensor(const int c[8], const DevObj *objs, double eps_bg, const double lo[3],
-                               const double hi[3], double T[9]) {
+// Kottke tensor of a voxel [lo, hi] whose 8 corner indices are c[]: ε̃ as
+// mean m and difference d of ε̃ = m I + d n nᵀ, with the normal n (m the
+// mean of the corner ε and d = 0 where more than two objects meet).
+__device__ void smoothed_tensor(const int c[8], const DevObj *objs, double eps_bg, const double lo[3],
+                                const double hi[3], double &m, double &d, double n[3]) {
   int qmin = c[0], qmax = c[0];
   for (int t = 1; t < 8; ++t) { qmin = min(qmin, c[t]); qmax = max(qmax, c[t]); }
-  int ndist = 1;
-  {
-    int seen[8];
-    int ns = 0;
-    for (int t = 0; t < 8; ++t) {
-      bool f = false;
-      for (int u = 0; u < ns; ++u) f = f || (seen[u] == c[t]);
-      if (!f) seen[ns++] = c[t];
-    }
-    ndist = ns;
-  }
-  for (int t = 0; t < 9; ++t) T[t] = 0.0;
-  if (ndist == 2) {
+  bool two = true;
+  for (int t = 0; t < 8; ++t) two = two && (c[t] == qmin || c[t] == qmax);
+  n[0] = n[1] = n[2] = 0.0;
+  if (two) {
     const double efg = obj_eps(objs, eps_bg, qmax), ebg = obj_eps(objs, eps_bg, qmin);
-    double xc[3], n[3], r0[3];
+    double xc[3], r0[3];
     for (int a = 0; a < 3; ++a) xc[a] = 0.5 * (lo[a] + hi[a]);
     normal_point(objs[qmax - 1], xc, n, r0);
     const double f = volfrac_plane(lo, hi, n, r0);
-    const double em = f * efg + (1.0 - f) * ebg;
+    m = f * efg + (1.0 - f) * ebg;
     const double eh = 1.0 / (f / efg + (1.0 - f) / ebg);
-    for (int a = 0; a < 3; ++a)
-      for (int b = 0; b < 3; ++b) T[3 * a + b] = (a == b ? em : 0.0) + (eh - em) * (n[a] * n[b]);
-  } else if (ndist > 2) {
+    d = eh - m;
+  } else {
     double s = 0.0;
     for (int t = 0; t < 8; ++t) s += obj_eps(objs, eps_bg, c[t]);
-    const double mean = s / 8.0;
-    T[0] = T[4] = T[8] = mean;
+    m = s / 8.0;
+    d = 0.0;
   }
-  return ndist;
 }
 
-// corner order matches the oracle's ravel of o[i:i+2, j:j+2, k:k+2]
-__device__ __forceinline__ void corners8(const int *o, int n0, int n1, int i, int j, int k, int c[8]) {
+// What the smoothing kernels read and write.  Voxel set s < 3 is ε_ss at its
+// E_s samples (voxel corners at H_s samples), set 3 the off-diagonal ε at
+// the E-voxel corners (voxel corners at cell centres).
+struct SmoothArgs {
+  int N[3], bloch[3];
+  long long nc;
+  const int *oe[3];   // object indices at the E_w samples (N³)
+  const int *ov[4];   // and at the voxel corners of each set ((N+1)³)
+  const double *prim[3], *dual[3];
+  const DevObj *objs;
+  double eps_bg;
+  double *eps, *eoff;
+  float *eps32, *eoff32;
+  uint8_t *smask;
+  unsigned int *nnz;
+  uint8_t *flag[3];   // off-diagonal flags of groups of TY, 1 and 2 rows
+  int tiles_x;
+};
+
+// Source index of extended index t along axis a of voxel set s: a symmetry
+// wall's dual ghost copies dual index 0, Bloch ghosts the periodic image.
+__device__ __forceinline__ int ghost_src(const SmoothArgs &A, int s, int a, int t) {
+  const bool dual = s == 3 || a != s;
+  if (dual) return t == 0 ? (A.bloch[a] ? A.N[a] : 1) : t;
+  return t == A.N[a] && A.bloch[a] ? 0 : t;
+}
+// the 8 corner indices in the oracle's order (ravel of o[i:i+2, j:j+2, k:k+2])
+__device__ __forceinline__ void corners8(const SmoothArgs &A, int s, int i, int j, int k, int c[8]) {
+  const int *o = A.ov[s];
+  const long long n0 = A.N[0] + 1, n1 = A.N[1] + 1;
+  const int x0 = ghost_src(A, s, 0, i), x1 = ghost_src(A, s, 0, i + 1);
+  const int y0 = ghost_src(A, s, 1, j), y1 = ghost_src(A, s, 1, j + 1);
+  const int z0 = ghost_src(A, s, 2, k), z1 = ghost_src(A, s, 2, k + 1);
+  const int xs[2] = {x0, x1}, ys[2] = {y0, y1}, zs[2] = {z0, z1};
   int t = 0;
+#pragma unroll
   for (int a = 0; a < 2; ++a)
+#pragma unroll
     for (int b = 0; b < 2; ++b)
-      for (int d = 0; d < 2; ++d) c[t++] = o[(i + a) + (long long)n0 * ((j + b) + (long long)n1 * (k + d))];
+#pragma unroll
+      for (int d = 0; d < 2; ++d) c[t++] = o[xs[a] + n0 * (ys[b] + n1 * zs[d])];
 }
 
-// ε_ww at E_w samples
-__global__ void k_smooth_diag(int w, int N0, int N1, int N2, const int *oe, const int *oh, Axes hax,
-                              const DevObj *objs, double eps_bg, double *eps, uint8_t *smask) {
-  const long long nc = (long long)N0 * N1 * N2;
-  for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < nc;
-       cell += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(cell % N0), j = (int)((cell / N0) % N1), k = (int)(cell / ((long long)N0 * N1));
-    int c[8];
-    corners8(oh, N0 + 1, N1 + 1, i, j, k, c);
-    bool same = true;
-    for (int t = 1; t < 8; ++t) same = same && (c[t] == c[0]);
-    if (same) {
-      eps[w * nc + cell] = obj_eps(objs, eps_bg, oe[cell]);
-      smask[4 * cell + w] = 0;
-      continue;
+// Voxels of one object: ε of that object, no smoothing.  The others are only
+// marked (smask 1) for k_smooth.  Threads run over the flattened x-y plane,
+// blockIdx.y strides the planes.
+__global__ void __launch_bounds__(256) k_classify(SmoothArgs A) {
+  const int plane = A.N[0] * A.N[1];
+  const int p = blockIdx.x * 256 + threadIdx.x;
+  if (p >= plane) return;
+  const int i = p % A.N[0], j = p / A.N[0];
+  for (int k = blockIdx.y; k < A.N[2]; k += gridDim.y) {
+    const long long cell = (long long)plane * k + p;
+    uchar4 mask = make_uchar4(0, 0, 0, 0);
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      int c[8];
+      corners8(A, s, i, j, k, c);
+      bool same = true;
+#pragma unroll
+      for (int t = 1; t < 8; ++t) same = same && (c[t] == c[0]);
+      if (!same) {
+        (&mask.x)[s] = 1;
+      } else if (s < 3) {
+        const double e = obj_eps(A.objs, A.eps_bg, A.oe[s][cell]);
+        A.eps[s * A.nc + cell] = e;
+        A.eps32[s * A.nc + cell] = (float)e;
+      } else {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          A.eoff[q * A.nc + cell] = 0.0;
+          A.eoff32[q * A.nc + cell] = 0.0f;
+        }
+      }
     }
-    const double lo[3] = {hax.pos[0][i], hax.pos[1][j], hax.pos[2][k]};
-    const double hi[3] = {hax.pos[0][i + 1], hax.pos[1][j + 1], hax.pos[2][k + 1]};
-    double T[9];
-    smoothed_tensor(c, objs, eps_bg, lo, hi, T);
-    eps[w * nc + cell] = T[4 * w];
-    smask[4 * cell + w] = 1;
+    reinterpret_cast<uchar4 *>(A.smask)[cell] = mask;
   }
 }
 
-// off-diagonal ε at E-voxel corners (voxel corners at cell centres)
-__global__ void k_smooth_off(int N0, int N1, int N2, const int *oc, Axes cax, const DevObj *objs, double eps_bg,
-                             double *eoff, uint8_t *smask, unsigned int *nnz) {
-  const long long nc = (long long)N0 * N1 * N2;
-  unsigned int cnt = 0;
-  for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < nc;
-       cell += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(cell % N0), j = (int)((cell / N0) % N1), k = (int)(cell / ((long long)N0 * N1));
-    int c[8];
-    corners8(oc, N0 + 1, N1 + 1, i, j, k, c);
-    bool same = true;
-    for (int t = 1; t < 8; ++t) same = same && (c[t] == c[0]);
-    if (same) {
-      eoff[cell] = eoff[nc + cell] = eoff[2 * nc + cell] = 0.0;
-      smask[4 * cell + 3] = 0;
-      continue;
-    }
-    const double lo[3] = {cax.pos[0][i], cax.pos[1][j], cax.pos[2][k]};
-    const double hi[3] = {cax.pos[0][i + 1], cax.pos[1][j + 1], cax.pos[2][k + 1]};
-    double T[9];
-    smoothed_tensor(c, objs, eps_bg, lo, hi, T);
-    eoff[cell] = T[1];
-    eoff[nc + cell] = T[5];
-    eoff[2 * nc + cell] = T[6];
-    smask[4 * cell + 3] = 1;
-    cnt += (T[1] != 0.0 || T[5] != 0.0 || T[6] != 0.0);
+// One marked voxel: its smoothed ε in both precisions and, where an
+// off-diagonal is not 0, the flags of the outputs that read it (the corner's
+// own cell and the one before it on each axis, in groups of g rows).
+__device__ void smooth_voxel(const SmoothArgs &A, long long entry, unsigned &cnt) {
+  const int s = (int)(entry & 3);
+  const long long cell = entry >> 2;
+  const int plane = A.N[0] * A.N[1];
+  const int k = (int)(cell / plane), p = (int)(cell - (long long)plane * k);
+  const int g[3] = {p % A.N[0], p / A.N[0], k};
+  int c[8];
+  corners8(A, s, g[0], g[1], g[2], c);
+  double lo[3], hi[3], n[3], m, d;
+  for (int a = 0; a < 3; ++a) {
+    const double *pos = (s < 3 && a == s) ? A.prim[a] : A.dual[a];
+    lo[a] = pos[g[a]];
+    hi[a] = pos[g[a] + 1];
   }
-  if (cnt) atomicAdd(nnz, cnt);
+  smoothed_tensor(c, A.objs, A.eps_bg, lo, hi, m, d, n);
+  if (s < 3) {
+    const double e = m + d * (n[s] * n[s]);
+    A.eps[s * A.nc + cell] = e;
+    A.eps32[s * A.nc + cell] = (float)e;
+    return;
+  }
+  const double o[3] = {0.0 + d * (n[0] * n[1]), 0.0 + d * (n[1] * n[2]), 0.0 + d * (n[2] * n[0])};
+  for (int q = 0; q < 3; ++q) {
+    A.eoff[q * A.nc + cell] = o[q];
+    A.eoff32[q * A.nc + cell] = (float)o[q];
+  }
+  if (o[0] == 0.0 && o[1] == 0.0 && o[2] == 0.0) return;
+  cnt++;
+  for (int f = 0; f < 3; ++f) {
+    const int rows = f == 0 ? TY : f;
+    for (int dx = 0; dx < 2; ++dx)
+      for (int dy = 0; dy < 2; ++dy) {
+        if (g[0] < dx || g[1] < dy) continue;
+        const long long tc = (g[0] - dx) / TX + (long long)A.tiles_x * ((g[1] - dy) / rows);
+        A.flag[f][tc * A.N[2] + k] = 1;
+        if (k > 0) A.flag[f][tc * A.N[2] + k - 1] = 1;
+      }
+  }
+}
+
+// The marked voxels, 32 at a time: about 300 FP64 instructions each (a dozen
+// divides), which cost a warp the same for one lane as for 32, and they lie
+// on surfaces — computed where they were found, nearly every warp that met
+// an interface paid for one or two lanes (514 µs at 96³ with 40 spheres).
+// Each warp scans the masks (its 32-cell groups interleaved over the grid, so
+// all warps meet about the same number) and queues what it finds.
+constexpr int SMOOTH_WARPS = 4;
+__global__ void __launch_bounds__(SMOOTH_WARPS * 32) k_smooth(SmoothArgs A) {
+  __shared__ long long queue[SMOOTH_WARPS][64];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  long long *q = queue[w];
+  const long long nw = (long long)gridDim.x * SMOOTH_WARPS;
+  unsigned cnt = 0;
+  int held = 0;
+  for (long long base = (blockIdx.x * (long long)SMOOTH_WARPS + w) * 32; base < A.nc; base += nw * 32) {
+    const long long cell = base + lane;
+    uchar4 m = make_uchar4(0, 0, 0, 0);
+    if (cell < A.nc) m = reinterpret_cast<const uchar4 *>(A.smask)[cell];
+    if (!__any_sync(0xffffffffu, (m.x | m.y | m.z | m.w) != 0)) continue;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      const bool hit = (&m.x)[s] != 0;
+      const unsigned b = __ballot_sync(0xffffffffu, hit);
+      if (hit) q[held + __popc(b & ((1u << lane) - 1u))] = 4 * cell + s;
+      held += __popc(b);
+      if (held >= 32) {
+        __syncwarp();
+        const long long e = q[lane], rest = q[32 + lane];
+        smooth_voxel(A, e, cnt);
+        held -= 32;
+        __syncwarp();
+        if (lane < held) q[lane] = rest;
+        __syncwarp();
+      }
+    }
+  }
+  __syncwarp();
+  if (lane < held) smooth_voxel(A, q[lane], cnt);
+  if (cnt) atomicAdd(A.nnz, cnt);
 }
 
 __device__ __forceinline__ int wrap_or_clamp(int t, int N, int bloch) {
@@ -350,28 +446,50 @@ __global__ void k_design_off(int N0, int N1, int N2, DesignDev d, double *eoff, 
 
 // ------------------------------------------------------------ host
 namespace {
-struct DevBuf {
-  std::vector<void *> ptrs;
-  ~DevBuf() {
-    for (void *p : ptrs) cudaFree(p);
+// Device scratch of one call, cut from one allocation.  Up to KEEP bytes stay
+// with the handle for the next call (an allocation and a free cost as much
+// as the smoothing itself at small sizes); larger ones are freed at the end.
+struct Scratch {
+  static constexpr size_t KEEP = 64u << 20;
+  fdfd_handle *h;
+  char *base = nullptr;
+  size_t used = 0;
+  explicit Scratch(fdfd_handle *h_) : h(h_) {}
+  ~Scratch() {
+    if (base && base != h->setup_scratch) cudaFree(base);
   }
-  template <typename T> T *get(fdfd_handle *h, size_t n, int *rc) {
-    void *p = nullptr;
-    if (dev_malloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-      cudaGetLastError();
-      *rc = set_error(h, FDFD_ERR_NOMEM, "cudaMalloc in fdfd_smooth_objects failed");
-      return nullptr;
+  static size_t pad(size_t n) { return (n + 255) / 256 * 256; }
+  int reserve(size_t bytes) {
+    if (bytes <= h->setup_bytes) {
+      base = static_cast<char *>(h->setup_scratch);
+      return FDFD_OK;
     }
-    ptrs.push_back(p);
-    return (T *)p;
+    void *p = nullptr;
+    if (dev_malloc(&p, bytes) != cudaSuccess) {
+      cudaGetLastError();
+      return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc in fdfd_smooth_objects failed");
+    }
+    base = static_cast<char *>(p);
+    if (bytes <= KEEP) {
+      cudaFree(h->setup_scratch);
+      h->setup_scratch = p;
+      h->setup_bytes = bytes;
+    }
+    return FDFD_OK;
+  }
+  template <typename T>
+  T *get(size_t n) {
+    T *p = reinterpret_cast<T *>(base + used);
+    used += pad(n * sizeof(T));
+    return p;
   }
 };
 
 // index range [first, last] of sorted positions within [a - tiny, b + tiny]
-void index_range(const std::vector<double> &pos, double a, double b, int *lo, int *hi) {
+void index_range(const double *pos, int n, double a, double b, int *lo, int *hi) {
   const double pad = 1e-9 * (1.0 + std::fabs(a) + std::fabs(b));
-  *lo = (int)(std::lower_bound(pos.begin(), pos.end(), a - pad) - pos.begin());
-  *hi = (int)(std::upper_bound(pos.begin(), pos.end(), b + pad) - pos.begin());
+  *lo = (int)(std::lower_bound(pos, pos + n, a - pad) - pos);
+  *hi = (int)(std::upper_bound(pos, pos + n, b + pad) - pos);
 }
 }  // namespace
 
@@ -407,31 +525,70 @@ int smooth_objects_impl(fdfd_handle *h, const double *const lprim[3], const fdfd
       if (design->lo[a] < 0 || design->hi[a] > h->N[a] || design->lo[a] >= design->hi[a] || !design->eps_cells)
         return set_error(h, FDFD_ERR_ARG, "bad design region");
   }
-  DevBuf buf;
-  double *dprim[3], *ddual[3];
-  for (int w = 0; w < 3; ++w) {
-    dprim[w] = buf.get<double>(h, prim[w].size(), &rc);
-    ddual[w] = buf.get<double>(h, dual[w].size(), &rc);
-    if (rc) return rc;
-    cudaMemcpy(dprim[w], prim[w].data(), prim[w].size() * sizeof(double), cudaMemcpyHostToDevice);
-    cudaMemcpy(ddual[w], dual[w].data(), dual[w].size() * sizeof(double), cudaMemcpyHostToDevice);
+  // Host side of one upload: positions, objects, the objects' index boxes in
+  // every sample set.  Set types per axis: 0 primal, 1 dual; extended sets
+  // ((N+1)³ with ghosts) take all N+1 positions, the N³ E samples the first N
+  // primal ones or the dual ones after the ghost.
+  auto is_dual = [](int set, int a) { return set == 6 || (set < 3 ? a == set : a != set - 3); };
+  const size_t nob = (size_t)std::max(1, nobj);
+  size_t npos = 0;
+  for (int w = 0; w < 3; ++w) npos += 2 * (size_t)(h->N[w] + 1);
+  const size_t ne = design ? (size_t)(design->hi[0] - design->lo[0]) * (design->hi[1] - design->lo[1]) *
+                                 (design->hi[2] - design->lo[2])
+                           : 0;
+  const size_t up_obj = Scratch::pad(npos * sizeof(double)), up_box = up_obj + Scratch::pad(nob * sizeof(DevObj));
+  const size_t up_nnz = up_box + Scratch::pad(6 * NSETS * nob * sizeof(int)), up_bytes = up_nnz + 256;
+  std::vector<char> up(up_bytes, 0);
+  double *hpos = reinterpret_cast<double *>(up.data());
+  const double *hprim[3], *hdual[3];
+  size_t off_prim[3], off_dual[3];
+  {
+    size_t o = 0;
+    for (int w = 0; w < 3; ++w) {
+      off_prim[w] = o;
+      hprim[w] = hpos + o;
+      o = std::copy(prim[w].begin(), prim[w].end(), hpos + o) - hpos;
+      off_dual[w] = o;
+      hdual[w] = hpos + o;
+      o = std::copy(dual[w].begin(), dual[w].end(), hpos + o) - hpos;
+    }
   }
-  std::vector<DevObj> hob(std::max(1, nobj));
+  DevObj *hob = reinterpret_cast<DevObj *>(up.data() + up_obj);
+  int *hbox = reinterpret_cast<int *>(up.data() + up_box);
+  long long vmax = 1;  // points of the largest index box
   for (int q = 0; q < nobj; ++q) {
     hob[q].kind = objs[q].kind;
     hob[q].eps = objs[q].eps;
     for (int t = 0; t < 6; ++t) hob[q].p[t] = objs[q].p[t];
+    double lo[3], hi[3];
+    if (objs[q].kind == FDFD_SHAPE_SPHERE)
+      for (int w = 0; w < 3; ++w) { lo[w] = objs[q].p[w] - objs[q].p[3]; hi[w] = objs[q].p[w] + objs[q].p[3]; }
+    else if (objs[q].kind == FDFD_SHAPE_CYLZ) {
+      for (int w = 0; w < 2; ++w) { lo[w] = objs[q].p[w] - objs[q].p[2]; hi[w] = objs[q].p[w] + objs[q].p[2]; }
+      lo[2] = -HUGE_VAL;
+      hi[2] = HUGE_VAL;
+    } else
+      for (int w = 0; w < 3; ++w) { lo[w] = objs[q].p[w]; hi[w] = objs[q].p[3 + w]; }
+    int r[3][2][2][2];  // [axis][dual][extended][lo, hi]
+    for (int w = 0; w < 3; ++w)
+      for (int e = 0; e < 2; ++e) {
+        index_range(hprim[w], h->N[w] + e, lo[w], hi[w], &r[w][0][e][0], &r[w][0][e][1]);
+        index_range(hdual[w] + (1 - e), h->N[w] + e, lo[w], hi[w], &r[w][1][e][0], &r[w][1][e][1]);
+      }
+    for (int set = 0; set < NSETS; ++set) {
+      long long vol = 1;
+      for (int w = 0; w < 3; ++w) {
+        const int *e = r[w][is_dual(set, w) ? 1 : 0][set < 3 ? 0 : 1];
+        for (int v = 0; v < 2; ++v) hbox[6 * ((size_t)set * nobj + q) + 3 * v + w] = e[v];
+        vol *= std::max(0, e[1] - e[0]);
+      }
+      vmax = std::max(vmax, vol);
+    }
   }
-  DevObj *dobj = buf.get<DevObj>(h, hob.size(), &rc);
-  int *dbox = buf.get<int>(h, 6 * hob.size(), &rc);
-  // oind arrays: H_w (3, ext), cell centres (ext), E_w (3, N³ sample positions)
-  int *oh[3], *oe[3];
-  for (int w = 0; w < 3; ++w) {
-    oh[w] = buf.get<int>(h, next, &rc);
-    oe[w] = buf.get<int>(h, nc, &rc);
-  }
-  int *oc = buf.get<int>(h, next, &rc);
-  unsigned int *dnnz = buf.get<unsigned int>(h, 1, &rc);
+
+  Scratch buf(h);
+  const size_t e_bytes = Scratch::pad(nc * sizeof(int)), x_bytes = Scratch::pad(next * sizeof(int));
+  if ((rc = buf.reserve(up_bytes + 3 * e_bytes + 4 * x_bytes + Scratch::pad(ne * sizeof(double))))) return rc;
   if (!h->smask) {
     if (dev_malloc(&h->smask, 4 * (size_t)nc) != cudaSuccess) {
       cudaGetLastError();
@@ -445,96 +602,56 @@ int smooth_objects_impl(fdfd_handle *h, const double *const lprim[3], const fdfd
       return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(eps off-diagonal) failed");
     }
   }
-  if (rc) return rc;
-  cudaMemcpy(dobj, hob.data(), hob.size() * sizeof(DevObj), cudaMemcpyHostToDevice);
+  if ((rc = ensure_oflags(h))) return rc;
+
+  char *dup = buf.get<char>(up_bytes);
+  int *oind = reinterpret_cast<int *>(buf.get<char>(3 * e_bytes + 4 * x_bytes));
+  double *deps = buf.get<double>(ne);
+  const double *dpos = reinterpret_cast<const double *>(dup);
+  const DevObj *dobj = reinterpret_cast<const DevObj *>(dup + up_obj);
   cudaStream_t st = h->stream;
+  if ((rc = cuda_check(h, cudaMemcpyAsync(dup, up.data(), up_bytes, cudaMemcpyHostToDevice, st), "upload objects")))
+    return rc;
+  if ((rc = cuda_check(h, cudaMemsetAsync(oind, 0, 3 * e_bytes + 4 * x_bytes, st), "memset indices"))) return rc;
 
-  // Assign one sample set: types[w] = 0 primal (positions prim), 1 dual (dual);
-  // ext = true: (N+1)³ with ghosts; false: the N³ E sample positions, which
-  // are the ext positions offset by one along the dual axes.
-  auto assign = [&](int *o, const int types[3], bool ext) -> int {
-    Axes ax;
-    std::vector<const std::vector<double> *> hpos(3);
+  SampleSets S;
+  SmoothArgs A;
+  for (int set = 0; set < NSETS; ++set) {
+    S.o[set] = reinterpret_cast<int *>(reinterpret_cast<char *>(oind) +
+                                       (set < 3 ? set * e_bytes : 3 * e_bytes + (set - 3) * x_bytes));
     for (int w = 0; w < 3; ++w) {
-      const bool du = types[w] == 1;
-      const double *base = du ? ddual[w] : dprim[w];
-      ax.pos[w] = (!ext && du) ? base + 1 : base;
-      ax.n[w] = ext ? h->N[w] + 1 : h->N[w];
-      hpos[w] = du ? &dual[w] : &prim[w];
+      const bool du = is_dual(set, w);
+      const double *base = dpos + (du ? off_dual[w] : off_prim[w]);
+      S.ax[set].pos[w] = (set < 3 && du) ? base + 1 : base;
+      S.ax[set].n[w] = set < 3 ? h->N[w] : h->N[w] + 1;
     }
-    const long long total = (long long)ax.n[0] * ax.n[1] * ax.n[2];
-    cudaMemsetAsync(o, 0, total * sizeof(int), st);
-    if (nobj > 0) {
-      std::vector<int> boxes(6 * nobj);
-      for (int q = 0; q < nobj; ++q) {
-        double a[3], b[3];
-        if (objs[q].kind == FDFD_SHAPE_SPHERE)
-          for (int w = 0; w < 3; ++w) { a[w] = objs[q].p[w] - objs[q].p[3]; b[w] = objs[q].p[w] + objs[q].p[3]; }
-        else if (objs[q].kind == FDFD_SHAPE_CYLZ) {
-          for (int w = 0; w < 2; ++w) { a[w] = objs[q].p[w] - objs[q].p[2]; b[w] = objs[q].p[w] + objs[q].p[2]; }
-          a[2] = -HUGE_VAL;
-          b[2] = HUGE_VAL;
-        } else
-          for (int w = 0; w < 3; ++w) { a[w] = objs[q].p[w]; b[w] = objs[q].p[3 + w]; }
-        for (int w = 0; w < 3; ++w) {
-          std::vector<double> pw(hpos[w]->begin() + ((!ext && types[w] == 1) ? 1 : 0),
-                                 hpos[w]->begin() + ((!ext && types[w] == 1) ? 1 : 0) + ax.n[w]);
-          int lo, hi;
-          index_range(pw, a[w], b[w], &lo, &hi);
-          boxes[6 * q + w] = lo;
-          boxes[6 * q + 3 + w] = hi;
-        }
-      }
-      cudaMemcpyAsync(dbox, boxes.data(), boxes.size() * sizeof(int), cudaMemcpyHostToDevice, st);
-      cudaStreamSynchronize(st);
-      dim3 grid(64, nobj);
-      k_assign<<<grid, 256, 0, st>>>(o, ax, dobj, dbox);
-      int e = cuda_check(h, cudaGetLastError(), "k_assign");
-      if (e) return e;
-    }
-    if (ext) {
-      for (int w = 0; w < 3; ++w) {
-        const int N = h->N[w];
-        if (types[w] == 0) {
-          if (h->bloch[w]) k_copy_plane<<<152, 256, 0, st>>>(o, N0 + 1, N1 + 1, N2 + 1, w, N, 0);
-        } else {
-          k_copy_plane<<<152, 256, 0, st>>>(o, N0 + 1, N1 + 1, N2 + 1, w, 0, h->bloch[w] ? N : 1);
-        }
-      }
-    }
-    return cuda_check(h, cudaGetLastError(), "k_copy_plane");
-  };
-
+  }
   for (int w = 0; w < 3; ++w) {
-    int te[3], th[3];
-    for (int a = 0; a < 3; ++a) {
-      te[a] = (a == w) ? 1 : 0;
-      th[a] = (a == w) ? 0 : 1;
-    }
-    if ((rc = assign(oe[w], te, false))) return rc;
-    if ((rc = assign(oh[w], th, true))) return rc;
+    A.N[w] = h->N[w];
+    A.bloch[w] = h->bloch[w];
+    A.oe[w] = S.o[w];
+    A.prim[w] = dpos + off_prim[w];
+    A.dual[w] = dpos + off_dual[w];
   }
-  {
-    const int tc[3] = {1, 1, 1};
-    if ((rc = assign(oc, tc, true))) return rc;
-  }
-  cudaMemsetAsync(dnnz, 0, sizeof(unsigned int), st);
-  for (int w = 0; w < 3; ++w) {
-    Axes hax;
-    for (int a = 0; a < 3; ++a) {
-      hax.pos[a] = (a == w) ? dprim[a] : ddual[a];
-      hax.n[a] = h->N[a] + 1;
-    }
-    k_smooth_diag<<<152 * 8, 256, 0, st>>>(w, N0, N1, N2, oe[w], oh[w], hax, dobj, eps_bg, h->eps64, h->smask);
-  }
-  {
-    Axes cax;
-    for (int a = 0; a < 3; ++a) {
-      cax.pos[a] = ddual[a];
-      cax.n[a] = h->N[a] + 1;
-    }
-    k_smooth_off<<<152 * 8, 256, 0, st>>>(N0, N1, N2, oc, cax, dobj, eps_bg, h->eoff64, h->smask, dnnz);
-  }
+  for (int s = 0; s < 4; ++s) A.ov[s] = S.o[3 + s];
+  A.nc = nc;
+  A.objs = dobj;
+  A.eps_bg = eps_bg;
+  A.eps = h->eps64;
+  A.eoff = h->eoff64;
+  A.eps32 = h->eps32;
+  A.eoff32 = h->eoff32;
+  A.smask = h->smask;
+  A.nnz = reinterpret_cast<unsigned int *>(dup + up_nnz);
+  A.flag[0] = h->oflag;
+  A.flag[1] = h->oflag_rows[0];
+  A.flag[2] = h->oflag_rows[1];
+  A.tiles_x = (h->N[0] + TX - 1) / TX;
+  const int gx = (int)std::min(64ll, vmax / 2048 + 1);  // about eight points per thread of the largest box
+  if (nobj > 0) k_assign<<<dim3(gx, nobj, NSETS), 256, 0, st>>>(S, dobj, reinterpret_cast<const int *>(dup + up_box));
+  const long long pblk = ((long long)N0 * N1 + 255) / 256;
+  k_classify<<<dim3((unsigned)pblk, (unsigned)std::min(N2, 65535)), 256, 0, st>>>(A);
+  k_smooth<<<152 * 2, SMOOTH_WARPS * 32, 0, st>>>(A);
   if ((rc = cuda_check(h, cudaGetLastError(), "smoothing kernels"))) return rc;
   h->has_design = design != nullptr;
   if (design) {
@@ -543,11 +660,9 @@ int smooth_objects_impl(fdfd_handle *h, const double *const lprim[3], const fdfd
       h->design_hi[a] = design->hi[a];
     }
     DesignDev dd;
-    const long long ne = (long long)(design->hi[0] - design->lo[0]) * (design->hi[1] - design->lo[1]) *
-                         (design->hi[2] - design->lo[2]);
-    double *deps = buf.get<double>(h, ne, &rc);
-    if (rc) return rc;
-    cudaMemcpy(deps, design->eps_cells, ne * sizeof(double), cudaMemcpyHostToDevice);
+    if ((rc = cuda_check(h, cudaMemcpyAsync(deps, design->eps_cells, ne * sizeof(double), cudaMemcpyHostToDevice, st),
+                         "upload design")))
+      return rc;
     for (int a = 0; a < 3; ++a) {
       dd.lo[a] = design->lo[a];
       dd.hi[a] = design->hi[a];
@@ -555,16 +670,18 @@ int smooth_objects_impl(fdfd_handle *h, const double *const lprim[3], const fdfd
     }
     dd.eps = deps;
     for (int w = 0; w < 3; ++w)
-      k_design_diag<<<152 * 8, 256, 0, st>>>(w, N0, N1, N2, dd, oc, dobj, eps_bg, h->eps64, h->smask);
+      k_design_diag<<<152 * 8, 256, 0, st>>>(w, N0, N1, N2, dd, S.o[6], dobj, eps_bg, h->eps64, h->smask);
     k_design_off<<<152 * 8, 256, 0, st>>>(N0, N1, N2, dd, h->eoff64, h->smask);
     if ((rc = cuda_check(h, cudaGetLastError(), "design kernels"))) return rc;
   }
   unsigned int nnz = 0;
-  cudaMemcpyAsync(&nnz, dnnz, sizeof(unsigned int), cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(&nnz, A.nnz, sizeof(unsigned int), cudaMemcpyDeviceToHost, st);
   if ((rc = cuda_check(h, cudaStreamSynchronize(st), "smoothing sync"))) return rc;
   // design zeroing can only remove off-diagonals; keep the flag conservative
   h->has_off = nnz > 0;
-  return finish_eps(h);
+  // the FP32 copies and the flags are written already, except where a design
+  // region changed ε since
+  return finish_eps(h, design != nullptr);
 }
 
 }  // namespace fdfd

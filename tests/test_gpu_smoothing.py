@@ -112,3 +112,39 @@ def test_smoothed_operator_matches_oracle(pkg, oracle):
     yr = S.A @ x
     assert np.linalg.norm(y - yr) / np.linalg.norm(yr) < 1e-12
     A.close()
+
+
+@pytest.mark.parametrize("bloch", [(False, False, False), (True, False, True), (True, True, True)])
+@pytest.mark.parametrize("N", [(40, 33, 21), (5, 67, 9), (33, 4, 3)])
+def test_resmoothing_one_handle(pkg, oracle, N, bloch):
+    """Several geometries on one handle (kept scratch, flags of the previous
+    geometry): interfaces on more and on fewer voxels than a warp's queue
+    holds, on the grid's faces, three objects in a voxel, none at all — ε
+    and masks as the oracle's each time, and A x with the new ε."""
+    O = oracle
+    rng = np.random.default_rng(8)
+    lp = tuple(np.concatenate([[0.0], np.cumsum(rng.uniform(0.7, 1.3, n))]) for n in N)
+    g = O.Grid(lp, bloch)
+    om = 2 * np.pi / 8
+    sdl_e, sdl_m = O.stretched_dl(g, om, ((0, 0, 0), (0, 0, 0)))
+    A = pkg.FDFDOperator(N, om, sdl_e, sdl_m, bloch)
+    L = np.array([l[-1] for l in lp])
+    geoms = [[("s", L / 2, 0.3 * L.min(), 12.25)],
+             [("s", L / 3, 0.25 * L.min(), 2.25), ("b", 0.4 * L, 0.9 * L, 4.0), ("s", 0.5 * L, 0.4 * L.max(), 9.0)],
+             [],
+             [("b", -1.0 + 0 * L, np.array([0.5 * L[0], L[1] + 1, L[2] + 1]), 6.0)]]
+    x = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    Ce, Cm = O.create_curls(g, sdl_e, sdl_m)
+    for geo in geoms:
+        po, oo = _objs(pkg, O, geo)
+        A.smooth_objects(lp, po, 1.0)
+        ed, eo, mask = A.get_eps()
+        red, reo, dbg = O.assign_smooth(g, oo, 1.0, None, return_debug=True)
+        assert np.max(np.abs(ed - red)) <= 1e-12 * np.max(red)
+        assert np.max(np.abs(eo - reo)) <= 1e-12 * np.max(red)
+        assert np.array_equal(mask, dbg["smask"])
+        if bloch == (False, False, False):
+            ref = O.create_A(om, O.create_paramop(g, red, reo, sdl_e, sdl_m), Ce, Cm) @ x
+            for prec, tol in (("c128", 1e-12), ("c64", 1e-5)):
+                assert np.linalg.norm(A.matvec(x, prec) - ref) <= tol * np.linalg.norm(ref)
+    A.close()
