@@ -171,7 +171,7 @@ struct fdfd_handle {
   // gives up (≈1 s); FDFD_WAIT_LIMIT_CLOCKS lowers it, so that a test can
   // make a wait run out and see FDFD_ERR_TIMEOUT without hanging anything
   long long wait_limit = 1ll << 31;
-  // layout of the second TMA operator kernel (stencil2.cu): picked by the
+  // layout of the second TMA operator kernel (stencil2.cuh): picked by the
   // autotuner among 4, 1 and 3 for complex64, or fixed by FDFD_OPERATOR_V2
   // at create: 0 = first TMA kernel only; 4 (default) = two
   // rows per warp, 4-slot ring, ε diagonal from global memory, 2 CTAs per SM;
@@ -207,7 +207,7 @@ template <typename R> OpArgs<R> op_args(const fdfd_handle *h);
 template <typename R>
 int launch_apply_fin(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y, int epi,
                      const typename CT<R>::C *aux0, int fin, KScalars *sc, bool transpose);
-// the second TMA operator kernel (stencil2.cu); FDFD_ERR_UNSUPPORTED when it
+// the second TMA operator kernel (stencil2.cuh); FDFD_ERR_UNSUPPORTED when it
 // does not serve the call (the caller then uses the first one)
 template <typename R>
 int launch_apply_v2(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y, int epi,

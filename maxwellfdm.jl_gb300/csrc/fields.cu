@@ -19,9 +19,9 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <type_traits>
 
 #include "operator_common.cuh"
+#include "pair_math.cuh"
 
 namespace fdfd {
 
@@ -61,32 +61,10 @@ __device__ __forceinline__ double2 mul_c(double2 c, double2 d) {
   return r;
 }
 
-// f(XR, YR, ZR) for three warp-uniform flags as compile-time constants: one
-// branch to a body that holds only the FP64 instructions it needs (branches
-// inside the body become predicated instructions, which take the pipe too:
-// 131 µs against 84 for k_h_from_e at 128×128×64).
-template <typename F>
-__device__ __forceinline__ void by_axis(bool xr, bool yr, bool zr, F f) {
-  using T = std::true_type;
-  using N = std::false_type;
-  if (xr) {
-    if (yr) {
-      if (zr) f(T{}, T{}, T{});
-      else f(T{}, T{}, N{});
-    } else {
-      if (zr) f(T{}, N{}, T{});
-      else f(T{}, N{}, N{});
-    }
-  } else {
-    if (yr) {
-      if (zr) f(N{}, T{}, T{});
-      else f(N{}, T{}, N{});
-    } else {
-      if (zr) f(N{}, N{}, T{});
-      else f(N{}, N{}, N{});
-    }
-  }
-}
+// by_axis (pair_math.cuh) branches once per cell to a body that holds only
+// the FP64 instructions it needs; with the tests inside the body they became
+// predicated instructions, which take the pipe too: 131 µs against 84 for
+// k_h_from_e at 128×128×64.
 
 // REALW: ω is real, so i/ω = i·s and s is folded into the curl coefficients.
 // BL: some axis is periodic.

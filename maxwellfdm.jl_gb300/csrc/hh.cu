@@ -9,7 +9,7 @@
 // Like the reference (whose Pε \ Cₘ needs a diagonal Pε), this path takes a
 // diagonal ε only.
 //
-// Kernel: the mirror image of the second E operator kernel (stencil2.cu).  A
+// Kernel: the mirror image of the second E operator kernel (stencil2.cuh).  A
 // CTA owns a 32 × TYT (x, y) tile, warp w rows RW·w …, lane = x, and marches
 // along z over a ring of H planes filled by cp.async (any Nx, periodic
 // axes).  Each thread keeps its cells' H and E' of two planes in registers:

@@ -1,7 +1,9 @@
-// Complex arithmetic of the z-marching operator kernels (stencil2.cu, hh.cu):
+// Complex arithmetic of the z-marching operator kernels (stencil2.cuh, hh.cu):
 // paired FP32 instructions for complex64, scalar FP64 for complex128, and
 // neighbour exchange within a warp.
 #pragma once
+
+#include <type_traits>
 
 #include "operator_common.cuh"
 
@@ -81,5 +83,46 @@ __device__ __forceinline__ double2 pmix(double2 u, double s, double2 v, double t
 // (u + v)·s for real s
 __device__ __forceinline__ float2 psums(float2 u, float2 v, float s) { return __fmul2_rn(__fadd2_rn(u, v), f2(s)); }
 __device__ __forceinline__ double2 psums(double2 u, double2 v, double s) { return cscale(cadd(u, v), s); }
+
+// complex128 runs at the FP64 pipe's rate — a warp's FP64 instruction holds
+// it for 64 cycles, predicated off or not — so its products take only the
+// parts they need, axis by axis: a·u − b·v with a real when AR, b when BR.
+template <bool AR, bool BR>
+__device__ __forceinline__ double2 pdiff_by(double2 a, double2 u, double2 b, double2 v) {
+  double2 t = make_double2(a.x * u.x, a.x * u.y);
+  if (!AR) t = make_double2(fma(-a.y, u.y, t.x), fma(a.y, u.x, t.y));
+  t = make_double2(fma(-b.x, v.x, t.x), fma(-b.x, v.y, t.y));
+  if (!BR) t = make_double2(fma(b.y, v.y, t.x), fma(-b.y, v.x, t.y));
+  return t;
+}
+
+// f(XR, YR, ZR) for three warp-uniform flags as compile-time constants: one
+// branch to a body that holds only the FP64 instructions it needs (FINE =
+// false: only the all-real and the all-complex body, less code).
+template <bool FINE = true, typename F>
+__device__ __forceinline__ void by_axis(bool xr, bool yr, bool zr, F f) {
+  using T = std::true_type;
+  using N = std::false_type;
+  if constexpr (!FINE) {
+    if (xr && yr && zr) f(T{}, T{}, T{});
+    else f(N{}, N{}, N{});
+  } else if (xr) {
+    if (yr) {
+      if (zr) f(T{}, T{}, T{});
+      else f(T{}, T{}, N{});
+    } else {
+      if (zr) f(T{}, N{}, T{});
+      else f(T{}, N{}, N{});
+    }
+  } else {
+    if (yr) {
+      if (zr) f(N{}, T{}, T{});
+      else f(N{}, T{}, N{});
+    } else {
+      if (zr) f(N{}, N{}, T{});
+      else f(N{}, N{}, N{});
+    }
+  }
+}
 
 }  // namespace fdfd

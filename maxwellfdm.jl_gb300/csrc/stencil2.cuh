@@ -34,6 +34,8 @@
 // periodic axes) k_apply_cp runs the same march on a ring filled by cp.async;
 // the first TMA kernel (stencil.cu) keeps the S-weighted COCG epilogue and
 // the plain-load kernel Aᵀ.
+#pragma once
+
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -263,6 +265,17 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   const bool rx = i0 - 1 >= a.rlo[0] && i0 + TX <= a.rhi[0];
   const bool ry = j0 + jw - 1 >= a.rlo[1] && j0 + jw + RW <= a.rhi[1];
 
+  // complex128: real coefficients axis by axis, of the warp's own cells and of
+  // the halo row j0−1 and column i0−1
+  constexpr bool FP64 = sizeof(R) == 8;
+  const int ilast = min(i0 + TX, a.N[0]) - 1;
+  const bool xr = i0 >= a.rlo[0] && ilast <= a.rhi[0], xrh = i0 - 1 >= a.rlo[0] && i0 - 1 <= a.rhi[0];
+  const int gj0 = j0 + jw;
+  const bool yr = gj0 >= a.rlo[1] && gj0 + RW - 1 <= a.rhi[1];
+  const bool yrh = j0 - 1 >= a.rlo[1] && j0 - 1 <= a.rhi[1];
+  const bool yrt = j0 >= a.rlo[1] && min(j0 + TYT, a.N[1]) - 1 <= a.rhi[1];
+  const bool rowin = !FP64 || RW > 1 || gj0 < a.N[1];  // the warp has a row to compute
+
   __syncthreads();
   // the copies of plane q into ring slot s: the E tile, and the off-diagonal
   // ε of the tile when plane q or q−1 carries off-diagonal terms (the
@@ -304,8 +317,10 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   // The march over the chunk.  WALL: the CTA touches a low PEC wall (i0 or j0
   // = 0, or planes from k0 − 1 ≤ 0) and may meet pinned DOFs; the other CTAs
   // run without the pin selects.
-  auto march = [&](auto wall_tag) {
+  // W2R: ω² is real (complex128; complex64 tests it where it is used).
+  auto march = [&](auto wall_tag, auto w2_tag) {
     constexpr bool WALL = decltype(wall_tag)::value;
+    constexpr bool W2R = decltype(w2_tag)::value;
     bool ok = true;
     if constexpr (CPA) {
       // planes k0−1 … k0+1 have landed (the newest group may be in flight)
@@ -355,8 +370,17 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         const C mz = zif(pin_i || pin_j[r], ev2<R, RW, NS>(sm, 0, 2, jj, lane));
         const C mzi = zif(pin_j[r], ev2<R, RW, NS>(sm, 0, 2, jj, lane + 1));
         const C mzj = zif(pin_i, ev2<R, RW, NS>(sm, 0, 2, jj + 1, lane));
-        hxp[r] = csub(cmul(cmy, csub(mzj, mz)), cmul(cmzm, csub(eo[r][1], my)));
-        hyp[r] = csub(cmul(cmzm, csub(eo[r][0], mx)), cmul(cmx, csub(mzi, mz)));
+        if constexpr (FP64) {
+          const C dy = csub(mzj, mz), dz = csub(eo[r][1], my), ex_ = csub(eo[r][0], mx), dx = csub(mzi, mz);
+          by_axis<W2R>(xr, yr, kfirst >= a.rlo[2] && kfirst <= a.rhi[2], [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            hxp[r] = pdiff_by<YR, ZR>(cmy, dy, cmzm, dz);
+            hyp[r] = pdiff_by<ZR, XR>(cmzm, ex_, cmx, dx);
+          });
+        } else {
+          hxp[r] = csub(cmul(cmy, csub(mzj, mz)), cmul(cmzm, csub(eo[r][1], my)));
+          hyp[r] = csub(cmul(cmzm, csub(eo[r][0], mx)), cmul(cmx, csub(mzi, mz)));
+        }
         ezp[r] = mz;
       }
     }
@@ -397,7 +421,8 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         phase ^= 1u << s1;
       }
       const C cmz = zt[p0], cez = zt[KC2 + p0];
-      const bool rc = rx && ry && k >= a.rlo[2] && k <= a.rhi[2];
+      const bool zr = k >= a.rlo[2] && k <= a.rhi[2];
+      const bool rc = rx && ry && zr;
       // E(k+1) at the thread's cells (true values; the curls take the pinned
       // entries as 0)
       C en[RW][3];
@@ -423,7 +448,15 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
           ezj = zif(pin_i, ev2<R, RW, NS>(sm, s0, 2, jj + 1, lane));
         }
         const C eny = zif(pin_i, en[r][1]), enx = zif(pin_j[r], en[r][0]);
-        if (rc) {
+        if constexpr (FP64) {
+          if (rowin)
+            by_axis<W2R>(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
+              constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+              hx[r] = pdiff_by<YR, ZR>(cmy, csub(ezj, eo[r][2]), cmz, csub(eny, eo[r][1]));
+              hy[r] = pdiff_by<ZR, XR>(cmz, csub(enx, eo[r][0]), cmx, csub(ezi, eo[r][2]));
+              hz[r] = pdiff_by<XR, YR>(cmx, csub(eyi, eo[r][1]), cmy, csub(exj, eo[r][0]));
+            });
+        } else if (rc) {
           hx[r] = pdiff<true>(cmy, psub(ezj, eo[r][2]), cmz, psub(eny, eo[r][1]));
           hy[r] = pdiff<true>(cmz, psub(enx, eo[r][0]), cmx, psub(ezi, eo[r][2]));
           hz[r] = pdiff<true>(cmx, psub(eyi, eo[r][1]), cmy, psub(exj, eo[r][0]));
@@ -444,8 +477,16 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         const C mz = zif(pin_i, ev2<R, RW, NS>(sm, s0, 2, -1, lane));
         const C myk = zif(pin_i, ev2<R, RW, NS>(sm, s1, 1, -1, lane));
         const C myi = zif(z0, ev2<R, RW, NS>(sm, s0, 1, -1, lane + 1));
-        xc_.hx[0][lane] = csub(cmul(cmy, csub(eo[0][2], mz)), cmul(cmz, csub(myk, my)));
-        xc_.hz[0][lane] = csub(cmul(cmx, csub(myi, my)), cmul(cmy, csub(eo[0][0], mx)));
+        if constexpr (FP64) {
+          by_axis<W2R>(xr, yrh, zr, [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            xc_.hx[0][lane] = pdiff_by<YR, ZR>(cmy, csub(eo[0][2], mz), cmz, csub(myk, my));
+            xc_.hz[0][lane] = pdiff_by<XR, YR>(cmx, csub(myi, my), cmy, csub(eo[0][0], mx));
+          });
+        } else {
+          xc_.hx[0][lane] = csub(cmul(cmy, csub(eo[0][2], mz)), cmul(cmz, csub(myk, my)));
+          xc_.hz[0][lane] = csub(cmul(cmx, csub(myi, my)), cmul(cmy, csub(eo[0][0], mx)));
+        }
       } else if (w == 1 && lane < TYT) {
         // column i0−1, tile row `lane` (reaches only pinned outputs when i0 = 0)
         const int jj = lane;
@@ -458,8 +499,16 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         const C exj = zif(z0, ev2<R, RW, NS>(sm, s0, 0, jj + 1, -1));
         const C ey0 = zif(pi0 || z0, ev2<R, RW, NS>(sm, s0, 1, jj, 0));
         const C ez0 = zif(pi0 || pj, ev2<R, RW, NS>(sm, s0, 2, jj, 0));
-        xc_.hyh[jj] = csub(cmul(cmz, csub(ex_k1, ex_k)), cmul(cmh, csub(ez0, ez_)));
-        xc_.hzh[jj] = csub(cmul(cmh, csub(ey0, ey_)), cmul(cmy, csub(exj, ex_k)));
+        if constexpr (FP64) {
+          by_axis<W2R>(xrh, yrt, zr, [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            xc_.hyh[jj] = pdiff_by<ZR, XR>(cmz, csub(ex_k1, ex_k), cmh, csub(ez0, ez_));
+            xc_.hzh[jj] = pdiff_by<XR, YR>(cmh, csub(ey0, ey_), cmy, csub(exj, ex_k));
+          });
+        } else {
+          xc_.hyh[jj] = csub(cmul(cmz, csub(ex_k1, ex_k)), cmul(cmh, csub(ez0, ez_)));
+          xc_.hzh[jj] = csub(cmul(cmh, csub(ey0, ey_)), cmul(cmy, csub(exj, ex_k)));
+        }
       }
       // ---- off-diagonal ε: corner terms of this warp's cells, folded into the
       // diagonal term (½ of each of the two corners around an output; pinned
@@ -582,7 +631,15 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
           hyim = xc_.hyh[jj];
         }
         C yx, yy, yz;
-        if (rc) {
+        if (!rowin) break;  // nothing below it in this plane but outputs
+        if constexpr (FP64) {
+          by_axis<W2R>(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            yx = pdiff_by<YR, ZR>(cey, csub(hz[r], hzjm), cez, csub(hy[r], hyp[r]));
+            yy = pdiff_by<ZR, XR>(cez, csub(hx[r], hxp[r]), cex, csub(hz[r], hzim));
+            yz = pdiff_by<XR, YR>(cex, csub(hy[r], hyim), cey, csub(hx[r], hxjm));
+          });
+        } else if (rc) {
           yx = pdiff<true>(cey, psub(hz[r], hzjm), cez, psub(hy[r], hyp[r]));
           yy = pdiff<true>(cez, psub(hx[r], hxp[r]), cex, psub(hz[r], hzim));
           yz = pdiff<true>(cex, psub(hy[r], hyim), cey, psub(hx[r], hxjm));
@@ -611,24 +668,39 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
           if (py) t1 = ev2<R, RW, NS>(sm, s0, 1, jj, lane);
           if (pz) t2 = ev2<R, RW, NS>(sm, s0, 2, jj, lane);
         }
-        C d0 = pfma(t0, e0, od[r][0]), d1 = pfma(t1, e1, od[r][1]), d2 = pfma(t2, e2, od[r][2]);
-        if (offd) {
-          if (lane == TX - 1 && !px) d0 = pfma(xc_.xce[jj], R(0.5), d0);
-          if (r == RW - 1 && !py) d1 = pfma(xc_.yc[w + 1][lane], R(0.5), d1);
-        }
         if (WALL) {
           if (px) yx = czero<C>();
           if (py) yy = czero<C>();
           if (pz) yz = czero<C>();
         }
-        if (a.w2.y == R(0)) {
-          yx = pfma(d0, -a.w2.x, yx);
-          yy = pfma(d1, -a.w2.x, yy);
-          yz = pfma(d2, -a.w2.x, yz);
+        if constexpr (FP64 && W2R) {
+          // −ω²ε as one factor; the corner terms only where there are any
+          yx = pfma(t0, -a.w2.x * e0, yx);
+          yy = pfma(t1, -a.w2.x * e1, yy);
+          yz = pfma(t2, -a.w2.x * e2, yz);
+          if (offd) {
+            C d0 = od[r][0], d1 = od[r][1];
+            if (lane == TX - 1 && !px) d0 = pfma(xc_.xce[jj], R(0.5), d0);
+            if (r == RW - 1 && !py) d1 = pfma(xc_.yc[w + 1][lane], R(0.5), d1);
+            yx = pfma(d0, -a.w2.x, yx);
+            yy = pfma(d1, -a.w2.x, yy);
+            yz = pfma(od[r][2], -a.w2.x, yz);
+          }
         } else {
-          yx = csub(yx, cmul(a.w2, d0));
-          yy = csub(yy, cmul(a.w2, d1));
-          yz = csub(yz, cmul(a.w2, d2));
+          C d0 = pfma(t0, e0, od[r][0]), d1 = pfma(t1, e1, od[r][1]), d2 = pfma(t2, e2, od[r][2]);
+          if (offd) {
+            if (lane == TX - 1 && !px) d0 = pfma(xc_.xce[jj], R(0.5), d0);
+            if (r == RW - 1 && !py) d1 = pfma(xc_.yc[w + 1][lane], R(0.5), d1);
+          }
+          if (!FP64 && a.w2.y == R(0)) {
+            yx = pfma(d0, -a.w2.x, yx);
+            yy = pfma(d1, -a.w2.x, yy);
+            yz = pfma(d2, -a.w2.x, yz);
+          } else {
+            yx = csub(yx, cmul(a.w2, d0));
+            yy = csub(yy, cmul(a.w2, d1));
+            yz = csub(yz, cmul(a.w2, d2));
+          }
         }
         if (act[r]) {
           const int ce = cell[r];
@@ -683,8 +755,14 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
     }
   };
   // a chunk starting at plane 1 reads the z = 0 wall plane as its plane k−1
-  if (i0 == 0 || j0 == 0 || k0 <= 1) march(std::true_type{});
-  else march(std::false_type{});
+  if constexpr (FP64) {
+    // the selects of the wall form are free next to the FP64 pipe
+    if (a.w2.y == R(0)) march(std::true_type{}, std::true_type{});
+    else march(std::true_type{}, std::false_type{});
+  } else {
+    if (i0 == 0 || j0 == 0 || k0 <= 1) march(std::true_type{}, std::false_type{});
+    else march(std::false_type{}, std::false_type{});
+  }
 
   if (CPA) cp_async_wait<0>();
   if (!CPA && !run) {
@@ -902,9 +980,5 @@ int launch_apply_v2(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::
   }
   return FDFD_ERR_UNSUPPORTED;
 }
-template int launch_apply_v2<float>(fdfd_handle *, const float2 *, float2 *, int, const float2 *, int, KScalars *, int,
-                                    bool);
-template int launch_apply_v2<double>(fdfd_handle *, const double2 *, double2 *, int, const double2 *, int, KScalars *,
-                                     int, bool);
 
 }  // namespace fdfd

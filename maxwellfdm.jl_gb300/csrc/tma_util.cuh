@@ -1,4 +1,4 @@
-// Inline-PTX helpers of the TMA operator kernels (stencil.cu, stencil2.cu):
+// Inline-PTX helpers of the TMA operator kernels (stencil.cu, stencil2.cuh):
 // shared-memory addresses, mbarrier set-up and bounded waits, and the tiled
 // bulk tensor copies (cp.async.bulk.tensor) that complete on an mbarrier.
 #pragma once
