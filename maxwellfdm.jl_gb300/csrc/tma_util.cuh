@@ -87,7 +87,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, long lo
 // try_wait may suspend the thread for up to `hint_ns` until the phase
 // completes, so a late copy costs a few polls rather than a spinning loop.
 __device__ __forceinline__ bool mbar_wait_sleep(uint32_t bar, uint32_t parity, long long limit, uint32_t hint_ns) {
-  if (limit <= 0) return mbar_wait(bar, parity, 0);
+  if (mbar_wait(bar, parity, 0)) return true;  // landed already: no clock to read
+  if (limit <= 0) return false;
   const long long t0 = clock64();
   while (true) {
     uint32_t done;
