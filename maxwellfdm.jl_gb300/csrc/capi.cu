@@ -242,9 +242,10 @@ static int ensure_eps_buffers(fdfd_handle *h, bool off) {
 }
 
 // After new ε data: refresh the FP32 copies from the FP64 masters and rebuild
-// the flags (refresh = false where the caller wrote them itself), retune
+// the flags (refresh = false where the caller wrote them itself, corners:
+// the number of corners where it queued their lists as well), retune
 // where the off-diagonal tensor came or went.
-int finish_eps(fdfd_handle *h, bool refresh) {
+int finish_eps(fdfd_handle *h, bool refresh, const unsigned *corners = nullptr) {
   const long long n = 3 * h->ncell;
   int rc = FDFD_OK;
   if (refresh) {
@@ -258,6 +259,7 @@ int finish_eps(fdfd_handle *h, bool refresh) {
     rc = build_oflags(h);
     if (rc) return rc;
   }
+  if ((rc = build_corner_lists(h, corners))) return rc;
   rc = cuda_check(h, cudaStreamSynchronize(h->stream), "stream sync");
   if (rc == FDFD_OK && h->tuned_off >= 0 && h->tuned_off != (h->has_off ? 1 : 0)) {
     // retune the z-chunk for the new operator; captured graphs hold the old
@@ -535,6 +537,9 @@ void fdfd_destroy(fdfd_handle *h) {
     cudaFree(h->oflag_rows[1]);
     cudaFree(h->smask);
     cudaFree(h->setup_scratch);
+    cudaFree(h->corner_list);
+    cudaFree(h->corner_mask);
+    cudaFree(h->corners);
     cudaFree(h->work[0]);
     cudaFree(h->work[1]);
   }
@@ -770,6 +775,10 @@ static fdfd_handle *make_worker(fdfd_handle *p, int *rc) {
   w->oflag_rows[0] = p->oflag_rows[0];
   w->oflag_rows[1] = p->oflag_rows[1];
   w->has_off = p->has_off;
+  w->corner_list = p->corner_list;
+  w->corner_mask = p->corner_mask;
+  w->corners = p->corners;
+  w->corner_ok = p->corner_ok;
   w->smask = p->smask;
   w->slice2d = p->slice2d;
   w->ft = p->ft;

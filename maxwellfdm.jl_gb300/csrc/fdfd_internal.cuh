@@ -138,6 +138,12 @@ struct fdfd_handle {
   uint8_t *oflag = nullptr;
   uint8_t *oflag_rows[2] = {nullptr, nullptr};  // the same per x tile, group of 1 / 2 rows and plane
   bool has_off = false;
+  // the non-zero off-diagonal corners per (32×16 tile, plane), for complex64 on PEC walls (stencil3.cu)
+  int2 *corner_list = nullptr;
+  unsigned long long *corner_mask = nullptr;
+  int4 *corners = nullptr;
+  size_t corner_cap = 0;
+  bool corner_ok = false;  // built for the current ε
   void *setup_scratch = nullptr;  // kept between fdfd_smooth_objects calls (at most 64 MiB)
   size_t setup_bytes = 0;
   uint8_t *smask = nullptr;  // 4*ncell smoothing mask (from fdfd_smooth_objects)
@@ -171,13 +177,14 @@ struct fdfd_handle {
   // gives up (≈1 s); FDFD_WAIT_LIMIT_CLOCKS lowers it, so that a test can
   // make a wait run out and see FDFD_ERR_TIMEOUT without hanging anything
   long long wait_limit = 1ll << 31;
-  // layout of the second TMA operator kernel (stencil2.cuh): picked by the
-  // autotuner among 4, 1 and 3 for complex64, or fixed by FDFD_OPERATOR_V2
+  // layout of the second and third operator kernels: picked by the
+  // autotuner among 4, 5, 1 and 3 for complex64, or fixed by FDFD_OPERATOR_V2
   // at create: 0 = first TMA kernel only; 4 (default) = two
   // rows per warp, 4-slot ring, ε diagonal from global memory, 2 CTAs per SM;
   // 1 = one row per warp, 4 slots, 3 CTAs; 2 = two rows, 3 slots, ε diagonal
-  // through the ring; 3 = as 1 with 2 CTAs.  Measured at 320³ with 400
-  // spheres: 4: 439 µs, 2: 496 µs, 3: 494 µs, 1: 556 µs, first kernel 525 µs.
+  // through the ring; 3 = as 1 with 2 CTAs; 5 = the third kernel (stencil3.cu).
+  // Measured at 320³ with 400 spheres: 5: 392 µs, 4: 415 µs, 3: 424 µs; 2 and
+  // the first kernel above 490 µs.
   int op_variant = 4;
   int tuned_off = -1;                 // has_off at the last tuning (−1: not tuned yet)
   std::string err;
@@ -212,6 +219,12 @@ int launch_apply_fin(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>:
 template <typename R>
 int launch_apply_v2(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y, int epi,
                     const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc, bool tma);
+// the third operator kernel (stencil3.cu: complex64, PEC walls), as above
+bool v3_serves(const fdfd_handle *h);  // the third kernel takes this grid and ε
+int launch_apply_v3(fdfd_handle *h, const float2 *x, float2 *y, int epi, const float2 *aux0, int fin, KScalars *sc,
+                    int kc, bool tma);
+int build_corner_lists(fdfd_handle *h, const unsigned *queued);
+int queue_corner_lists(fdfd_handle *h, unsigned *next, bool *queued);
 // number of blocks launch_apply uses (reduction buffer sizing)
 int apply_blocks(const fdfd_handle *h);
 // pick the z-chunk length per precision by timing (stencil.cu)

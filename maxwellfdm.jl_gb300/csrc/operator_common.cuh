@@ -20,6 +20,9 @@ struct Extra {
   int ediag_tma;      // second TMA kernel: ε diagonal staged through the ring
   const uint8_t *oflag_w;  // second TMA kernel: off-diagonal flags per x tile, warp strip and plane
   long long wait_limit;  // TMA kernel: SM clocks a pipeline wait may take before it gives up
+  const int4 *corners;       // third kernel: non-zero off-diagonal corners (position in the tile, ε_xy, ε_yz, ε_zx), or null
+  const int2 *corner_list;   // third kernel: (start, count) in it per 32×16 tile and plane
+  const unsigned long long *corner_mask;  // and the mask of each of its 17 corner rows
   const int4 *work;      // second TMA kernel: (x tile, y tile, k0, k1) per block, or null (uniform chunks)
 };
 

@@ -31,7 +31,7 @@
 
 namespace fdfd {
 
-int finish_eps(fdfd_handle *h, bool refresh);
+int finish_eps(fdfd_handle *h, bool refresh, const unsigned *corners);
 int ensure_oflags(fdfd_handle *h);
 
 struct DevObj {
@@ -674,14 +674,18 @@ int smooth_objects_impl(fdfd_handle *h, const double *const lprim[3], const fdfd
     k_design_off<<<152 * 8, 256, 0, st>>>(N0, N1, N2, dd, h->eoff64, h->smask);
     if ((rc = cuda_check(h, cudaGetLastError(), "design kernels"))) return rc;
   }
-  unsigned int nnz = 0;
-  cudaMemcpyAsync(&nnz, A.nnz, sizeof(unsigned int), cudaMemcpyDeviceToHost, st);
+  // the corner lists of the new ε, so that their count comes with nnz (a
+  // design region's flags are not yet up to date)
+  bool lists = false;
+  if (!design && (rc = queue_corner_lists(h, A.nnz + 1, &lists))) return rc;
+  unsigned int cnt[2] = {0, 0};  // nnz, corners
+  cudaMemcpyAsync(cnt, A.nnz, sizeof(cnt), cudaMemcpyDeviceToHost, st);
   if ((rc = cuda_check(h, cudaStreamSynchronize(st), "smoothing sync"))) return rc;
   // design zeroing can only remove off-diagonals; keep the flag conservative
-  h->has_off = nnz > 0;
+  h->has_off = cnt[0] > 0;
   // the FP32 copies and the flags are written already, except where a design
   // region changed ε since
-  return finish_eps(h, design != nullptr);
+  return finish_eps(h, design != nullptr, lists ? &cnt[1] : nullptr);
 }
 
 }  // namespace fdfd

@@ -814,6 +814,9 @@ Extra<R> make_extra(const fdfd_handle *h) {
   ex.eoff_tma = 0;
   ex.ediag_tma = 0;
   ex.oflag_w = nullptr;
+  ex.corners = nullptr;
+  ex.corner_list = nullptr;
+  ex.corner_mask = nullptr;
   ex.wait_limit = h->wait_limit;
   ex.work = nullptr;
   const C *coef;
@@ -1072,10 +1075,11 @@ int autotune_kchunk(fdfd_handle *h) {
   const int cand[] = {4, 6, 8, 12, 16, 24, 32, 48, 64};
   const bool verbose = std::getenv("FDFD_VERBOSE") != nullptr;
   // complex64 also picks the tile layout of the second TMA kernel (two rows
-  // per warp with a 4-slot ring; one row per warp with 3 or 2 CTAs per SM)
-  // unless FDFD_OPERATOR_V2 fixed it; complex128 has one layout
+  // per warp with a 4-slot ring; one row per warp with 3 or 2 CTAs per SM) or
+  // the third kernel (5), unless FDFD_OPERATOR_V2 fixed it; complex128 has one
+  // layout
   const bool tune_layout = h->op_variant != 0 && std::getenv("FDFD_OPERATOR_V2") == nullptr;
-  const int layouts_c64[] = {4, 1, 3};
+  const int layouts_c64[] = {4, 5, 1, 3};
   int sms = 152;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess) {
     cudaGetLastError();
@@ -1118,9 +1122,12 @@ int autotune_kchunk(fdfd_handle *h) {
     // FDFD_SCHEDULE=w takes the w-wave schedule (weight 1) untimed, 0 none
     const char *fs = std::getenv("FDFD_SCHEDULE");
     const int forced = fs != nullptr ? std::atoi(fs) : -1;
-    const int nlay = (prec == 1 && tune_layout) ? 3 : 1;
+    const int nlay = (prec == 1 && tune_layout) ? 4 : 1;
     for (int li = 0; li < nlay && rc == FDFD_OK; ++li) {
-      if (prec == 1 && tune_layout) h->op_variant = layouts_c64[li];
+      if (prec == 1 && tune_layout) {
+        if (layouts_c64[li] == 5 && !v3_serves(h)) continue;
+        h->op_variant = layouts_c64[li];
+      }
       int last_chunks = -1;
       for (int kc : cand) {
         if (kc > h->N[2] && last_chunks == 1) break;

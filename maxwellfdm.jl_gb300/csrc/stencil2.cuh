@@ -992,6 +992,12 @@ int launch_apply_v2(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::
                     const typename CT<R>::C *aux0, int fin, KScalars *sc, int kc, bool tma) {
   // cell offsets are 32-bit in the kernel
   if (h->op_variant == 0 || 3 * h->ncell >= (1ll << 31)) return FDFD_ERR_UNSUPPORTED;
+  if constexpr (sizeof(R) == 4) {
+    if (h->op_variant == 5) {
+      const int rc = launch_apply_v3(h, x, y, epi, aux0, fin, sc, kc, tma);
+      if (rc != FDFD_ERR_UNSUPPORTED) return rc;
+    }
+  }
   switch (epi) {
     case EPI_STORE: return launch_any_e<R, EPI_STORE>(h, x, y, aux0, fin, sc, kc, tma);
     case EPI_RESID: return launch_any_e<R, EPI_RESID>(h, x, y, aux0, fin, sc, kc, tma);

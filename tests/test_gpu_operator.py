@@ -281,3 +281,36 @@ def test_cp_async_ring(pkg, oracle, monkeypatch, N, bloch, kc):
     assert np.linalg.norm(A.matvec(x, "c128") - ref) <= TOL64 * np.linalg.norm(ref)
     assert np.linalg.norm(A.matvec(x, "c64") - ref) <= TOL32 * np.linalg.norm(ref)
     A.close()
+
+
+@pytest.mark.parametrize("kc", [0, 1, 3])
+@pytest.mark.parametrize("N", [(32, 16, 4), (33, 17, 5), (34, 15, 7), (64, 33, 2), (70, 48, 6)])
+def test_corner_lists(pkg, oracle, monkeypatch, N, kc):
+    """The third operator kernel gives the oracle's A x for lists of every
+    length: none, a few corners, more than its first 64 and 128 per
+    tile-plane, and every corner of the grid — on tiles of one column or row
+    more or less than whole ones, even Nx (TMA) and odd (cp.async), at forced
+    z-chunks, with new ε of another density on the same handle each time and
+    a solve between them (whose graphs hold the lists)."""
+    monkeypatch.setenv("FDFD_OPERATOR_V2", "5")
+    if kc:
+        monkeypatch.setenv("FDFD_KCHUNK", str(kc))
+    O = oracle
+    g = O.Grid(_nonuniform(N, 5), (False, False, False))
+    om = 2 * np.pi / 1.5  # ω² ε dominates: a solve takes few iterations
+    npml = tuple(0 if n < 6 else 2 for n in N)
+    sdl_e, sdl_m = O.stretched_dl(g, om, (npml, npml))
+    Ce, Cm = O.create_curls(g, sdl_e, sdl_m, (0.0, 0.0, 0.0))
+    A = pkg.FDFDOperator(g.N, om, sdl_e, sdl_m, g.isbloch, (1.0, 1.0, 1.0))
+    rng = np.random.default_rng(4)
+    x = _rand(A.n, 12)
+    for density in (0.01, 1.0, 0.0, 0.2, 0.4):
+        ed = rng.uniform(4.0, 12.0, N + (3,))
+        eo = rng.uniform(-1.0, 1.0, N + (3,)) * (rng.uniform(0.0, 1.0, N + (1,)) < density)
+        A.set_eps(ed, eo)
+        Aref = O.create_A(om, O.create_paramop(g, ed, eo, sdl_e, sdl_m, (0.0, 0.0, 0.0)), Ce, Cm)
+        ref = Aref @ x
+        assert np.linalg.norm(A.matvec(x, "c64") - ref) <= TOL32 * np.linalg.norm(ref)
+        e, _ = A.solve(ref, tol=1e-6, maxit=400)
+        assert np.linalg.norm(Aref @ e - ref) <= 1.01e-6 * np.linalg.norm(ref)
+    A.close()
