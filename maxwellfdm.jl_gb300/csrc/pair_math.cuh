@@ -84,26 +84,18 @@ __device__ __forceinline__ double2 pmix(double2 u, double s, double2 v, double t
 __device__ __forceinline__ float2 psums(float2 u, float2 v, float s) { return __fmul2_rn(__fadd2_rn(u, v), f2(s)); }
 __device__ __forceinline__ double2 psums(double2 u, double2 v, double s) { return cscale(cadd(u, v), s); }
 
-// A curl coefficient as the products below take it: complex64 with its real
-// part twice (the operand of a paired multiply; 16 bytes, one shared-memory
-// load), complex128 as it is.
+// A complex64 curl coefficient as csum takes it: its real part twice (the
+// operand of a paired multiply; 16 bytes, one shared-memory load).
 template <typename R> struct Coef;
 template <> struct __align__(16) Coef<float> {
   float2 xx;
   float y, pad;
 };
-template <> struct Coef<double> {
-  double x, y;
-};
 __device__ __forceinline__ Coef<float> coef_of(float2 c) { return {make_float2(c.x, c.x), c.y, 0.f}; }
-__device__ __forceinline__ Coef<double> coef_of(double2 c) { return {c.x, c.y}; }
 
-// a·u + b·v for coefficients a (real when AR) and b (real when BR).
-// complex64: the real parts in paired instructions, the imaginary ones in
-// scalar instructions (paired ones would first swap the halves of u and v).
-// complex128 runs at the FP64 pipe's rate — a warp's FP64 instruction holds
-// it for 64 cycles, predicated off or not — so its products take only the
-// parts they need, axis by axis.
+// a·u + b·v for coefficients a (real when AR) and b (real when BR): the real
+// parts in paired instructions, the imaginary ones in scalar instructions
+// (paired ones would first swap the halves of u and v).
 template <bool AR, bool BR>
 __device__ __forceinline__ float2 csum(const Coef<float> &a, float2 u, const Coef<float> &b, float2 v) {
   if constexpr (AR && BR) {
@@ -115,12 +107,16 @@ __device__ __forceinline__ float2 csum(const Coef<float> &a, float2 u, const Coe
     return __ffma2_rn(a.xx, u, t);
   }
 }
+
+// complex128 runs at the FP64 pipe's rate — a warp's FP64 instruction holds
+// it for 64 cycles, predicated off or not — so its products take only the
+// parts they need, axis by axis: a·u − b·v with a real when AR, b when BR.
 template <bool AR, bool BR>
-__device__ __forceinline__ double2 csum(const Coef<double> &a, double2 u, const Coef<double> &b, double2 v) {
+__device__ __forceinline__ double2 pdiff_by(double2 a, double2 u, double2 b, double2 v) {
   double2 t = make_double2(a.x * u.x, a.x * u.y);
   if (!AR) t = make_double2(fma(-a.y, u.y, t.x), fma(a.y, u.x, t.y));
-  t = make_double2(fma(b.x, v.x, t.x), fma(b.x, v.y, t.y));
-  if (!BR) t = make_double2(fma(-b.y, v.y, t.x), fma(b.y, v.x, t.y));
+  t = make_double2(fma(-b.x, v.x, t.x), fma(-b.x, v.y, t.y));
+  if (!BR) t = make_double2(fma(b.y, v.y, t.x), fma(-b.y, v.x, t.y));
   return t;
 }
 

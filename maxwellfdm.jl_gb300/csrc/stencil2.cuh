@@ -91,20 +91,14 @@ struct V2 {
   static constexpr int EXCH_OFF = ED_OFF + NS * ED_SLOT;
   static constexpr int XT_OFF = EXCH_OFF + 2 * (int)sizeof(Exch);
   static constexpr int XT_N = TX + 2;   // x coefficients of columns i0−1 … i0+32
-  // y and z: the curl coefficients cm, ce as the products take them (Coef),
-  // then the averaging weights wm, wp
-  using K = Coef<R>;
-  static constexpr int YK_OFF = XT_OFF + 4 * XT_N * (int)sizeof(C);
-  static constexpr int ZK_OFF = YK_OFF + 2 * (TYT + 2) * (int)sizeof(K);
-  static constexpr int YT_OFF = ZK_OFF + 2 * KC2 * (int)sizeof(K);
-  static constexpr int ZT_OFF = YT_OFF + 2 * (TYT + 2) * (int)sizeof(C);
-  static constexpr int ZF_OFF = ZT_OFF + 2 * KC2 * (int)sizeof(C);
+  static constexpr int YT_OFF = XT_OFF + 4 * XT_N * (int)sizeof(C);
+  static constexpr int ZT_OFF = YT_OFF + 4 * (TYT + 2) * (int)sizeof(C);
+  static constexpr int ZF_OFF = ZT_OFF + 4 * KC2 * (int)sizeof(C);
   static constexpr int ZA_OFF = ZF_OFF + KC2 * NW;  // per plane: any strip flagged
   static constexpr int BAR_OFF = (ZA_OFF + KC2 + 15) / 16 * 16;
   static constexpr int SMEM = BAR_OFF + NS * 8;
   static_assert(SLOT % 128 == 0 && EXCH_OFF % 128 == 0, "TMA destination alignment");
   static_assert(SMEM <= 227 * 1024, "shared memory per CTA");
-  static_assert(YK_OFF % 16 == 0, "coefficient alignment");
   static_assert(XW * 6 <= 256, "TMA box inner extent");
 };
 
@@ -152,9 +146,6 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   extern __shared__ __align__(128) unsigned char sm[];
   X *xch = reinterpret_cast<X *>(sm + G::EXCH_OFF);
   C *xt = reinterpret_cast<C *>(sm + G::XT_OFF);
-  using K = typename G::K;
-  K *yk = reinterpret_cast<K *>(sm + G::YK_OFF);
-  K *zk = reinterpret_cast<K *>(sm + G::ZK_OFF);
   C *yt = reinterpret_cast<C *>(sm + G::YT_OFF);
   C *zt = reinterpret_cast<C *>(sm + G::ZT_OFF);
   unsigned char *zf = sm + G::ZF_OFF;
@@ -162,8 +153,7 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   uint64_t *bars = reinterpret_cast<uint64_t *>(sm + G::BAR_OFF);
   pdl_trigger();
 
-  // (the shuffle tells the compiler that w is the same for the whole warp)
-  const int tid = threadIdx.x, lane = tid & 31, w = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   // the block's column (x tile, y tile) and planes [k0, k1): uniform
   // chunks of ex.kchunk planes, or an entry of the balanced schedule
   int bx = blockIdx.x, by = blockIdx.y, k0 = blockIdx.z * ex.kchunk, k1;
@@ -233,20 +223,20 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   }
   if (tid < TYT + 2) {  // y coefficients, tile rows −1 … TYT
     const int c = cidx(a, 1, j0 + tid - 1);
-    yk[tid] = coef_of(a.cm[1][c]);
-    yk[(TYT + 2) + tid] = coef_of(a.ce[1][c]);
-    yt[tid] = a.wm[1][c];
-    yt[(TYT + 2) + tid] = a.wp[1][c];
+    yt[tid] = a.cm[1][c];
+    yt[(TYT + 2) + tid] = a.ce[1][c];
+    yt[2 * (TYT + 2) + tid] = a.wm[1][c];
+    yt[3 * (TYT + 2) + tid] = a.wp[1][c];
   }
   {  // z coefficients and off-diagonal flags over planes kfirst … k1 (k1 − kfirst ≤ KCMAX + 1)
     const int t = tid - 64;
     const int q = kfirst + t;
     if (t >= 0 && t < KC2 && q <= k1) {
       const int c = cidx(a, 2, q);
-      zk[t] = coef_of(a.cm[2][c]);
-      zk[KC2 + t] = coef_of(a.ce[2][c]);
-      zt[t] = a.wm[2][c];
-      zt[KC2 + t] = a.wp[2][c];
+      zt[t] = a.cm[2][c];
+      zt[KC2 + t] = a.ce[2][c];
+      zt[2 * KC2 + t] = a.wm[2][c];
+      zt[3 * KC2 + t] = a.wp[2][c];
       // one flag per warp strip (RW rows): its outputs at plane q read a
       // non-zero off-diagonal ε (the 32×8 tile flags stand in when the
       // strip flags are absent)
@@ -270,17 +260,21 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
     }
   }
   const int cxi = cidx(a, 0, gi);
-  const K cmx = coef_of(a.cm[0][cxi]), cex = coef_of(a.ce[0][cxi]);
-  // where the curl coefficients are real, per axis: the warp's own cells, and
-  // the halo row j0−1 and column i0−1 (complex64 branches on all three axes
-  // of the own cells together, complex128 axis by axis)
+  const C cmx = a.cm[0][cxi], cex = a.ce[0][cxi];
+  // real coefficient ranges for this warp: columns i0−1 … i0+32, rows jw−1 … jw+RW
+  const bool rx = i0 - 1 >= a.rlo[0] && i0 + TX <= a.rhi[0];
+  const bool ry = j0 + jw - 1 >= a.rlo[1] && j0 + jw + RW <= a.rhi[1];
+
+  // complex128: real coefficients axis by axis, of the warp's own cells and of
+  // the halo row j0−1 and column i0−1
   constexpr bool FP64 = sizeof(R) == 8;
+  const int ilast = min(i0 + TX, a.N[0]) - 1;
+  const bool xr = i0 >= a.rlo[0] && ilast <= a.rhi[0], xrh = i0 - 1 >= a.rlo[0] && i0 - 1 <= a.rhi[0];
   const int gj0 = j0 + jw;
-  const bool xr = i0 >= a.rlo[0] && min(i0 + TX, a.N[0]) - 1 <= a.rhi[0];
-  const bool yr = gj0 >= a.rlo[1] && min(gj0 + RW, a.N[1]) - 1 <= a.rhi[1];
-  const bool xrh = i0 - 1 >= a.rlo[0] && i0 - 1 <= a.rhi[0], yrh = j0 - 1 >= a.rlo[1] && j0 - 1 <= a.rhi[1];
+  const bool yr = gj0 >= a.rlo[1] && gj0 + RW - 1 <= a.rhi[1];
+  const bool yrh = j0 - 1 >= a.rlo[1] && j0 - 1 <= a.rhi[1];
   const bool yrt = j0 >= a.rlo[1] && min(j0 + TYT, a.N[1]) - 1 <= a.rhi[1];
-  const bool rowin = gj0 < a.N[1];  // the warp has a row to compute
+  const bool rowin = !FP64 || RW > 1 || gj0 < a.N[1];  // the warp has a row to compute
 
   __syncthreads();
   // the copies of plane q into ring slot s: the E tile, and the off-diagonal
@@ -320,16 +314,13 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
   const int plane = a.N[0] * a.N[1];  // 3·Ncell < 2³¹ (checked at launch)
   const int nc = (int)a.ncell;
 
-  // The march over the chunk.  Pinned DOFs (tangential E on the low PEC
-  // walls) are zeroed behind warp-uniform branches: pw, the warp holds some
-  // on the x or y wall; z0, the plane is the z wall.  The other warps of a
-  // tile run without a select (complex64, 128×128×96 in vacuum: 56.9 → 53.7 µs;
-  // 64×64×96 at a Bloch vector 11.4 → 10.9; 320³ with corners, which wait for
-  // the corner terms, no change).  W2R: ω² is real (complex128; complex64
-  // tests it where it is used).
-  auto march = [&](auto w2_tag) {
+  // The march over the chunk.  WALL: the CTA touches a low PEC wall (i0 or j0
+  // = 0, or planes from k0 − 1 ≤ 0) and may meet pinned DOFs; the other CTAs
+  // run without the pin selects.
+  // W2R: ω² is real (complex128; complex64 tests it where it is used).
+  auto march = [&](auto wall_tag, auto w2_tag) {
+    constexpr bool WALL = decltype(wall_tag)::value;
     constexpr bool W2R = decltype(w2_tag)::value;
-    constexpr bool FINE = FP64 && W2R;  // branch axis by axis
     bool ok = true;
     if constexpr (CPA) {
       // planes k0−1 … k0+1 have landed (the newest group may be in flight)
@@ -341,83 +332,57 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
       ok = mbar_wait_sleep(smem_u32(&bars[0]), 0, ex.wait_limit, 100000u);
       ok = ok && mbar_wait_sleep(smem_u32(&bars[1]), 0, ex.wait_limit, 100000u);
     }
-    // E component c of the cell di columns and dj rows from the thread's first
-    // one, in the slot at byte offset b
-    auto ev = [&](int b, int c, int dj, int di) -> C {
-      return *reinterpret_cast<const C *>(sm + b + ((dj * G::XW + di) * 3 + c) * (int)sizeof(C));
-    };
-    const int b_own = ((jw + 1) * G::XW + lane + G::XOFF) * 3 * (int)sizeof(C);
-    const C zero = czero<C>();
-    const bool wall_i = i0 == 0 && !bx_, pj0 = gj0 == 0 && !by_;  // pj0: row 0 of warp 0
-    const bool pw = wall_i || pj0;
-    const bool pin_i = wall_i && lane == 0;  // PEC x wall: E_y, E_z at i = 0 are pinned
-    // zero the pinned entries of own-cell values of a plane other than the z wall
-    auto pin_own = [&](C (&v)[RW][3]) {
-#pragma unroll
-      for (int r = 0; r < RW; ++r) {
-        const bool pj = pj0 && r == 0;
-        v[r][0] = zif(pj, v[r][0]);
-        v[r][1] = zif(pin_i, v[r][1]);
-        v[r][2] = zif(pin_i || pj, v[r][2]);
-      }
-    };
+    const bool pin_i = WALL && gi == 0 && !bx_;  // PEC x wall: E_y, E_z at i = 0 are pinned
     C eo[RW][3];         // E(k), pinned DOFs zeroed
-    C od[RW][3];         // off-diagonal ε terms of plane k (½ of each corner around an output), when it has any
+    C od[RW][3];         // off-diagonal ε terms of plane k (½ of each corner around an output)
     C hxp[RW], hyp[RW];  // H_x, H_y at k−1
     C ezp[RW];           // E_z(k−1), pinned zeroed
     C zcn[RW];           // z-directed corner term at plane k (valid when zvalid)
     bool zvalid = false;
-    bool act[RW];
-    int off[RW];         // the cell in its plane
+    bool pin_j[RW], act[RW];
+    int cell[RW];  // cell index at plane k
 #pragma unroll
     for (int r = 0; r < RW; ++r) {
-      act[r] = gi < a.N[0] && gj0 + r < a.N[1];
-      off[r] = gi + a.N[0] * (gj0 + r);
-      zcn[r] = zero;
+      const int gj = j0 + jw + r;
+      pin_j[r] = WALL && gj == 0 && !by_;
+      act[r] = gi < a.N[0] && gj < a.N[1];
+      cell[r] = gi + a.N[0] * gj + plane * k0;
+      zcn[r] = czero<C>();
     }
     {
-      const int bm = b_own, b0 = b_own + G::SLOT;
-      C em[RW][3], mzi[RW], mzj[RW];
+      const bool zpin0 = WALL && k0 == 0 && !bz_, zpinm = WALL && kfirst == 0 && !bz_;
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          eo[r][c] = ev(b0, c, r, 0);
-          em[r][c] = ev(bm, c, r, 0);
-        }
-        mzi[r] = ev(bm, 2, r, 1);
-        mzj[r] = ev(bm, 2, r + 1, 0);
+        const int jj = jw + r;
+        const C v0 = ev2<R, RW, NS>(sm, 1, 0, jj, lane), v1 = ev2<R, RW, NS>(sm, 1, 1, jj, lane),
+                v2 = ev2<R, RW, NS>(sm, 1, 2, jj, lane);
+        eo[r][0] = zif(pin_j[r] || zpin0, v0);
+        eo[r][1] = zif(pin_i || zpin0, v1);
+        eo[r][2] = zif(pin_i || pin_j[r], v2);
       }
-      if (pw) {
-        pin_own(eo);
-        pin_own(em);
+      const C cmzm = zt[0];
 #pragma unroll
-        for (int r = 0; r < RW; ++r) {
-          mzi[r] = zif(pj0 && r == 0, mzi[r]);
-          mzj[r] = zif(pin_i, mzj[r]);
+      for (int r = 0; r < RW; ++r) {
+        const int jj = jw + r;
+        const C cmy = yt[jj + 1];
+        const C mx = zif(pin_j[r] || zpinm, ev2<R, RW, NS>(sm, 0, 0, jj, lane));
+        const C my = zif(pin_i || zpinm, ev2<R, RW, NS>(sm, 0, 1, jj, lane));
+        const C mz = zif(pin_i || pin_j[r], ev2<R, RW, NS>(sm, 0, 2, jj, lane));
+        const C mzi = zif(pin_j[r], ev2<R, RW, NS>(sm, 0, 2, jj, lane + 1));
+        const C mzj = zif(pin_i, ev2<R, RW, NS>(sm, 0, 2, jj + 1, lane));
+        if constexpr (FP64) {
+          const C dy = csub(mzj, mz), dz = csub(eo[r][1], my), ex_ = csub(eo[r][0], mx), dx = csub(mzi, mz);
+          by_axis<W2R>(xr, yr, kfirst >= a.rlo[2] && kfirst <= a.rhi[2], [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            hxp[r] = pdiff_by<YR, ZR>(cmy, dy, cmzm, dz);
+            hyp[r] = pdiff_by<ZR, XR>(cmzm, ex_, cmx, dx);
+          });
+        } else {
+          hxp[r] = csub(cmul(cmy, csub(mzj, mz)), cmul(cmzm, csub(eo[r][1], my)));
+          hyp[r] = csub(cmul(cmzm, csub(eo[r][0], mx)), cmul(cmx, csub(mzi, mz)));
         }
+        ezp[r] = mz;
       }
-      if (k0 <= 1 && !bz_) {
-#pragma unroll
-        for (int r = 0; r < RW; ++r)
-#pragma unroll
-          for (int c = 0; c < 2; ++c) {
-            if (k0 == 0) eo[r][c] = zero;
-            else em[r][c] = zero;
-          }
-      }
-      const K cmzm = zk[0];
-      by_axis<FINE>(xr, yr, kfirst >= a.rlo[2] && kfirst <= a.rhi[2], [&](auto tx, auto ty, auto tz) {
-        constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-          const K cmy = yk[jw + r + 1];
-          hxp[r] = csum<YR, ZR>(cmy, psub(mzj[r], em[r][2]), cmzm, psub(em[r][1], eo[r][1]));
-          hyp[r] = csum<ZR, XR>(cmzm, psub(eo[r][0], em[r][0]), cmx, psub(em[r][2], mzi[r]));
-        }
-      });
-#pragma unroll
-      for (int r = 0; r < RW; ++r) ezp[r] = em[r][2];
     }
     if (!CPA) run = !__syncthreads_or(!ok);
 
@@ -425,12 +390,10 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
     // each slot, advanced without divisions
     int sm1 = 0, s0 = 1, s1 = 2 % NS;
     unsigned phase = 0x3u;  // slots 0 and 1 have completed phase 0
-    const R *ek = a.eps + (long long)plane * k0;  // the plane's ε and outputs (uniform addresses)
-    C *yp = y + 3ll * plane * k0;
     for (int k = k0; run && k < k1; ++k) {
       const int p0 = k - kfirst;
       X &xc_ = xch[k & 1];
-      const bool z0 = k == 0 && !bz_;
+      const bool z0 = WALL && k == 0 && !bz_;
       // diagonal ε (when it does not come through the ring) and the epilogue
       // operand at plane k: their latency overlaps this plane's curls
       R epk[RW][3];
@@ -439,16 +402,17 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
       for (int r = 0; r < RW; ++r) {
         epk[r][0] = epk[r][1] = epk[r][2] = R(0);
         if (!edr && act[r]) {
-          epk[r][0] = ek[off[r]];
-          epk[r][1] = (ek + nc)[off[r]];
-          epk[r][2] = (ek + 2ll * nc)[off[r]];
+          epk[r][0] = a.eps[cell[r]];
+          epk[r][1] = a.eps[nc + cell[r]];
+          epk[r][2] = a.eps[2 * nc + cell[r]];
         }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) od[r][c] = czero<C>();
         if (EPI == EPI_RESID || EPI == EPI_DOT_AUX) {
           if (act[r]) {
-            const C *ax = aux0 + 3ll * plane * k + 3 * off[r];
-            aux[r][0] = ax[0];
-            aux[r][1] = ax[1];
-            aux[r][2] = ax[2];
+            aux[r][0] = aux0[3 * cell[r]];
+            aux[r][1] = aux0[3 * cell[r] + 1];
+            aux[r][2] = aux0[3 * cell[r] + 2];
           }
         }
       }
@@ -456,110 +420,125 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         ok = mbar_wait_sleep(smem_u32(&bars[s1]), (phase >> s1) & 1u, ex.wait_limit, 100000u);
         phase ^= 1u << s1;
       }
-      const int b0 = b_own + s0 * G::SLOT, b1 = b_own + s1 * G::SLOT;
-      const K cmz = zk[p0], cez = zk[KC2 + p0];
+      const C cmz = zt[p0], cez = zt[KC2 + p0];
       const bool zr = k >= a.rlo[2] && k <= a.rhi[2];
-      const bool offd = zf[p0 * NW + w] != 0;
-      // E(k+1) at the thread's cells and E(k) at their i+1 and j+1 neighbours
-      C en[RW][3], eyi[RW], ezi[RW], exj, ezj;
+      const bool rc = rx && ry && zr;
+      // E(k+1) at the thread's cells (true values; the curls take the pinned
+      // entries as 0)
+      C en[RW][3];
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) en[r][c] = ev(b1, c, r, 0);
-        eyi[r] = ev(b0, 1, r, 1);
-        ezi[r] = ev(b0, 2, r, 1);
-      }
-      exj = ev(b0, 0, RW, 0);
-      ezj = ev(b0, 2, RW, 0);
-      if (pw) {
-        pin_own(en);
-        ezi[0] = zif(pj0, ezi[0]);
-        ezj = zif(pin_i, ezj);
-      }
-      if (z0) {
-#pragma unroll
-        for (int r = 0; r < RW; ++r) eyi[r] = zero;
-        exj = zero;
+        for (int c = 0; c < 3; ++c) en[r][c] = ev2<R, RW, NS>(sm, s1, c, jw + r, lane);
       }
       // ---- H(k) at the thread's cells
       C hx[RW], hy[RW], hz[RW];
-      if (!FP64 || rowin)
-        by_axis<FINE>(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
-          constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
 #pragma unroll
-          for (int r = 0; r < RW; ++r) {
-            const K cmy = yk[jw + r + 1];
-            const C xj = r + 1 < RW ? eo[r + 1 < RW ? r + 1 : r][0] : exj, zj = r + 1 < RW ? eo[r + 1 < RW ? r + 1 : r][2] : ezj;
-            hx[r] = csum<YR, ZR>(cmy, psub(zj, eo[r][2]), cmz, psub(eo[r][1], en[r][1]));
-            hy[r] = csum<ZR, XR>(cmz, psub(en[r][0], eo[r][0]), cmx, psub(eo[r][2], ezi[r]));
-            hz[r] = csum<XR, YR>(cmx, psub(eyi[r], eo[r][1]), cmy, psub(eo[r][0], xj));
-          }
-        });
+      for (int r = 0; r < RW; ++r) {
+        const int jj = jw + r;
+        const C cmy = yt[jj + 1];
+        const C eyi = zif(z0, ev2<R, RW, NS>(sm, s0, 1, jj, lane + 1));
+        const C ezi = zif(pin_j[r], ev2<R, RW, NS>(sm, s0, 2, jj, lane + 1));
+        C exj, ezj;
+        if (r + 1 < RW) {
+          exj = eo[r + 1][0];
+          ezj = eo[r + 1][2];
+        } else {
+          exj = zif(z0, ev2<R, RW, NS>(sm, s0, 0, jj + 1, lane));
+          ezj = zif(pin_i, ev2<R, RW, NS>(sm, s0, 2, jj + 1, lane));
+        }
+        const C eny = zif(pin_i, en[r][1]), enx = zif(pin_j[r], en[r][0]);
+        if constexpr (FP64) {
+          if (rowin)
+            by_axis<W2R>(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
+              constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+              hx[r] = pdiff_by<YR, ZR>(cmy, csub(ezj, eo[r][2]), cmz, csub(eny, eo[r][1]));
+              hy[r] = pdiff_by<ZR, XR>(cmz, csub(enx, eo[r][0]), cmx, csub(ezi, eo[r][2]));
+              hz[r] = pdiff_by<XR, YR>(cmx, csub(eyi, eo[r][1]), cmy, csub(exj, eo[r][0]));
+            });
+        } else if (rc) {
+          hx[r] = pdiff<true>(cmy, psub(ezj, eo[r][2]), cmz, psub(eny, eo[r][1]));
+          hy[r] = pdiff<true>(cmz, psub(enx, eo[r][0]), cmx, psub(ezi, eo[r][2]));
+          hz[r] = pdiff<true>(cmx, psub(eyi, eo[r][1]), cmy, psub(exj, eo[r][0]));
+        } else {
+          hx[r] = pdiff<false>(cmy, psub(ezj, eo[r][2]), cmz, psub(eny, eo[r][1]));
+          hy[r] = pdiff<false>(cmz, psub(enx, eo[r][0]), cmx, psub(ezi, eo[r][2]));
+          hz[r] = pdiff<false>(cmx, psub(eyi, eo[r][1]), cmy, psub(exj, eo[r][0]));
+        }
+      }
       // last row's H_x, H_z for the warp above
       xc_.hx[w + 1][lane] = hx[RW - 1];
       xc_.hz[w + 1][lane] = hz[RW - 1];
       if (w == 0) {
         // tile row j0−1 (its values reach only outputs of pinned DOFs when j0 = 0)
-        const K cmy = yk[0];
-        C mx = ev(b0, 0, -1, 0), my = ev(b0, 1, -1, 0), mz = ev(b0, 2, -1, 0);
-        C myk = ev(b1, 1, -1, 0), myi = ev(b0, 1, -1, 1);
-        if (wall_i) {
-          my = zif(pin_i, my);
-          mz = zif(pin_i, mz);
-          myk = zif(pin_i, myk);
+        const C cmy = yt[0];
+        const C mx = zif(z0, ev2<R, RW, NS>(sm, s0, 0, -1, lane));
+        const C my = zif(pin_i || z0, ev2<R, RW, NS>(sm, s0, 1, -1, lane));
+        const C mz = zif(pin_i, ev2<R, RW, NS>(sm, s0, 2, -1, lane));
+        const C myk = zif(pin_i, ev2<R, RW, NS>(sm, s1, 1, -1, lane));
+        const C myi = zif(z0, ev2<R, RW, NS>(sm, s0, 1, -1, lane + 1));
+        if constexpr (FP64) {
+          by_axis<W2R>(xr, yrh, zr, [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            xc_.hx[0][lane] = pdiff_by<YR, ZR>(cmy, csub(eo[0][2], mz), cmz, csub(myk, my));
+            xc_.hz[0][lane] = pdiff_by<XR, YR>(cmx, csub(myi, my), cmy, csub(eo[0][0], mx));
+          });
+        } else {
+          xc_.hx[0][lane] = csub(cmul(cmy, csub(eo[0][2], mz)), cmul(cmz, csub(myk, my)));
+          xc_.hz[0][lane] = csub(cmul(cmx, csub(myi, my)), cmul(cmy, csub(eo[0][0], mx)));
         }
-        if (z0) mx = my = myi = zero;
-        by_axis<FINE>(xr, yrh, zr, [&](auto tx, auto ty, auto tz) {
-          constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
-          xc_.hx[0][lane] = csum<YR, ZR>(cmy, psub(eo[0][2], mz), cmz, psub(my, myk));
-          xc_.hz[0][lane] = csum<XR, YR>(cmx, psub(myi, my), cmy, psub(mx, eo[0][0]));
-        });
       } else if (w == 1 && lane < TYT) {
         // column i0−1, tile row `lane` (reaches only pinned outputs when i0 = 0)
         const int jj = lane;
-        const bool pj = j0 + jj == 0 && !by_;
-        const K cmy = yk[jj + 1], cmh = coef_of(xt[0]);
-        C ex_k = ev2<R, RW, NS>(sm, s0, 0, jj, -1), ex_k1 = ev2<R, RW, NS>(sm, s1, 0, jj, -1);
-        C ey_ = ev2<R, RW, NS>(sm, s0, 1, jj, -1), ez_ = ev2<R, RW, NS>(sm, s0, 2, jj, -1);
-        C exj_ = ev2<R, RW, NS>(sm, s0, 0, jj + 1, -1);
-        C ey0 = ev2<R, RW, NS>(sm, s0, 1, jj, 0), ez0 = ev2<R, RW, NS>(sm, s0, 2, jj, 0);
-        if (wall_i) ey0 = ez0 = zero;
-        if (pj) ex_k = ex_k1 = ez_ = ez0 = zero;
-        if (z0) ex_k = ey_ = exj_ = ey0 = zero;
-        by_axis<FINE>(xrh, yrt, zr, [&](auto tx, auto ty, auto tz) {
-          constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
-          xc_.hyh[jj] = csum<ZR, XR>(cmz, psub(ex_k1, ex_k), cmh, psub(ez_, ez0));
-          xc_.hzh[jj] = csum<XR, YR>(cmh, psub(ey0, ey_), cmy, psub(ex_k, exj_));
-        });
+        const bool pj = WALL && j0 + jj == 0 && !by_, pi0 = WALL && i0 == 0 && !bx_;
+        const C cmy = yt[jj + 1], cmh = xt[0];
+        const C ex_k = zif(pj || z0, ev2<R, RW, NS>(sm, s0, 0, jj, -1));
+        const C ex_k1 = zif(pj, ev2<R, RW, NS>(sm, s1, 0, jj, -1));
+        const C ey_ = zif(z0, ev2<R, RW, NS>(sm, s0, 1, jj, -1));
+        const C ez_ = zif(pj, ev2<R, RW, NS>(sm, s0, 2, jj, -1));
+        const C exj = zif(z0, ev2<R, RW, NS>(sm, s0, 0, jj + 1, -1));
+        const C ey0 = zif(pi0 || z0, ev2<R, RW, NS>(sm, s0, 1, jj, 0));
+        const C ez0 = zif(pi0 || pj, ev2<R, RW, NS>(sm, s0, 2, jj, 0));
+        if constexpr (FP64) {
+          by_axis<W2R>(xrh, yrt, zr, [&](auto tx, auto ty, auto tz) {
+            constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
+            xc_.hyh[jj] = pdiff_by<ZR, XR>(cmz, csub(ex_k1, ex_k), cmh, csub(ez0, ez_));
+            xc_.hzh[jj] = pdiff_by<XR, YR>(cmh, csub(ey0, ey_), cmy, csub(exj, ex_k));
+          });
+        } else {
+          xc_.hyh[jj] = csub(cmul(cmz, csub(ex_k1, ex_k)), cmul(cmh, csub(ez0, ez_)));
+          xc_.hzh[jj] = csub(cmul(cmh, csub(ey0, ey_)), cmul(cmy, csub(exj, ex_k)));
+        }
       }
       // ---- off-diagonal ε: corner terms of this warp's cells, folded into the
       // diagonal term (½ of each of the two corners around an output; pinned
       // outputs take none); lane 31's column i0+32 and the last row's row
       // above arrive through the exchange after the barrier
+      const bool offd = zf[p0 * NW + w] != 0;
       // corner terms with real averaging weights outside the PML
       auto corners = [&](auto rc_tag) {
         constexpr bool RCW = decltype(rc_tag)::value;
         const C wmx = xt[2 * (TX + 2) + lane + 1], wpx = xt[3 * (TX + 2) + lane + 1];
-        const C wmz = zt[p0], wpz = zt[KC2 + p0];
+        const C wmz = zt[2 * KC2 + p0], wpz = zt[3 * KC2 + p0];
 #pragma unroll
         for (int r = 0; r < RW; ++r) {
           const int jj = jw + r;
-          const bool pj = pj0 && r == 0;
-          const C wmy = yt[jj + 1], wpy = yt[(TYT + 2) + jj + 1];
+          const C wmy = yt[2 * (TYT + 2) + jj + 1], wpy = yt[3 * (TYT + 2) + jj + 1];
+          const C enx = zif(pin_j[r], en[r][0]), eny = zif(pin_i, en[r][1]);
           // E_x(i−1) at k and k+1
-          C exm = shfl_up1(eo[r][0]), exm1 = shfl_up1(en[r][0]);
+          C exm = shfl_up1(eo[r][0]), exm1 = shfl_up1(enx);
           if (lane == 0) {
-            exm = zif(pj || z0, ev(b0, 0, r, -1));
-            exm1 = zif(pj, ev(b1, 0, r, -1));
+            exm = zif(pin_j[r] || z0, ev2<R, RW, NS>(sm, s0, 0, jj, -1));
+            exm1 = zif(pin_j[r], ev2<R, RW, NS>(sm, s1, 0, jj, -1));
           }
           // E_y(j−1) at k and k+1
           C eym, eym1;
           if (r > 0) {
-            eym = eo[r > 0 ? r - 1 : 0][1];
-            eym1 = en[r > 0 ? r - 1 : 0][1];
+            eym = eo[r - 1][1];
+            eym1 = zif(pin_i, en[r - 1][1]);
           } else {
-            eym = zif(pin_i || z0, ev(b0, 1, -1, 0));
-            eym1 = zif(pin_i, ev(b1, 1, -1, 0));
+            eym = zif(pin_i || z0, ev2<R, RW, NS>(sm, s0, 1, jj - 1, lane));
+            eym1 = zif(pin_i, ev2<R, RW, NS>(sm, s1, 1, jj - 1, lane));
           }
           const R exy = eps_off(s0, 0, jj, lane, k), eyz = eps_off(s0, 1, jj, lane, k),
                   ezx = eps_off(s0, 2, jj, lane, k);
@@ -570,38 +549,42 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
           const C xcv = cadd(cscale(ay, exy), cscale(az, ezx));
           const C ycv = cadd(cscale(ax, exy), cscale(az, eyz));
           const C zc0 = zvalid ? zcn[r] : cadd(cscale(ax, ezx), cscale(ay, eyz));
-          const C ax1 = wsum<RCW>(wmx, exm1, wpx, en[r][0]);
-          const C ay1 = wsum<RCW>(wmy, eym1, wpy, en[r][1]);
+          const C ax1 = wsum<RCW>(wmx, exm1, wpx, enx);
+          const C ay1 = wsum<RCW>(wmy, eym1, wpy, eny);
           const C zc1 = cadd(cscale(ax1, ezx1), cscale(ay1, eyz1));
           zcn[r] = zc1;
           C xn = shfl_down1(xcv);
-          if (lane == TX - 1) xn = zero;
-          od[r][0] = cscale(cadd(xcv, xn), R(0.5));
-          od[r][2] = cscale(cadd(zc0, zc1), R(0.5));
-          od[r][1] = cscale(ycv, R(0.5));
-          if (r > 0) od[r > 0 ? r - 1 : 0][1] = cadd(od[r > 0 ? r - 1 : 0][1], cscale(ycv, R(0.5)));
-          else xc_.yc[w][lane] = ycv;
+          if (lane == TX - 1) xn = czero<C>();
+          const bool px = pin_j[r] || z0, py = pin_i || z0, pz = pin_i || pin_j[r];
+          if (!px) od[r][0] = cscale(cadd(xcv, xn), R(0.5));
+          if (!pz) od[r][2] = cscale(cadd(zc0, zc1), R(0.5));
+          if (!py) od[r][1] = cscale(ycv, R(0.5));
+          if (r > 0) {
+            if (!py) od[r - 1][1] = cadd(od[r - 1][1], cscale(ycv, R(0.5)));
+          } else {
+            xc_.yc[w][lane] = ycv;
+          }
         }
       };
       if (offd) {
-        if (xr && yr && zr) corners(std::true_type{});
+        if (rc) corners(std::true_type{});
         else corners(std::false_type{});
       } else {
         // a warp without off-diagonal terms leaves zeros for its neighbours
-        xc_.yc[w][lane] = zero;
+        xc_.yc[w][lane] = czero<C>();
       }
       zvalid = offd;
       if (w == 2 && lane < TYT && zf[p0 * NW + lane / RW]) {
         // x-directed corner terms at column i0+32, tile row `lane`
         const int jj = lane;
-        const bool pj = j0 + jj == 0 && !by_;
-        const C wmy = yt[jj + 1], wpy = yt[(TYT + 2) + jj + 1];
+        const bool pj = WALL && j0 + jj == 0 && !by_;
+        const C wmy = yt[2 * (TYT + 2) + jj + 1], wpy = yt[3 * (TYT + 2) + jj + 1];
         const C eym = zif(z0, ev2<R, RW, NS>(sm, s0, 1, jj - 1, TX));
         const C ey0 = zif(z0, ev2<R, RW, NS>(sm, s0, 1, jj, TX));
         const C ezm = zif(pj, ev2<R, RW, NS>(sm, sm1, 2, jj, TX));
         const C ez0 = zif(pj, ev2<R, RW, NS>(sm, s0, 2, jj, TX));
         const C ay = wsum<false>(wmy, eym, wpy, ey0);
-        const C az = wsum<false>(zt[p0], ezm, zt[KC2 + p0], ez0);
+        const C az = wsum<false>(zt[2 * KC2 + p0], ezm, zt[3 * KC2 + p0], ez0);
         xc_.xce[jj] = cadd(cscale(ay, eps_off(s0, 0, jj, TX, k)), cscale(az, eps_off(s0, 2, jj, TX, k)));
       } else if (w == 3 && zf[p0 * NW + NW - 1]) {
         // y-directed corner terms at row j0+TYT
@@ -611,7 +594,7 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         const C ezm = zif(pin_i, ev2<R, RW, NS>(sm, sm1, 2, jj, lane));
         const C ez0 = zif(pin_i, ev2<R, RW, NS>(sm, s0, 2, jj, lane));
         const C ax = wsum<false>(xt[2 * (TX + 2) + lane + 1], exm, xt[3 * (TX + 2) + lane + 1], ex0);
-        const C az = wsum<false>(zt[p0], ezm, zt[KC2 + p0], ez0);
+        const C az = wsum<false>(zt[2 * KC2 + p0], ezm, zt[3 * KC2 + p0], ez0);
         xc_.yc[NW][lane] = cadd(cscale(ax, eps_off(s0, 0, jj, lane, k)), cscale(az, eps_off(s0, 1, jj, lane, k)));
       }
       // ---- all H(k) and corner terms written; planes k and k+1 no longer
@@ -636,130 +619,123 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         }
       }
       // ---- outputs y(k)
-      if (!FP64 || rowin) {
-        C yv[RW][3];
-        {
-          const C hzj0 = xc_.hz[w][lane], hxj0 = xc_.hx[w][lane];
-          C hzim[RW], hyim[RW];
 #pragma unroll
-          for (int r = 0; r < RW; ++r) {
-            hzim[r] = shfl_up1(hz[r]);
-            hyim[r] = shfl_up1(hy[r]);
-            if (lane == 0) {
-              hzim[r] = xc_.hzh[jw + r];
-              hyim[r] = xc_.hyh[jw + r];
-            }
-          }
-          by_axis<FINE>(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
+      for (int r = 0; r < RW; ++r) {
+        const int jj = jw + r;
+        const C cey = yt[(TYT + 2) + jj + 1];
+        const C hzjm = r > 0 ? hz[r - 1] : xc_.hz[w][lane];
+        const C hxjm = r > 0 ? hx[r - 1] : xc_.hx[w][lane];
+        C hzim = shfl_up1(hz[r]), hyim = shfl_up1(hy[r]);
+        if (lane == 0) {
+          hzim = xc_.hzh[jj];
+          hyim = xc_.hyh[jj];
+        }
+        C yx, yy, yz;
+        if (!rowin) break;  // nothing below it in this plane but outputs
+        if constexpr (FP64) {
+          by_axis<W2R>(xr, yr, zr, [&](auto tx, auto ty, auto tz) {
             constexpr bool XR = decltype(tx)::value, YR = decltype(ty)::value, ZR = decltype(tz)::value;
-#pragma unroll
-            for (int r = 0; r < RW; ++r) {
-              const K cey = yk[(TYT + 2) + jw + r + 1];
-              const C hzjm = r > 0 ? hz[r > 0 ? r - 1 : 0] : hzj0, hxjm = r > 0 ? hx[r > 0 ? r - 1 : 0] : hxj0;
-              yv[r][0] = csum<YR, ZR>(cey, psub(hz[r], hzjm), cez, psub(hyp[r], hy[r]));
-              yv[r][1] = csum<ZR, XR>(cez, psub(hx[r], hxp[r]), cex, psub(hzim[r], hz[r]));
-              yv[r][2] = csum<XR, YR>(cex, psub(hy[r], hyim[r]), cey, psub(hxjm, hx[r]));
-            }
+            yx = pdiff_by<YR, ZR>(cey, csub(hz[r], hzjm), cez, csub(hy[r], hyp[r]));
+            yy = pdiff_by<ZR, XR>(cez, csub(hx[r], hxp[r]), cex, csub(hz[r], hzim));
+            yz = pdiff_by<XR, YR>(cex, csub(hy[r], hyim), cey, csub(hx[r], hxjm));
           });
+        } else if (rc) {
+          yx = pdiff<true>(cey, psub(hz[r], hzjm), cez, psub(hy[r], hyp[r]));
+          yy = pdiff<true>(cez, psub(hx[r], hxp[r]), cex, psub(hz[r], hzim));
+          yz = pdiff<true>(cex, psub(hy[r], hyim), cey, psub(hx[r], hxjm));
+        } else {
+          yx = pdiff<false>(cey, psub(hz[r], hzjm), cez, psub(hy[r], hyp[r]));
+          yy = pdiff<false>(cez, psub(hx[r], hxp[r]), cex, psub(hz[r], hzim));
+          yz = pdiff<false>(cex, psub(hy[r], hyim), cey, psub(hx[r], hxjm));
         }
-        // Pε E at the cell: the diagonal with the true E (eo holds 0 at pinned
-        // DOFs; the ring slot of plane k still has them) plus the corner terms
-        C tv[RW][3];
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-#pragma unroll
-          for (int c = 0; c < 3; ++c) tv[r][c] = eo[r][c];
-          if (edr) {
-            const R *edk = reinterpret_cast<const R *>(sm + G::ED_OFF + s0 * G::ED_SLOT);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) epk[r][c] = edk[(c * TYT + jw + r) * TX + lane];
-          }
-          if (offd) {  // the corners beyond the warp's own
-            if (lane == TX - 1) od[r][0] = pfma(xc_.xce[jw + r], R(0.5), od[r][0]);
-            if (r == RW - 1) od[r][1] = pfma(xc_.yc[w + 1][lane], R(0.5), od[r][1]);
-          }
-          if (pw || z0) {  // pinned outputs: −ω²ε E alone
-            const bool pj = pj0 && r == 0;
-            const bool pn[3] = {pj || z0, pin_i || z0, pin_i || pj};
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              if (pn[c]) {
-                tv[r][c] = ev(b0, c, r, 0);
-                yv[r][c] = zero;
-                if (offd) od[r][c] = zero;
-              }
-            }
-          }
+        const bool px = pin_j[r] || z0, py = pin_i || z0, pz = pin_i || pin_j[r];
+        // Pε E at the cell: the diagonal with the true E (the ring slot of
+        // plane k still holds it where eo has a pinned 0) plus the corner terms
+        R e0, e1, e2;
+        if (edr) {
+          const R *edk = reinterpret_cast<const R *>(sm + G::ED_OFF + s0 * G::ED_SLOT);
+          e0 = edk[jj * TX + lane];
+          e1 = edk[(TYT + jj) * TX + lane];
+          e2 = edk[(2 * TYT + jj) * TX + lane];
+        } else {
+          e0 = epk[r][0];
+          e1 = epk[r][1];
+          e2 = epk[r][2];
         }
-        if (FP64 ? W2R : a.w2.y == R(0)) {
-          if constexpr (FP64) {
-            // −ω²ε as one factor; the corner terms only where there are any
-#pragma unroll
-            for (int r = 0; r < RW; ++r)
-#pragma unroll
-              for (int c = 0; c < 3; ++c) yv[r][c] = pfma(tv[r][c], -a.w2.x * epk[r][c], yv[r][c]);
-            if (offd)
-#pragma unroll
-              for (int r = 0; r < RW; ++r)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) yv[r][c] = pfma(od[r][c], -a.w2.x, yv[r][c]);
-          } else if (offd) {
-#pragma unroll
-            for (int r = 0; r < RW; ++r)
-#pragma unroll
-              for (int c = 0; c < 3; ++c) yv[r][c] = pfma(pfma(tv[r][c], epk[r][c], od[r][c]), -a.w2.x, yv[r][c]);
-          } else {
-#pragma unroll
-            for (int r = 0; r < RW; ++r)
-#pragma unroll
-              for (int c = 0; c < 3; ++c) yv[r][c] = pfma(cscale(tv[r][c], epk[r][c]), -a.w2.x, yv[r][c]);
+        C t0 = eo[r][0], t1 = eo[r][1], t2 = eo[r][2];
+        if (WALL) {
+          if (px) t0 = ev2<R, RW, NS>(sm, s0, 0, jj, lane);
+          if (py) t1 = ev2<R, RW, NS>(sm, s0, 1, jj, lane);
+          if (pz) t2 = ev2<R, RW, NS>(sm, s0, 2, jj, lane);
+        }
+        if (WALL) {
+          if (px) yx = czero<C>();
+          if (py) yy = czero<C>();
+          if (pz) yz = czero<C>();
+        }
+        if constexpr (FP64 && W2R) {
+          // −ω²ε as one factor; the corner terms only where there are any
+          yx = pfma(t0, -a.w2.x * e0, yx);
+          yy = pfma(t1, -a.w2.x * e1, yy);
+          yz = pfma(t2, -a.w2.x * e2, yz);
+          if (offd) {
+            C d0 = od[r][0], d1 = od[r][1];
+            if (lane == TX - 1 && !px) d0 = pfma(xc_.xce[jj], R(0.5), d0);
+            if (r == RW - 1 && !py) d1 = pfma(xc_.yc[w + 1][lane], R(0.5), d1);
+            yx = pfma(d0, -a.w2.x, yx);
+            yy = pfma(d1, -a.w2.x, yy);
+            yz = pfma(od[r][2], -a.w2.x, yz);
           }
         } else {
-#pragma unroll
-          for (int r = 0; r < RW; ++r)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              C d = cscale(tv[r][c], epk[r][c]);
-              if (offd) d = pfma(tv[r][c], epk[r][c], od[r][c]);
-              yv[r][c] = csub(yv[r][c], cmul(a.w2, d));
-            }
+          C d0 = pfma(t0, e0, od[r][0]), d1 = pfma(t1, e1, od[r][1]), d2 = pfma(t2, e2, od[r][2]);
+          if (offd) {
+            if (lane == TX - 1 && !px) d0 = pfma(xc_.xce[jj], R(0.5), d0);
+            if (r == RW - 1 && !py) d1 = pfma(xc_.yc[w + 1][lane], R(0.5), d1);
+          }
+          if (!FP64 && a.w2.y == R(0)) {
+            yx = pfma(d0, -a.w2.x, yx);
+            yy = pfma(d1, -a.w2.x, yy);
+            yz = pfma(d2, -a.w2.x, yz);
+          } else {
+            yx = csub(yx, cmul(a.w2, d0));
+            yy = csub(yy, cmul(a.w2, d1));
+            yz = csub(yz, cmul(a.w2, d2));
+          }
         }
-#pragma unroll
-        for (int r = 0; r < RW; ++r) {
-          if (!act[r]) continue;
-          C *v = yv[r];
+        if (act[r]) {
+          const int ce = cell[r];
           if (EPI == EPI_RESID) {
-#pragma unroll
-            for (int c = 0; c < 3; ++c) v[c] = csub(aux[r][c], v[c]);
-            acc.r0.add(v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
-                       v[2].y * v[2].y);
-          } else if (EPI == EPI_DOT_AUX || EPI == EPI_DOT_TS) {
-            // (r̂, y), or (t, s) with the true input s
-            const C q0 = EPI == EPI_DOT_AUX ? cdotc(aux[r][0], v[0]) : cdotc(v[0], tv[r][0]);
-            const C q1 = EPI == EPI_DOT_AUX ? cdotc(aux[r][1], v[1]) : cdotc(v[1], tv[r][1]);
-            const C q2 = EPI == EPI_DOT_AUX ? cdotc(aux[r][2], v[2]) : cdotc(v[2], tv[r][2]);
+            yx = csub(aux[r][0], yx);
+            yy = csub(aux[r][1], yy);
+            yz = csub(aux[r][2], yz);
+            acc.r0.add(yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
+          } else if (EPI == EPI_DOT_AUX) {
+            const C q0 = cdotc(aux[r][0], yx), q1 = cdotc(aux[r][1], yy), q2 = cdotc(aux[r][2], yz);
             acc.r0.add(q0.x + q1.x + q2.x);
             acc.i0.add(q0.y + q1.y + q2.y);
-            if (EPI == EPI_DOT_TS)
-              acc.r1.add(v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
-                         v[2].y * v[2].y);
+          } else if (EPI == EPI_DOT_TS) {
+            // (t, s) with the true input s (its pinned entries are not in eo)
+            const C sx = t0, sy = t1, sz = t2;
+            const C q0 = cdotc(yx, sx), q1 = cdotc(yy, sy), q2 = cdotc(yz, sz);
+            acc.r0.add(q0.x + q1.x + q2.x);
+            acc.i0.add(q0.y + q1.y + q2.y);
+            acc.r1.add(yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
           } else if (EPI == EPI_DOT_SHD) {
-            const int ce = 3 * (plane * k + off[r]);
-            const C s0_ = shadow<R>(ce), s1_ = shadow<R>(ce + 1), s2_ = shadow<R>(ce + 2);
-            if constexpr (FP64) {  // straight into the sums: 12 FP64 instructions
-              dot_into(acc.r0.s, acc.i0.s, s0_, v[0]);
-              dot_into(acc.r0.s, acc.i0.s, s1_, v[1]);
-              dot_into(acc.r0.s, acc.i0.s, s2_, v[2]);
+            const C s0 = shadow<R>(3ll * ce), s1 = shadow<R>(3ll * ce + 1), s2 = shadow<R>(3ll * ce + 2);
+            if constexpr (sizeof(R) == 8) {  // straight into the sums: 12 FP64 instructions
+              dot_into(acc.r0.s, acc.i0.s, s0, yx);
+              dot_into(acc.r0.s, acc.i0.s, s1, yy);
+              dot_into(acc.r0.s, acc.i0.s, s2, yz);
             } else {
-              const C q = pdot3(s0_, v[0], s1_, v[1], s2_, v[2]);
+              const C q = pdot3(s0, yx, s1, yy, s2, yz);
               acc.r0.add(q.x);
               acc.i0.add(q.y);
             }
           }
-          C *yo = yp + 3 * off[r];
-          yo[0] = v[0];
-          yo[1] = v[1];
-          yo[2] = v[2];
+          C *yo = y + 3 * ce;
+          yo[0] = yx;
+          yo[1] = yy;
+          yo[2] = yz;
         }
       }
       // ---- advance to plane k+1
@@ -768,21 +744,24 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
         hxp[r] = hx[r];
         hyp[r] = hy[r];
         ezp[r] = eo[r][2];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) eo[r][c] = en[r][c];
+        eo[r][0] = zif(pin_j[r], en[r][0]);
+        eo[r][1] = zif(pin_i, en[r][1]);
+        eo[r][2] = zif(pin_i || pin_j[r], en[r][2]);
+        cell[r] += plane;
       }
-      ek += plane;
-      yp += 3ll * plane;
       sm1 = s0;
       s0 = s1;
       s1 = s1 + 1 == NS ? 0 : s1 + 1;
     }
   };
+  // a chunk starting at plane 1 reads the z = 0 wall plane as its plane k−1
   if constexpr (FP64) {
-    if (a.w2.y == R(0)) march(std::true_type{});
-    else march(std::false_type{});
+    // the selects of the wall form are free next to the FP64 pipe
+    if (a.w2.y == R(0)) march(std::true_type{}, std::true_type{});
+    else march(std::true_type{}, std::false_type{});
   } else {
-    march(std::false_type{});
+    if (i0 == 0 || j0 == 0 || k0 <= 1) march(std::true_type{}, std::false_type{});
+    else march(std::false_type{}, std::false_type{});
   }
 
   if (CPA) cp_async_wait<0>();
