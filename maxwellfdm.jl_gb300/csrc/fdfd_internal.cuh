@@ -225,8 +225,10 @@ int launch_apply_v3(fdfd_handle *h, const float2 *x, float2 *y, int epi, const f
                     int kc, bool tma);
 int build_corner_lists(fdfd_handle *h, const unsigned *queued);
 int queue_corner_lists(fdfd_handle *h, unsigned *next, bool *queued);
-// number of blocks launch_apply uses (reduction buffer sizing)
+// number of blocks launch_apply uses (reduction buffer sizing), and those of
+// the H formulation's kernel (hh.cu)
 int apply_blocks(const fdfd_handle *h);
+int hh_blocks(const fdfd_handle *h);
 // pick the z-chunk length per precision by timing (stencil.cu)
 int autotune_kchunk(fdfd_handle *h);
 

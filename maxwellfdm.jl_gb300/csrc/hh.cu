@@ -379,16 +379,31 @@ static int hh_chunk(const fdfd_handle *h, int tiles) {
   return best;
 }
 
+// Thread blocks of a launch, and the larger of the two precisions'.
+template <typename R>
+static constexpr int hh_rows() { return sizeof(R) == 4 ? 2 : 1; }  // rows per warp
+template <typename R>
+static dim3 hh_grid(const fdfd_handle *h, int *kchunk) {
+  constexpr int TYT = HG<R, hh_rows<R>()>::TYT;
+  dim3 grid((h->N[0] + TX - 1) / TX, (h->N[1] + TYT - 1) / TYT, 1);
+  *kchunk = hh_chunk(h, (int)(grid.x * grid.y));
+  grid.z = (h->N[2] + *kchunk - 1) / *kchunk;
+  return grid;
+}
+int hh_blocks(const fdfd_handle *h) {
+  int kc;
+  const dim3 a = hh_grid<float>(h, &kc), b = hh_grid<double>(h, &kc);
+  return (int)std::max(a.x * a.y * a.z, b.x * b.y * b.z);
+}
+
 template <typename R, int EPI, bool W2R>
 static int launch_hh_t(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R>::C *y,
                        const typename CT<R>::C *aux0, int fin, KScalars *sc) {
-  constexpr int RW = sizeof(R) == 4 ? 2 : 1;
+  constexpr int RW = hh_rows<R>();
   using G = HG<R, RW>;
   const auto kern = k_apply_hh<R, EPI, RW, W2R>;
   Extra<R> ex = make_extra<R>(h);
-  dim3 grid((h->N[0] + TX - 1) / TX, (h->N[1] + G::TYT - 1) / G::TYT, 1);
-  ex.kchunk = hh_chunk(h, (int)(grid.x * grid.y));
-  grid.z = (h->N[2] + ex.kchunk - 1) / ex.kchunk;
+  const dim3 grid = hh_grid<R>(h, &ex.kchunk);
   if (EPI != EPI_STORE) {
     int rc = ensure_red(h, (int)(grid.x * grid.y * grid.z));
     if (rc) return rc;

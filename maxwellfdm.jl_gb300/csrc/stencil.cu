@@ -801,9 +801,12 @@ static int blocks_for(const fdfd_handle *h, int kc) {
   return ((h->N[0] + TX - 1) / TX) * ((h->N[1] + TY - 1) / TY) * ((h->N[2] + kc - 1) / kc);
 }
 
+// The most thread blocks an operator launch takes, in either precision and
+// either formulation (the H kernel has a z-chunk rule of its own): the
+// reduction buffer holds that many before a solver batch is captured.
 int apply_blocks(const fdfd_handle *h) {
   const int a = blocks_for(h, kchunk_for(h, true)), b = blocks_for(h, kchunk_for(h, false));
-  return std::max(std::max(a, b), std::max(h->nwork[0], h->nwork[1]));
+  return std::max({a, b, h->nwork[0], h->nwork[1], hh_blocks(h)});
 }
 
 template <typename R>

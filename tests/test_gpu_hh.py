@@ -114,3 +114,23 @@ def test_hh_matvec_tile_edges(pkg, oracle, monkeypatch, N, bloch, kc):
         assert np.linalg.norm(A.matvec(x, "c128") - ref) <= 1e-12 * np.linalg.norm(ref)
         assert np.linalg.norm(A.matvec(x, "c64") - ref) <= 1e-5 * np.linalg.norm(ref)
         A.close()
+
+
+def test_hh_mixed_bicgstab_graph(pkg, oracle, monkeypatch):
+    """A mixed-precision BiCGSTAB solve of the H formulation, replayed as a
+    graph, where the complex64 H kernel has more thread blocks (858) than the
+    complex128 one (780) and than any launch of the E kernels on one-wave
+    schedules: the reduction buffer has to hold its partial sums before the
+    capture begins."""
+    monkeypatch.setenv("FDFD_SCHEDULE", "1")
+    N = (192, 208, 64)
+    om = 2 * np.pi / 1.5  # ω² dominates: a solve takes few iterations
+    sdl_e, sdl_m = oracle.stretched_dl(oracle.uniform_grid(N), om, ((0, 0, 0), (0, 0, 0)))
+    A = pkg.FDFDOperator(N, om, sdl_e, sdl_m)
+    A.set_eps(np.full(N + (3,), 9.0))
+    A.set_field_type("H")
+    rng = np.random.default_rng(2)
+    b = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    x, st = A.solve(b, tol=1e-4, precision="mixed", method="bicgstab", maxit=200)
+    assert np.linalg.norm(b - A.matvec(x, "c128")) <= 1.01e-4 * np.linalg.norm(b), st
+    A.close()
