@@ -5,6 +5,8 @@
 // All reducing kernels use a fixed grid (RED_BLOCKS × 256 threads) and a
 // grid-stride loop, so the per-block partials and therefore the reduced
 // values are deterministic for a given problem size.
+#include <algorithm>
+
 #include "krylov_fin.cuh"
 
 namespace fdfd {
@@ -12,19 +14,39 @@ namespace fdfd {
 constexpr int VB = 256;          // threads per block
 constexpr int RED_BLOCKS = 152 * 4;
 
+// Partial sums of at least `blocks` thread blocks (32 bytes each).  Captured
+// solver graphs hold the buffer's addresses: they are dropped when it is
+// replaced, and it is never replaced during a capture.  It starts with what
+// any method's vector kernels need (the Gram matrix of BiCGStab(4): eight
+// slots a block), so that solves of different methods on one handle neither
+// grow it nor capture again.
 int ensure_red(fdfd_handle *h, int blocks) {
-  if (blocks < RED_BLOCKS) blocks = RED_BLOCKS;
-  if (h->red.part != nullptr && h->red_blocks >= blocks) return FDFD_OK;
-  if (h->red.part) cudaFree(h->red.part);
-  if (h->red.count) cudaFree(h->red.count);
+  blocks = std::max(blocks, 8 * RED_BLOCKS);
+  if (h->red.part != nullptr && h->red.count != nullptr && h->red_blocks >= blocks) return FDFD_OK;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  int rc = cuda_check(h, cudaStreamIsCapturing(h->stream, &cs), "cudaStreamIsCapturing");
+  if (rc) return rc;
+  if (cs != cudaStreamCaptureStatusNone)
+    return set_error(h, FDFD_ERR_CUDA, "the reduction buffer is too small for a launch that is being captured");
+  if ((rc = cuda_check(h, cudaStreamSynchronize(h->stream), "stream sync"))) return rc;
+  drop_graphs(h);
+  cudaFree(h->red.part);
+  cudaFree(h->red.count);
   h->red.part = nullptr;
   h->red.count = nullptr;
-  cudaError_t e = dev_malloc(&h->red.part, sizeof(double2) * 2 * (size_t)blocks);
-  if (e != cudaSuccess) return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(reduction partials) failed");
-  e = dev_malloc(&h->red.count, sizeof(unsigned int));
-  if (e != cudaSuccess) return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(reduction counter) failed");
-  e = cudaMemsetAsync(h->red.count, 0, sizeof(unsigned int), h->stream);
-  if (e != cudaSuccess) return cuda_check(h, e, "cudaMemsetAsync(counter)");
+  h->red_blocks = 0;
+  if (dev_malloc(&h->red.part, sizeof(double2) * 2 * (size_t)blocks) != cudaSuccess) {
+    cudaGetLastError();
+    h->red.part = nullptr;
+    return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(reduction partials) failed");
+  }
+  if (dev_malloc(&h->red.count, sizeof(unsigned int)) != cudaSuccess) {
+    cudaGetLastError();
+    h->red.count = nullptr;
+    return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(reduction counter) failed");
+  }
+  if ((rc = cuda_check(h, cudaMemsetAsync(h->red.count, 0, sizeof(unsigned int), h->stream), "cudaMemsetAsync(counter)")))
+    return rc;
   h->red_blocks = blocks;
   return FDFD_OK;
 }

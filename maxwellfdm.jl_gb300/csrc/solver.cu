@@ -283,9 +283,8 @@ static int batch_graph(fdfd_handle *h, Workspace *ws, int method, int ell, bool 
   const int pi = sizeof(R) == 4 ? 1 : 0;
   const int mi = method == FDFD_COCG ? 1 : method == FDFD_BICGSTABL ? 2 : 0;
   const int ti = tr ? 1 : 0;
-  // lazily-sized buffers must exist before any capture (the Gram kernel of
-  // BiCGStab(ℓ) keeps up to 16 partials per block)
-  TRY(ensure_red(h, std::max(apply_blocks(h), method == FDFD_BICGSTABL ? 8 * 152 * 4 : 0)));
+  // lazily-sized buffers must exist before any capture
+  TRY(ensure_red(h, apply_blocks(h)));
   cudaGraphExec_t &ge = ws->gexec[pi][mi][ti];
   cudaGraph_t &gg = ws->graph[pi][mi][ti];
   if (ge && (ws->gbatch[pi][mi][ti] != batch || ws->gell[pi][mi][ti] != ell)) {
@@ -331,7 +330,7 @@ static long long batch_kernels(Workspace *ws, int method, bool tr) {
 template <typename R>
 static int run_batch(fdfd_handle *h, Workspace *ws, int method, int ell, bool tr, int batch, bool use_graph) {
   if (!use_graph) {
-    TRY(ensure_red(h, std::max(apply_blocks(h), method == FDFD_BICGSTABL ? 8 * 152 * 4 : 0)));
+    TRY(ensure_red(h, apply_blocks(h)));
     for (int i = 0; i < batch; ++i) {
       if (method == FDFD_COCG) TRY(cocg_iter<R>(h, ws, tr));
       else if (method == FDFD_BICGSTABL) TRY(bl_iter<R>(h, ws, ell, tr));

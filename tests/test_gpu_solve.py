@@ -176,3 +176,19 @@ def test_exact_after_one_step(pkg, oracle, precision, ell):
     x, st = A.solve(b, tol=1e-10, precision=precision, ell=ell)
     assert np.linalg.norm(b - S.A @ x) <= 1e-10, st
     A.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_methods_in_turn_on_one_handle(pkg, sysx, precision):
+    """BiCGSTAB, BiCGStab(4) and BiCGSTAB again on one handle, each from its
+    captured graph: the second BiCGSTAB solve replays the first one's, whose
+    reduction buffer the solve between them must not have replaced, and takes
+    the same steps to the same result."""
+    S, b, xd = sysx
+    A = _op(pkg, S)
+    got = [A.solve(b, tol=1e-8, precision=precision, method=m) for m in ("bicgstab", "bicgstabl", "bicgstab")]
+    for x, st in got:
+        assert np.linalg.norm(b - S.A @ x) <= 1.01e-8 * np.linalg.norm(b), st
+    assert np.array_equal(got[0][0], got[2][0])
+    assert got[0][1][0]["iterations"] == got[2][1][0]["iterations"]
+    A.close()
