@@ -135,51 +135,26 @@ int build_weights(fdfd_handle *h, double2 *w64, float2 *w32, double2 *d64, float
   return cuda_check(h, cudaGetLastError(), "k_weights");
 }
 
-// Flag (xy tile, plane k) if any off-diagonal ε that the tile's outputs at
-// plane k read is non-zero: corners i ∈ [i0, i0+TX], j ∈ [j0, j0+TY],
-// planes k and k+1.
-__global__ void k_oflags(const double *eoff, long long ncell, int N0, int N1, int N2, int tiles_x, uint8_t *flag) {
-  for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < ncell;
-       cell += (long long)gridDim.x * blockDim.x) {
-    if (eoff[cell] == 0.0 && eoff[ncell + cell] == 0.0 && eoff[2 * ncell + cell] == 0.0) continue;
-    const int i = (int)(cell % N0), j = (int)((cell / N0) % N1), k = (int)(cell / ((long long)N0 * N1));
-    const int tx0 = i / TX, ty0 = j / TY;
-    for (int dx = -1; dx <= 0; ++dx) {
-      const int tx = tx0 + dx;
-      if (tx < 0 || (dx == -1 && i % TX != 0)) continue;
-      for (int dy = -1; dy <= 0; ++dy) {
-        const int ty = ty0 + dy;
-        if (ty < 0 || (dy == -1 && j % TY != 0)) continue;
-        const long long tc = tx + (long long)tiles_x * ty;
-        flag[tc * N2 + k] = 1;
-        if (k > 0) flag[tc * N2 + k - 1] = 1;
-      }
-    }
-  }
-}
-
 // Flag (x tile, group of g rows, plane k) if any off-diagonal ε that the
 // outputs of those rows at plane k read is non-zero: corners i ∈ [i0, i0+TX],
-// rows j ∈ [g·t, g·t+g], planes k and k+1 (the second TMA kernel's warps own
-// g rows each).
-__global__ void k_oflags_rows(const double *eoff, long long ncell, int N0, int N1, int N2, int tiles_x, int g,
-                              uint8_t *flag) {
+// rows j ∈ [g·t, g·t+g], planes k and k+1 — the corner one past the last cell
+// of a periodic axis being its corner 0.  (g = TY: the tiles of the first
+// kernels; 1 and 2: the warp strips of the second.)
+__global__ void k_oflags(const double *eoff, long long ncell, int N0, int N1, int N2, int b0, int b1, int b2,
+                         int tiles_x, int g, uint8_t *flag) {
   for (long long cell = blockIdx.x * (long long)blockDim.x + threadIdx.x; cell < ncell;
        cell += (long long)gridDim.x * blockDim.x) {
     if (eoff[cell] == 0.0 && eoff[ncell + cell] == 0.0 && eoff[2 * ncell + cell] == 0.0) continue;
     const int i = (int)(cell % N0), j = (int)((cell / N0) % N1), k = (int)(cell / ((long long)N0 * N1));
-    const int tx0 = i / TX, ty0 = j / g;
-    for (int dx = -1; dx <= 0; ++dx) {
-      const int tx = tx0 + dx;
-      if (tx < 0 || (dx == -1 && i % TX != 0)) continue;
-      for (int dy = -1; dy <= 0; ++dy) {
-        const int ty = ty0 + dy;
-        if (ty < 0 || (dy == -1 && j % g != 0)) continue;
-        const long long tc = tx + (long long)tiles_x * ty;
+    // the cells whose outputs read this corner: it and the one before it on each axis
+    const int is[2] = {i, cell_before(i, N0, b0)}, js[2] = {j, cell_before(j, N1, b1)};
+    const int kb = cell_before(k, N2, b2);
+    for (const int u : is)
+      for (const int v : js) {
+        const long long tc = u / TX + (long long)tiles_x * (v / g);
         flag[tc * N2 + k] = 1;
-        if (k > 0) flag[tc * N2 + k - 1] = 1;
+        flag[tc * N2 + kb] = 1;
       }
-    }
   }
 }
 
@@ -206,13 +181,12 @@ int build_oflags(fdfd_handle *h) {
   const int tiles_x = (h->N[0] + TX - 1) / TX;
   int rc = ensure_oflags(h);
   if (rc) return rc;
-  k_oflags<<<152 * 4, 256, 0, h->stream>>>(h->eoff64, h->ncell, h->N[0], h->N[1], h->N[2], tiles_x, h->oflag);
-  if ((rc = cuda_check(h, cudaGetLastError(), "k_oflags"))) return rc;
-  // per groups of 1 and 2 rows (the second kernel's warp strips)
-  for (int g = 1; g <= 2; ++g) {
-    k_oflags_rows<<<152 * 4, 256, 0, h->stream>>>(h->eoff64, h->ncell, h->N[0], h->N[1], h->N[2], tiles_x, g,
-                                                  h->oflag_rows[g - 1]);
-    if ((rc = cuda_check(h, cudaGetLastError(), "k_oflags_rows"))) return rc;
+  const int rows[3] = {TY, 1, 2};
+  uint8_t *const f[3] = {h->oflag, h->oflag_rows[0], h->oflag_rows[1]};
+  for (int q = 0; q < 3; ++q) {
+    k_oflags<<<152 * 4, 256, 0, h->stream>>>(h->eoff64, h->ncell, h->N[0], h->N[1], h->N[2], h->bloch[0], h->bloch[1],
+                                             h->bloch[2], tiles_x, rows[q], f[q]);
+    if ((rc = cuda_check(h, cudaGetLastError(), "k_oflags"))) return rc;
   }
   return FDFD_OK;
 }

@@ -112,6 +112,10 @@ struct KScalars {
   int bl_steps;                   // steps of the current cycle whose α is applied
 };
 
+// Index before t along an axis of N cells: the last one before 0 where the
+// axis is periodic, else 0 itself.
+__host__ __device__ __forceinline__ int cell_before(int t, int N, int bloch) { return t > 0 ? t - 1 : bloch ? N - 1 : 0; }
+
 struct Workspace;  // solver vectors (solver.cu)
 
 }  // namespace fdfd

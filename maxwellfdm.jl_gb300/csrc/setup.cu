@@ -292,7 +292,8 @@ __global__ void __launch_bounds__(256) k_classify(SmoothArgs A) {
 
 // One marked voxel: its smoothed ε in both precisions and, where an
 // off-diagonal is not 0, the flags of the outputs that read it (the corner's
-// own cell and the one before it on each axis, in groups of g rows).
+// own cell and the one before it on each axis — across the wrap of a periodic
+// one — in groups of g rows).
 __device__ void smooth_voxel(const SmoothArgs &A, long long entry, unsigned &cnt) {
   const int s = (int)(entry & 3);
   const long long cell = entry >> 2;
@@ -321,14 +322,16 @@ __device__ void smooth_voxel(const SmoothArgs &A, long long entry, unsigned &cnt
   }
   if (o[0] == 0.0 && o[1] == 0.0 && o[2] == 0.0) return;
   cnt++;
+  const int is[2] = {g[0], cell_before(g[0], A.N[0], A.bloch[0])};
+  const int js[2] = {g[1], cell_before(g[1], A.N[1], A.bloch[1])};
+  const int kb = cell_before(k, A.N[2], A.bloch[2]);
   for (int f = 0; f < 3; ++f) {
     const int rows = f == 0 ? TY : f;
-    for (int dx = 0; dx < 2; ++dx)
-      for (int dy = 0; dy < 2; ++dy) {
-        if (g[0] < dx || g[1] < dy) continue;
-        const long long tc = (g[0] - dx) / TX + (long long)A.tiles_x * ((g[1] - dy) / rows);
+    for (const int u : is)
+      for (const int v : js) {
+        const long long tc = u / TX + (long long)A.tiles_x * (v / rows);
         A.flag[f][tc * A.N[2] + k] = 1;
-        if (k > 0) A.flag[f][tc * A.N[2] + k - 1] = 1;
+        A.flag[f][tc * A.N[2] + kb] = 1;
       }
   }
 }

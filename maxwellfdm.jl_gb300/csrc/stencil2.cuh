@@ -917,12 +917,7 @@ static int launch_cp_t(fdfd_handle *h, const typename CT<R>::C *x, typename CT<R
     if (e != cudaSuccess) return cuda_check(h, e, "cudaFuncSetAttribute(carveout)");
     attr.set(h->dev);
   }
-  // periodic grids take the flags of the 32×8 tiles, as the plain kernel
-  // does: neither set of flags follows the wrap of an axis (a corner on plane
-  // 0 that the last cells read), and with the same ones both kernels include
-  // the same corner terms
-  const bool periodic = h->bloch[0] || h->bloch[1] || h->bloch[2];
-  ex.oflag_w = h->has_off && !periodic ? h->oflag_rows[RW - 1] : nullptr;
+  ex.oflag_w = h->has_off ? h->oflag_rows[RW - 1] : nullptr;
   const OpArgs<R> a = op_args<R>(h);
   const cudaError_t e = launch_k(h, k_apply_cp<R, EPI, RW, NS, MB>, grid, dim3(G::NT, 1, 1), (size_t)G::SMEM, a, ex, x,
                                  y, aux0, h->red, fin, sc);

@@ -314,3 +314,29 @@ def test_corner_lists(pkg, oracle, monkeypatch, N, kc):
         e, _ = A.solve(ref, tol=1e-6, maxit=400)
         assert np.linalg.norm(Aref @ e - ref) <= 1.01e-6 * np.linalg.norm(ref)
     A.close()
+
+
+@pytest.mark.parametrize("tma", ["0", "1"])
+@pytest.mark.parametrize("corner", [(0, 5, 3), (9, 0, 4), (11, 7, 0), (0, 0, 0)])
+def test_off_diagonal_on_a_periodic_face(pkg, oracle, monkeypatch, corner, tma):
+    """Off-diagonal ε at a corner on the first plane of a periodic axis
+    reaches the outputs of the last cells along it, which lie in another tile
+    and plane (whose off-diagonal flags must be set too)."""
+    monkeypatch.setenv("FDFD_DISABLE_TMA", tma)
+    O = oracle
+    N = (70, 40, 9)
+    g = O.uniform_grid(N, isbloch=(True, True, True))
+    kb = (0.03, 0.05, 0.1)
+    om = 2 * np.pi / 8
+    sdl_e, sdl_m = O.stretched_dl(g, om, ((0, 0, 0), (0, 0, 0)))
+    ed, eo = np.full(N + (3,), 2.0), np.zeros(N + (3,))
+    eo[corner] = (0.7, -0.4, 0.9)
+    Ce, Cm = O.create_curls(g, sdl_e, sdl_m, kb)
+    Aref = O.create_A(om, O.create_paramop(g, ed, eo, sdl_e, sdl_m, kb), Ce, Cm)
+    A = pkg.FDFDOperator(N, om, sdl_e, sdl_m, (True,) * 3, [np.exp(-1j * kb[w] * g.L[w]) for w in range(3)])
+    A.set_eps(ed, eo)
+    x = _rand(A.n, 4)
+    ref = Aref @ x
+    assert np.linalg.norm(A.matvec(x, "c128") - ref) <= TOL64 * np.linalg.norm(ref)
+    assert np.linalg.norm(A.matvec(x, "c64") - ref) <= TOL32 * np.linalg.norm(ref)
+    A.close()

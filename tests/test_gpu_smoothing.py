@@ -148,3 +148,27 @@ def test_resmoothing_one_handle(pkg, oracle, N, bloch):
             for prec, tol in (("c128", 1e-12), ("c64", 1e-5)):
                 assert np.linalg.norm(A.matvec(x, prec) - ref) <= tol * np.linalg.norm(ref)
     A.close()
+
+
+@pytest.mark.parametrize("bloch", [(True, False, False), (False, True, False), (False, False, True), (True, True, True)])
+@pytest.mark.parametrize("N", [(40, 33, 21), (33, 4, 40)])
+def test_smoothed_operator_on_periodic_axes(pkg, oracle, N, bloch):
+    """A x after on-device smoothing of a sphere that every low face of the
+    grid cuts: its off-diagonal ε on the first planes of the periodic axes
+    belongs to the last cells' outputs too."""
+    O = oracle
+    g = O.uniform_grid(N, isbloch=bloch)
+    om = 2 * np.pi / 8
+    sdl_e, sdl_m = O.stretched_dl(g, om, ((0, 0, 0), (0, 0, 0)))
+    po, oo = _objs(pkg, O, [("s", np.array([1.2, 1.4, 1.7]), 2.9, 12.25)])
+    A = pkg.FDFDOperator(N, om, sdl_e, sdl_m, bloch)
+    A.smooth_objects(g.lprim_full, po, 1.0)
+    red, reo = O.assign_smooth(g, oo, 1.0, None)
+    assert any(np.any(np.take(reo, 0, axis=w) != 0.0) for w in range(3) if bloch[w])
+    Ce, Cm = O.create_curls(g, sdl_e, sdl_m)
+    rng = np.random.default_rng(6)
+    x = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    ref = O.create_A(om, O.create_paramop(g, red, reo, sdl_e, sdl_m), Ce, Cm) @ x
+    for prec, tol in (("c128", 1e-12), ("c64", 1e-5)):
+        assert np.linalg.norm(A.matvec(x, prec) - ref) <= tol * np.linalg.norm(ref), prec
+    A.close()
