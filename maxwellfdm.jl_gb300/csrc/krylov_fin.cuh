@@ -107,7 +107,10 @@ __device__ inline void finalise(int mode, KScalars *sc, double2 d0, double2 d1) 
       double2 rho0 = mode == FIN_BL_RHO ? rho : rho_pre;
       if (mode == FIN_BL_CYCLE) {
         rho0 = make_double2(-(omega.x * rho.x - omega.y * rho.y), -(omega.x * rho.y + omega.y * rho.x));
-        if (w) sc->rho_pre = rho0;
+        if (w) {
+          sc->rho_pre = rho0;
+          sc->bl_steps = 0;  // x holds this cycle's steps: a breakdown found from here on has none to add
+        }
       }
       if (!dfinite(d0)) { stop(4); break; }
       if (zero(rho0)) { broken(mode == FIN_BL_CYCLE); break; }

@@ -192,3 +192,58 @@ def test_methods_in_turn_on_one_handle(pkg, sysx, precision):
     assert np.array_equal(got[0][0], got[2][0])
     assert got[0][1][0]["iterations"] == got[2][1][0]["iterations"]
     A.close()
+
+
+def _shadow(dof):
+    """The library's BiCGStab(l) shadow vector, in units of 1/32768: both halves of the 32-bit hash, as signed integers."""
+    x = dof.astype(np.uint64)
+    for mul, shift in ((0x7feb352d, 16), (0x846ca68b, 15)):
+        x = ((x ^ (x >> np.uint64(shift))) * np.uint64(mul)) & np.uint64(0xffffffff)
+    x ^= x >> np.uint64(16)
+    return (x & np.uint64(0xffff)).astype(np.uint16).view(np.int16).astype(np.int64), \
+        (x >> np.uint64(16)).astype(np.uint16).view(np.int16).astype(np.int64)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_breakdown_at_the_end_of_a_cycle(pkg, precision):
+    """A cycle of BiCGStab(1) whose minimal-residual coefficient is exactly 0
+    ends in a breakdown with its step already in x, once.  On pinned wall
+    DOFs A is diagonal; with d = 2 on the set P, d = −1 on Q and b the shadow
+    vector r̂ there, α = (r̂, b)/(r̂, D b) = 1 and (D r, r) = 0 when
+    Σ_P |r̂|² = 2 Σ_Q |r̂|² — on entries of r̂ with so few bits that every
+    product and sum is exact.  One step: x = b, ‖b − A x‖ = √2 ‖b‖."""
+    N = (128, 128, 4)
+    cell = np.arange(N[0] * N[1])
+    dof = np.sort(np.concatenate([3 * cell, 3 * cell + 1]))  # E_x, E_y on the plane k = 0
+    re, im = _shadow(dof)
+    few = (re % 16 == 0) & (im % 16 == 0) & (re != 0)
+    dof, re, im = dof[few][:60], re[few][:60] // 16, im[few][:60] // 16
+    K = re * re + im * im
+    i, j = np.triu_indices(len(dof), 1)
+    pair = {int(s): q for q, s in enumerate(K[i] + K[j])}
+    found = None
+    for q in range(len(i)):  # Σ over two pairs = 2 Σ over a third one
+        for p in range(len(i)):
+            r = pair.get(int(2 * (K[i[q]] + K[j[q]]) - K[i[p]] - K[j[p]]))
+            if r is not None and len({i[q], j[q], i[p], j[p], i[r], j[r]}) == 6:
+                found = ([i[p], j[p], i[r], j[r]], [i[q], j[q]])
+                break
+        if found:
+            break
+    P, Q = (dof[f] for f in found)
+    sdl = [np.ones(n, complex) for n in N]
+    A = pkg.FDFDOperator(N, 1.0, sdl, sdl)  # pinned rows: −ω² ε = −ε
+    eps = np.ones(N + (3,))
+    for d in P:
+        eps[(d // 3) % N[0], (d // 3) // N[0], 0, d % 3] = -2.0
+    A.set_eps(eps)
+    b = np.zeros(A.n, complex)
+    for f in found:
+        b[dof[f]] = (re[f] + 1j * im[f]) / 2048.0
+    with pytest.raises(pkg.FDFDError) as ei:
+        A.solve(b, tol=1e-6, precision=precision, ell=1, maxit=1, check_every=1)
+    st = ei.value.stats[0]
+    assert st["iterations"] == 1
+    assert abs(st["relres"] - np.sqrt(2.0)) <= 1e-12
+    assert np.array_equal(ei.value.x, b)
+    A.close()
