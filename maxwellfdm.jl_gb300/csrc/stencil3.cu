@@ -499,7 +499,10 @@ __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<f
       if (OFF) {
         const int nr = max(rounds(t), rounds(t + 1));
         if (nr > G::NH + w) {
-          if (!CPA) ok = mbar_wait_sleep(smem_u32(&bars[s1]), (phase >> s1) & 1u, ex.wait_limit, 100000u);
+          // (a wait that gave up is reported here: carried to the barrier below,
+          // it cost a live register, 384 → 390 µs at 320³)
+          if (!CPA && !mbar_wait_sleep(smem_u32(&bars[s1]), (phase >> s1) & 1u, ex.wait_limit, 100000u))
+            atomicExch(errflag, 1);
 #pragma unroll 1
           for (int n = G::NH + w; n < nr; n += NW) {
             const int4 e = entry(k, n), e1 = entry(k + 1, n);

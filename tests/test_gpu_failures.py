@@ -118,3 +118,30 @@ def test_multi_solve_reports_a_nonfinite_entry(pkg, oracle):
         bq = b if q == 0 else 2.0 * b
         assert np.linalg.norm(bq - S.A @ x) / np.linalg.norm(bq) < 1.02e-8
     A.close()
+
+
+@pytest.mark.parametrize("spheres", [True, False])
+def test_bounded_wait_of_the_third_kernel(pkg, oracle, monkeypatch, spheres):
+    """The third operator kernel (with corner lists, and in vacuum) when its
+    pipeline waits run out: FDFD_ERR_TIMEOUT, and a fresh handle on the same
+    kernel applies the operator."""
+    N = (64, 64, 64)
+    S = _system(oracle, N)
+    if not spheres:
+        S = oracle.System(S.grid, S.omega, ((3, 3, 3), (3, 3, 3)), [])
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal(3 * S.grid.ncell) + 1j * rng.standard_normal(3 * S.grid.ncell)
+    monkeypatch.setenv("FDFD_OPERATOR_V2", "5")
+    monkeypatch.setenv("FDFD_KCHUNK", "4")
+    monkeypatch.setenv("FDFD_WAIT_LIMIT_CLOCKS", "0")
+    A = _operator(pkg, S)
+    with pytest.raises(pkg.FDFDError) as ei:
+        A.matvec(x, precision="c64")
+    assert ei.value.code == FDFD_ERR_TIMEOUT
+    A.close()
+    monkeypatch.delenv("FDFD_WAIT_LIMIT_CLOCKS")
+    B = _operator(pkg, S)
+    y = B.matvec(x, precision="c64")
+    ref = S.A @ x
+    assert np.linalg.norm(y - ref) / np.linalg.norm(ref) < 1e-5
+    B.close()
