@@ -66,18 +66,38 @@ __device__ __forceinline__ double2 mul_c(double2 c, double2 d) {
 // predicated instructions, which take the pipe too: 131 µs against 84 for
 // k_h_from_e at 128×128×64.
 
+// The thread's cell p of the plane and its planes [k0, k1), and whether it
+// stores (a lane that does not repeats a cell).  zs > 1 (planes of at most 16
+// cells): one warp per block, which takes zs z-chunks side by side.  k0 < 0:
+// the whole warp lies past the plane.
+__device__ __forceinline__ bool plane_thread(int plane, int nz, int kc, int zs, int &p, int &k0, int &k1) {
+  bool act;
+  if (zs > 1) {
+    int sub = threadIdx.x / plane;
+    p = threadIdx.x - sub * plane;
+    act = sub < zs && (blockIdx.y * zs + sub) * kc < nz;
+    k0 = (blockIdx.y * zs + (act ? sub : 0)) * kc;
+  } else {
+    const int p0 = blockIdx.x * FB + threadIdx.x;
+    act = p0 < plane;
+    p = act ? p0 : plane - 1;
+    k0 = (p0 & ~31) < plane ? (int)blockIdx.y * kc : -1;
+  }
+  k1 = min(k0 + kc, nz);
+  return act;
+}
+
 // REALW: ω is real, so i/ω = i·s and s is folded into the curl coefficients.
 // BL: some axis is periodic.
 template <bool REALW, bool BL>
 __global__ void __launch_bounds__(FB) k_h_from_e(OpArgs<double> a, Extra<double> ex, const double2 *__restrict__ e,
                                                  const double2 *__restrict__ jm, double2 *__restrict__ hout,
-                                                 double2 iow, int kc) {
+                                                 double2 iow, int kc, int zs) {
   const int plane = a.N[0] * a.N[1];
-  const int p0 = blockIdx.x * FB + threadIdx.x;
-  const bool act = p0 < plane;
-  const int p = act ? p0 : plane - 1;  // idle lanes of the last warp repeat a cell (and store nothing)
+  int p, k0, k1;
+  const bool act = plane_thread(plane, a.N[2], kc, zs, p, k0, k1);
+  if (k0 < 0) return;
   const int i = p % a.N[0], j = p / a.N[0];
-  const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, a.N[2]);
   const bool blx = BL && a.bloch[0], bly = BL && a.bloch[1], blz = BL && a.bloch[2];
   const bool pi = !blx && i == 0, pj = !bly && j == 0;
   const double sc = REALW ? iow.y : 1.0;
@@ -198,13 +218,12 @@ struct MeanW {
 
 template <bool HF, bool BL>
 __global__ void __launch_bounds__(FB) k_corner_mean(OpArgs<double> a, Extra<double> ex, MeanW wt,
-                                                    const double2 *__restrict__ in, double2 *__restrict__ out, int kc) {
+                                                    const double2 *__restrict__ in, double2 *__restrict__ out, int kc, int zs) {
   const int plane = a.N[0] * a.N[1];
-  const int p0 = blockIdx.x * FB + threadIdx.x;
-  const bool act = p0 < plane;
-  const int p = act ? p0 : plane - 1;
+  int p, k0, k1;
+  const bool act = plane_thread(plane, a.N[2], kc, zs, p, k0, k1);
+  if (k0 < 0) return;
   const int i = p % a.N[0], j = p / a.N[0];
-  const int k0 = blockIdx.y * kc, k1 = min(k0 + kc, a.N[2]);
   const double2 ox = wt.own[0][i], nx = wt.nb[0][i], oy = wt.own[1][j], ny = wt.nb[1][j];
   const bool xr = __all_sync(0xffffffffu, ox.y == 0.0 && nx.y == 0.0);
   const bool yr = __all_sync(0xffffffffu, oy.y == 0.0 && ny.y == 0.0);
@@ -364,16 +383,27 @@ int d2h_real(fdfd_handle *h, const double *src, double *dst, int mask) {
                     "D2H values");
 }
 
-// Grid of a z-marching plane kernel: blocks over the flattened plane, and
-// chunks of kc planes short enough to give the chip about eight blocks per
-// SM (a chunk re-reads one plane, so at most 16 planes gain nothing more).
-static dim3 plane_grid(const fdfd_handle *h, int *kc) {
-  const long long bx = ((long long)h->N[0] * h->N[1] + FB - 1) / FB;
-  const long long k = bx * h->N[2] / (152 * 8);
-  *kc = (int)std::max(1ll, std::min(16ll, k));
+// Launch shape of a z-marching plane kernel: blocks over the flattened plane,
+// and chunks of kc planes short enough to give the chip about 64 warps per SM
+// (a chunk re-reads one plane, so at most 16 planes gain nothing more).  Where
+// a plane has fewer than FB cells a block is its warps, and at most 16
+// cells share their warp with the next chunks: 2×2×4096 in blocks of FB
+// threads, with 4 of them at work, took 61 µs for h_from_e, now 6.5.
+struct PlaneShape {
+  dim3 grid;
+  int threads, kc, zs;
+};
+static PlaneShape plane_shape(const fdfd_handle *h) {
+  const long long plane = (long long)h->N[0] * h->N[1], warps = (plane + 31) / 32;
+  PlaneShape s;
+  s.threads = (int)std::min<long long>(FB, 32 * warps);
+  s.zs = plane <= 16 ? (int)(32 / plane) : 1;
+  s.kc = (int)std::max(1ll, std::min(16ll, warps * h->N[2] / (152 * 64 * s.zs)));
   // blockIdx.y is limited to 65535 chunks
-  *kc = std::max(*kc, (h->N[2] + 65534) / 65535);
-  return dim3((unsigned)bx, (unsigned)((h->N[2] + *kc - 1) / *kc), 1);
+  s.kc = std::max(s.kc, (h->N[2] + 65534) / 65535);
+  const int chunks = (h->N[2] + s.kc - 1) / s.kc;
+  s.grid = dim3((unsigned)((plane + FB - 1) / FB), (unsigned)((chunks + s.zs - 1) / s.zs), 1);
+  return s;
 }
 
 int h_from_e_dev_impl(fdfd_handle *h, const double2 *e, const double2 *jm, double2 *hout) {
@@ -383,12 +413,11 @@ int h_from_e_dev_impl(fdfd_handle *h, const double2 *e, const double2 *jm, doubl
   const double wr = h->omega[0], wi = h->omega[1], d = wr * wr + wi * wi;
   if (!(d > 0.0)) return set_error(h, FDFD_ERR_ARG, "h_from_e needs ω ≠ 0");
   const double2 iow = make_double2(wi / d, wr / d);
-  int kc;
-  const dim3 grid = plane_grid(h, &kc);
+  const PlaneShape ps = plane_shape(h);
   const bool bl = h->bloch[0] || h->bloch[1] || h->bloch[2];
   const auto kern = iow.x == 0.0 ? (bl ? k_h_from_e<true, true> : k_h_from_e<true, false>)
                                  : (bl ? k_h_from_e<false, true> : k_h_from_e<false, false>);
-  kern<<<grid, FB, 0, h->stream>>>(a, ex, e, jm, hout, iow, kc);
+  kern<<<ps.grid, ps.threads, 0, h->stream>>>(a, ex, e, jm, hout, iow, ps.kc, ps.zs);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "k_h_from_e");
 }
@@ -416,12 +445,11 @@ int corner_mean_dev_impl(fdfd_handle *h, int hfield, const double2 *in, double2 
     wt.own[w] = hfield ? h->coef64 + 6 * h->coef_stride + h->coef_off[w] : a.wp[w];
     wt.nb[w] = hfield ? h->coef64 + 7 * h->coef_stride + h->coef_off[w] : a.wm[w];
   }
-  int kc;
-  const dim3 grid = plane_grid(h, &kc);
+  const PlaneShape ps = plane_shape(h);
   const bool bl = h->bloch[0] || h->bloch[1] || h->bloch[2];
   const auto kern = hfield ? (bl ? k_corner_mean<true, true> : k_corner_mean<true, false>)
                            : (bl ? k_corner_mean<false, true> : k_corner_mean<false, false>);
-  kern<<<grid, FB, 0, h->stream>>>(a, ex, wt, in, out, kc);
+  kern<<<ps.grid, ps.threads, 0, h->stream>>>(a, ex, wt, in, out, ps.kc, ps.zs);
   h->launches++;
   return cuda_check(h, cudaGetLastError(), "k_corner_mean");
 }

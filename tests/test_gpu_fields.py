@@ -116,3 +116,29 @@ def test_field_kernels_plane_edges(pkg, oracle, bloch, N):
                          (A.corner_mean(v, "E"), Mce @ v), (A.corner_mean(v, "H"), Mcm @ v)):
             assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
         A.close()
+
+
+@pytest.mark.parametrize("N,bloch", [((1, 1, 37), (True, True, False)), ((2, 2, 19), (False, False, True)),
+                                     ((3, 5, 7), (False, True, False)), ((16, 1, 5), (False, True, True)),
+                                     ((4, 4, 40), (False, False, False)), ((17, 1, 6), (True, True, False))])
+def test_field_kernels_thin_planes(pkg, oracle, N, bloch):
+    """h_from_e and the corner means on planes of 1, 4, 15, 16 and 17 cells,
+    where several z-chunks share a warp (and where they just do not), with
+    the last warp part full; the bound is that of the other tests here."""
+    O = oracle
+    rng = np.random.default_rng(43)
+    lp = tuple(np.concatenate([[0.0], np.cumsum(rng.uniform(0.6, 1.4, n))]) for n in N)
+    g = O.Grid(lp, bloch)
+    kb = tuple(0.17 if b else 0.0 for b in bloch)
+    npml = tuple(0 if bloch[w] or N[w] < 8 else 3 for w in range(3))
+    om = 2 * np.pi / 6.5
+    sdl_e, sdl_m = O.stretched_dl(g, om, (npml, npml))
+    Ce, _ = O.create_curls(g, sdl_e, sdl_m, kb)
+    Mce, Mcm = O.create_Mcs(g, sdl_e, sdl_m, kb)
+    A = pkg.FDFDOperator(g.N, om, sdl_e, sdl_m, bloch, [np.exp(-1j * kb[w] * g.L[w]) for w in range(3)])
+    v = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    jm = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    for got, ref in ((A.h_from_e(v, jm), O.h_from_e(v, om, Ce, jm)), (A.corner_mean(v, "E"), Mce @ v),
+                     (A.corner_mean(v, "H"), Mcm @ v)):
+        assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+    A.close()
