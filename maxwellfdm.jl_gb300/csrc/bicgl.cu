@@ -242,32 +242,27 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
   R ar[NV], ai[NV];
 #pragma unroll
   for (int q = 0; q < NV; ++q) ar[q] = ai[q] = R(0);
-  auto one = [&](const C (&v)[L + 1]) {
+  // adds the products of one element (complex128), or of a pair of elements
+  // (complex64, a zero one for an odd tail): a pair's products are summed
+  // first, so that the plain FP32 chains have one term per pair
+  auto add = [&](int q, const C &a, const C &b, const C &a2, const C &b2, bool real) {
+    if constexpr (sizeof(R) == 8) {
+      ar[q] = fma(a.y, b.y, fma(a.x, b.x, ar[q]));
+      if (!real) ai[q] = fma(-a.y, b.x, fma(a.x, b.y, ai[q]));
+    } else {
+      const C d = cadd(cdotc(a, b), cdotc(a2, b2));
+      ar[q] += d.x;
+      ai[q] += d.y;
+    }
+  };
+  auto two = [&](const C (&v)[L + 1], const C (&w)[L + 1]) {
     int q = 0;
 #pragma unroll
     for (int j = 1; j <= L; ++j)
 #pragma unroll
-      for (int i = 1; i <= j; ++i, ++q) {
-        if constexpr (sizeof(R) == 8) {
-          ar[q] = fma(v[i].y, v[j].y, fma(v[i].x, v[j].x, ar[q]));
-          if (i < j) ai[q] = fma(-v[i].y, v[j].x, fma(v[i].x, v[j].y, ai[q]));  // (r_i, r_i) is real
-        } else {
-          const C d = cdotc(v[i], v[j]);
-          ar[q] += d.x;
-          ai[q] += d.y;
-        }
-      }
+      for (int i = 1; i <= j; ++i, ++q) add(q, v[i], v[j], w[i], w[j], i == j);  // (r_i, r_i) is real
 #pragma unroll
-    for (int i = 1; i <= L; ++i, ++q) {
-      if constexpr (sizeof(R) == 8) {
-        ar[q] = fma(v[i].y, v[0].y, fma(v[i].x, v[0].x, ar[q]));
-        ai[q] = fma(-v[i].y, v[0].x, fma(v[i].x, v[0].y, ai[q]));
-      } else {
-        const C d = cdotc(v[i], v[0]);
-        ar[q] += d.x;
-        ai[q] += d.y;
-      }
-    }
+    for (int i = 1; i <= L; ++i, ++q) add(q, v[i], v[0], w[i], w[0], false);
   };
   visit<R>(
       n,
@@ -288,8 +283,7 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
         C none = czero<C>();
         replay<L, false>(va, ua, none, hist);
         replay<L, false>(vb, ub, none, hist);
-        one(va);
-        one(vb);
+        two(va, vb);
       },
       [&](long long e) {
         C v[L + 1], ue[L], xe = czero<C>();
@@ -307,7 +301,8 @@ __global__ void __launch_bounds__(VB, 2) k_bl_gram(VSet<typename CT<R>::C> r, VS
             u.v[i][e] = ue[i];
           }
         }
-        one(v);
+        const C nil[L + 1] = {};
+        two(v, nil);
       });
   if (KEEP && blockIdx.x == 0 && threadIdx.x == 0) sc->bl_steps = 0;  // x holds this cycle's steps
   if constexpr (sizeof(R) == 4) {

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(HG<R, RW>::NT, 2)
       eo[r][c] = zero;
     }
   const C cmx = xt[lane], cex = xt[TX + 1 + lane];
-  ShortAcc<R> a0r, a0i, a1r;
+  RowAcc<R, RW> a0r, a0i, a1r;
 
   int sm1 = 0, s0 = 1;  // slots of planes q−1 and q
   for (int q = k0; q <= k1; ++q) {
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(HG<R, RW>::NT, 2)
         if (EPI == EPI_RESID) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) v[c] = csub(aux[r][c], v[c]);
-          a0r.add(v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
+          a0r.add(r, v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
                   v[2].y * v[2].y);
         } else if (EPI == EPI_DOT_AUX || EPI == EPI_DOT_TS || EPI == EPI_DOT_SHD) {
           C d[3];
@@ -277,10 +277,10 @@ __global__ void __launch_bounds__(HG<R, RW>::NT, 2)
             else if (EPI == EPI_DOT_TS) d[c] = cdotc(v[c], hp[r][c]);
             else d[c] = cdotc(shadow<R>(3 * cell[r] + c), v[c]);
           }
-          a0r.add(d[0].x + d[1].x + d[2].x);
-          a0i.add(d[0].y + d[1].y + d[2].y);
+          a0r.add(r, d[0].x + d[1].x + d[2].x);
+          a0i.add(r, d[0].y + d[1].y + d[2].y);
           if (EPI == EPI_DOT_TS)
-            a1r.add(v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
+            a1r.add(r, v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
                     v[2].y * v[2].y);
         }
         C *yo = y + 3 * cell[r];
@@ -288,6 +288,9 @@ __global__ void __launch_bounds__(HG<R, RW>::NT, 2)
         yo[1] = v[1];
         yo[2] = v[2];
       }
+      a0r.end_plane();
+      a0i.end_plane();
+      a1r.end_plane();
 #pragma unroll
       for (int r = 0; r < RW; ++r) cell[r] += plane;
     }
@@ -358,7 +361,7 @@ __global__ void __launch_bounds__(HG<R, RW>::NT, 2)
   cp_async_wait<0>();
   if (EPI != EPI_STORE) {
     __syncthreads();
-    sum_finalise<G::NT>(a0r, a0i, a1r, red, fin, sc);
+    sum_finalise<G::NT>(a0r.acc, a0i.acc, a1r.acc, red, fin, sc);
   }
 }
 

@@ -429,8 +429,8 @@ template <> struct Acc<float> {
   }
 };
 
-// Short per-thread sum (the operator kernel's epilogue adds at most
-// 3 × z-chunk terms per thread): plain FP32 for float kernels.
+// Short per-thread sum (an operator kernel's epilogue adds at most one term
+// per cell of a thread's z-chunk): plain FP32 for float kernels.
 template <typename R> struct ShortAcc;
 template <> struct ShortAcc<double> {
   double s = 0.0;
@@ -441,6 +441,26 @@ template <> struct ShortAcc<float> {
   float s = 0.f;
   __device__ __forceinline__ void add(float v) { s += v; }
   __device__ __forceinline__ DF df() const { return DF{s, 0.f}; }
+};
+
+// The same where a thread owns RW rows: a plane's terms are summed first, so
+// that the chain has one term per plane as with one row per thread (added row
+// by row, its FP32 error was 1.3 to 1.9 times as large: random data, 4 to 32
+// planes).
+template <typename R, int RW>
+struct RowAcc {
+  ShortAcc<R> acc;
+  R p = R(0);
+  __device__ __forceinline__ void add(int r, R v) {
+    if constexpr (RW == 1) acc.add(v);
+    else p = r == 0 ? v : p + v;
+  }
+  __device__ __forceinline__ void end_plane() {
+    if constexpr (RW > 1) {
+      acc.add(p);
+      p = R(0);
+    }
+  }
 };
 
 // Grid sums a0 = a0r + i·a0i and a1 (real) of a reducing kernel, then the

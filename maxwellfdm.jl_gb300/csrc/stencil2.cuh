@@ -108,9 +108,9 @@ __device__ __forceinline__ typename CT<R>::C ev2(const unsigned char *sm, int s,
   return reinterpret_cast<const typename CT<R>::C *>(sm + s * G::SLOT)[((jj + 1) * G::XW + ii + G::XOFF) * 3 + c];
 }
 
-template <typename R>
+template <typename R, int RW>
 struct Accs2 {
-  ShortAcc<R> r0, i0, r1;
+  RowAcc<R, RW> r0, i0, r1;
 };
 
 template <typename R, bool BL>
@@ -327,7 +327,7 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
     return eoff_at<R, CPA>(a, p, i0 + ii, j0 + jj, gk);
   };
 
-  Accs2<R> acc;
+  Accs2<R, RW> acc;
   int kstop = k0;
   bool run = true;
   const int plane = a.N[0] * a.N[1];  // 3·Ncell < 2³¹ (checked at launch)
@@ -727,28 +727,28 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
             yx = csub(aux[r][0], yx);
             yy = csub(aux[r][1], yy);
             yz = csub(aux[r][2], yz);
-            acc.r0.add(yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
+            acc.r0.add(r, yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
           } else if (EPI == EPI_DOT_AUX) {
             const C q0 = cdotc(aux[r][0], yx), q1 = cdotc(aux[r][1], yy), q2 = cdotc(aux[r][2], yz);
-            acc.r0.add(q0.x + q1.x + q2.x);
-            acc.i0.add(q0.y + q1.y + q2.y);
+            acc.r0.add(r, q0.x + q1.x + q2.x);
+            acc.i0.add(r, q0.y + q1.y + q2.y);
           } else if (EPI == EPI_DOT_TS) {
             // (t, s) with the true input s (its pinned entries are not in eo)
             const C sx = t0, sy = t1, sz = t2;
             const C q0 = cdotc(yx, sx), q1 = cdotc(yy, sy), q2 = cdotc(yz, sz);
-            acc.r0.add(q0.x + q1.x + q2.x);
-            acc.i0.add(q0.y + q1.y + q2.y);
-            acc.r1.add(yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
+            acc.r0.add(r, q0.x + q1.x + q2.x);
+            acc.i0.add(r, q0.y + q1.y + q2.y);
+            acc.r1.add(r, yx.x * yx.x + yx.y * yx.y + yy.x * yy.x + yy.y * yy.y + yz.x * yz.x + yz.y * yz.y);
           } else if (EPI == EPI_DOT_SHD) {
             const C s0 = shadow<R>(3ll * ce), s1 = shadow<R>(3ll * ce + 1), s2 = shadow<R>(3ll * ce + 2);
             if constexpr (sizeof(R) == 8) {  // straight into the sums: 12 FP64 instructions
-              dot_into(acc.r0.s, acc.i0.s, s0, yx);
-              dot_into(acc.r0.s, acc.i0.s, s1, yy);
-              dot_into(acc.r0.s, acc.i0.s, s2, yz);
+              dot_into(acc.r0.acc.s, acc.i0.acc.s, s0, yx);
+              dot_into(acc.r0.acc.s, acc.i0.acc.s, s1, yy);
+              dot_into(acc.r0.acc.s, acc.i0.acc.s, s2, yz);
             } else {
               const C q = pdot3(s0, yx, s1, yy, s2, yz);
-              acc.r0.add(q.x);
-              acc.i0.add(q.y);
+              acc.r0.add(r, q.x);
+              acc.i0.add(r, q.y);
             }
           }
           C *yo = y + 3 * ce;
@@ -757,6 +757,9 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
           yo[2] = yz;
         }
       }
+      acc.r0.end_plane();
+      acc.i0.end_plane();
+      acc.r1.end_plane();
       // ---- advance to plane k+1
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
@@ -797,7 +800,7 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
     }
   }
   __syncthreads();
-  if (EPI != EPI_STORE) sum_finalise<G::NT>(acc.r0, acc.i0, acc.r1, red, fin, sc);
+  if (EPI != EPI_STORE) sum_finalise<G::NT>(acc.r0.acc, acc.i0.acc, acc.r1.acc, red, fin, sc);
 }
 
 template <typename R, int EPI, int RW, int NS, int MB, bool EDR>

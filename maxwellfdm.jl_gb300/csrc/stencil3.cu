@@ -307,7 +307,7 @@ __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<f
     return n < G::NB ? its[q % 3 * (G::NB * 32) + i] : ex.corners[l.x + i];
   };
   auto rounds = [&](int t) { return OFF ? (zl[t].y + 31) >> 5 : 0; };
-  ShortAcc<R> acr, aci, ac1;
+  RowAcc<R, RW> acr, aci, ac1;
   int kstop = k0;
   bool run = true;
   if (helper) {
@@ -682,29 +682,32 @@ __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<f
         if (EPI == EPI_RESID) {
 #pragma unroll
           for (int c = 0; c < 3; ++c) v[c] = csub(aux[r][c], v[c]);
-          acr.add(v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
+          acr.add(r, v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
                   v[2].y * v[2].y);
         } else if (EPI == EPI_DOT_AUX || EPI == EPI_DOT_TS) {
           // (r̂, y), or (t, s) with the true input s
           const C q0 = EPI == EPI_DOT_AUX ? cdotc(aux[r][0], v[0]) : cdotc(v[0], tv[r][0]);
           const C q1 = EPI == EPI_DOT_AUX ? cdotc(aux[r][1], v[1]) : cdotc(v[1], tv[r][1]);
           const C q2 = EPI == EPI_DOT_AUX ? cdotc(aux[r][2], v[2]) : cdotc(v[2], tv[r][2]);
-          acr.add(q0.x + q1.x + q2.x);
-          aci.add(q0.y + q1.y + q2.y);
+          acr.add(r, q0.x + q1.x + q2.x);
+          aci.add(r, q0.y + q1.y + q2.y);
           if (EPI == EPI_DOT_TS)
-            ac1.add(v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
+            ac1.add(r, v[0].x * v[0].x + v[0].y * v[0].y + v[1].x * v[1].x + v[1].y * v[1].y + v[2].x * v[2].x +
                     v[2].y * v[2].y);
         } else if (EPI == EPI_DOT_SHD) {
           const int ce = 3 * (plane * k + off[r]);
           const C q = pdot3(shadow<R>(ce), v[0], shadow<R>(ce + 1), v[1], shadow<R>(ce + 2), v[2]);
-          acr.add(q.x);
-          aci.add(q.y);
+          acr.add(r, q.x);
+          aci.add(r, q.y);
         }
         C *yo = yp + 3 * off[r];
         yo[0] = v[0];
         yo[1] = v[1];
         yo[2] = v[2];
       }
+      acr.end_plane();
+      aci.end_plane();
+      ac1.end_plane();
       // ---- advance to plane k+1
 #pragma unroll
       for (int r = 0; r < RW; ++r) {
@@ -732,7 +735,7 @@ __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<f
       mbar_wait(smem_u32(&bars[(q - kfirst) % NS]), ((q - kfirst) / NS) & 1);
   }
   __syncthreads();
-  if (EPI != EPI_STORE) sum_finalise<G::NT>(acr, aci, ac1, red, fin, sc);
+  if (EPI != EPI_STORE) sum_finalise<G::NT>(acr.acc, aci.acc, ac1.acc, red, fin, sc);
 }
 
 template <int EPI, bool OFF>
