@@ -222,6 +222,11 @@ static int ensure_eps_buffers(fdfd_handle *h, bool off) {
 int finish_eps(fdfd_handle *h, bool refresh, const unsigned *corners = nullptr) {
   const long long n = 3 * h->ncell;
   int rc = FDFD_OK;
+  // captured solver graphs hold whether the operator has off-diagonal terms
+  if (h->eps_off != (h->has_off ? 1 : 0)) {
+    drop_graphs(h);
+    h->eps_off = h->has_off ? 1 : 0;
+  }
   if (refresh) {
     k_to_f32<<<152 * 4, 256, 0, h->stream>>>(h->eps32, h->eps64, n);
     if ((rc = cuda_check(h, cudaGetLastError(), "k_to_f32"))) return rc;

@@ -190,6 +190,7 @@ struct fdfd_handle {
   // Measured at 320³ with 400 spheres: 5: 392 µs, 4: 415 µs, 3: 424 µs; 2 and
   // the first kernel above 490 µs.
   int op_variant = 4;
+  int eps_off = -1;                   // has_off at the last change of ε
   int tuned_off = -1;                 // has_off at the last tuning (−1: not tuned yet)
   std::string err;
 };

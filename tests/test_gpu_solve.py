@@ -247,3 +247,24 @@ def test_breakdown_at_the_end_of_a_cycle(pkg, precision):
     assert abs(st["relres"] - np.sqrt(2.0)) <= 1e-12
     assert np.array_equal(ei.value.x, b)
     A.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_graphs_follow_the_off_diagonal_tensor(pkg, oracle, sysx, monkeypatch, precision):
+    """Vacuum, a smoothed sphere and vacuum again on one handle with a forced
+    z-chunk (no tuning in between): each solve's captured batch has the
+    operator of its own ε, so it takes the steps of a fresh handle's solve."""
+    monkeypatch.setenv("FDFD_KCHUNK", "4")
+    S, b, xd = sysx
+    ones = np.ones(S.grid.N + (3,))
+    A = pkg.FDFDOperator(S.grid.N, S.omega, S.sdl_e, S.sdl_m)
+    for eps in ((ones, None), (S.eps_diag, S.eps_off), (ones, None)):
+        A.set_eps(*eps)
+        x, st = A.solve(b, tol=1e-8, precision=precision, maxit=5000)
+        B = pkg.FDFDOperator(S.grid.N, S.omega, S.sdl_e, S.sdl_m)
+        B.set_eps(*eps)
+        y, sb = B.solve(b, tol=1e-8, precision=precision, maxit=5000)
+        assert st[0]["iterations"] == sb[0]["iterations"]
+        assert np.array_equal(x, y)
+        B.close()
+    A.close()
