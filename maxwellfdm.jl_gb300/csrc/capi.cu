@@ -196,23 +196,27 @@ __global__ void k_to_f32(float *dst, const double *src, long long n) {
     dst[i] = (float)src[i];
 }
 
-static int ensure_eps_buffers(fdfd_handle *h, bool off) {
-  const size_t n = 3 * (size_t)h->ncell;
-  if (!h->eps64) {
-    if (dev_malloc(&h->eps64, n * sizeof(double)) != cudaSuccess ||
-        dev_malloc(&h->eps32, n * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(eps) failed");
-    }
-  }
-  if (off && !h->eoff64) {
-    if (dev_malloc(&h->eoff64, n * sizeof(double)) != cudaSuccess ||
-        dev_malloc(&h->eoff32, n * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(eps off-diagonal) failed");
-    }
+// Allocate *p once.  Every buffer is tested by itself: after a failure the
+// ones that were had stay, and the next call allocates only what is missing.
+template <typename T>
+static int ensure_buf(fdfd_handle *h, T **p, size_t count, const char *what) {
+  if (*p) return FDFD_OK;
+  if (dev_malloc(p, count * sizeof(T)) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+    return set_error(h, FDFD_ERR_NOMEM, std::string("cudaMalloc(") + what + ") failed");
   }
   return FDFD_OK;
+}
+
+int ensure_eps_buffers(fdfd_handle *h, bool off) {
+  const size_t n = 3 * (size_t)h->ncell;
+  int rc;
+  if ((rc = ensure_buf(h, &h->eps32, n, "eps"))) return rc;
+  if ((rc = ensure_buf(h, &h->eps64, n, "eps"))) return rc;
+  if (!off) return FDFD_OK;
+  if ((rc = ensure_buf(h, &h->eoff32, n, "eps off-diagonal"))) return rc;
+  return ensure_buf(h, &h->eoff64, n, "eps off-diagonal");
 }
 
 // After new ε data: refresh the FP32 copies from the FP64 masters and rebuild
@@ -257,8 +261,10 @@ int upload_eps(fdfd_handle *h, const double *eps_diag_aos, const double *eps_off
   bool off = false;
   if (eps_off_aos)
     for (long long i = 0; i < 3 * nc && !off; ++i) off = eps_off_aos[i] != 0.0;
+  // every allocation first: one that fails leaves the handle's ε as it was
   int rc = ensure_eps_buffers(h, off);
   if (rc) return rc;
+  if (off && (rc = ensure_oflags(h))) return rc;
   std::vector<double> soa(3 * (size_t)nc);
   for (long long cell = 0; cell < nc; ++cell)
     for (int c = 0; c < 3; ++c) soa[c * nc + cell] = eps_diag_aos[c + 3 * cell];
@@ -279,21 +285,12 @@ int upload_eps(fdfd_handle *h, const double *eps_diag_aos, const double *eps_off
 
 static int ensure_scratch(fdfd_handle *h, bool c64) {
   const size_t n = 3 * (size_t)h->ncell;
-  if (!h->vx64) {
-    if (dev_malloc(&h->vx64, n * sizeof(double2)) != cudaSuccess ||
-        dev_malloc(&h->vy64, n * sizeof(double2)) != cudaSuccess) {
-      cudaGetLastError();
-      return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(scratch) failed");
-    }
-  }
-  if (c64 && !h->vx32) {
-    if (dev_malloc(&h->vx32, n * sizeof(float2)) != cudaSuccess ||
-        dev_malloc(&h->vy32, n * sizeof(float2)) != cudaSuccess) {
-      cudaGetLastError();
-      return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(scratch c64) failed");
-    }
-  }
-  return FDFD_OK;
+  int rc;
+  if ((rc = ensure_buf(h, &h->vx64, n, "scratch"))) return rc;
+  if ((rc = ensure_buf(h, &h->vy64, n, "scratch"))) return rc;
+  if (!c64) return FDFD_OK;
+  if ((rc = ensure_buf(h, &h->vx32, n, "scratch c64"))) return rc;
+  return ensure_buf(h, &h->vy32, n, "scratch c64");
 }
 
 static bool transpose_ok(const fdfd_handle *h) {

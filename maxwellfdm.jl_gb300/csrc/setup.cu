@@ -33,6 +33,7 @@ namespace fdfd {
 
 int finish_eps(fdfd_handle *h, bool refresh, const unsigned *corners);
 int ensure_oflags(fdfd_handle *h);
+int ensure_eps_buffers(fdfd_handle *h, bool off);
 
 struct DevObj {
   int kind;
@@ -598,13 +599,7 @@ int smooth_objects_impl(fdfd_handle *h, const double *const lprim[3], const fdfd
       return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(smask) failed");
     }
   }
-  if (!h->eoff64) {
-    if (dev_malloc(&h->eoff64, 3 * nc * sizeof(double)) != cudaSuccess ||
-        dev_malloc(&h->eoff32, 3 * nc * sizeof(float)) != cudaSuccess) {
-      cudaGetLastError();
-      return set_error(h, FDFD_ERR_NOMEM, "cudaMalloc(eps off-diagonal) failed");
-    }
-  }
+  if ((rc = ensure_eps_buffers(h, true))) return rc;
   if ((rc = ensure_oflags(h))) return rc;
 
   char *dup = buf.get<char>(up_bytes);

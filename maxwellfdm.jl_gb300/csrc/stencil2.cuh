@@ -253,7 +253,7 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
           // periodic y: the strip past the last row forms the corner terms of
           // row N_y (corner row 0) for the last strip's outputs
           if (by_ && tr * RW == a.N[1]) --tr;
-          const bool in = a.eoff != nullptr && q >= 0 && q < a.N[2] && tr < tiles_yr;
+          const bool in = ex.oflag_w != nullptr && q >= 0 && q < a.N[2] && tr < tiles_yr;
           f[s] = in ? ex.oflag_w[(bx + (long long)tiles_x * tr) * a.N[2] + q] : 0;
         }
 #pragma unroll

@@ -145,3 +145,26 @@ def test_bounded_wait_of_the_third_kernel(pkg, oracle, monkeypatch, spheres):
     ref = S.A @ x
     assert np.linalg.norm(y - ref) / np.linalg.norm(ref) < 1e-5
     B.close()
+
+
+def test_failed_material_update_leaves_the_handle_whole(pkg, oracle, monkeypatch):
+    """An allocation that fails half way through the buffers of the
+    off-diagonal tensor: FDFD_ERR_NOMEM, the operator of the old ε still
+    applies, and the same update succeeds once there is memory."""
+    S = _system(oracle, (24, 24, 24))
+    A = pkg.FDFDOperator(S.grid.N, S.omega, S.sdl_e, S.sdl_m)
+    rng = np.random.default_rng(7)
+    x = rng.standard_normal(A.n) + 1j * rng.standard_normal(A.n)
+    y0 = [A.matvec(x, p) for p in ("c128", "c64")]
+    monkeypatch.setenv("FDFD_FAIL_ALLOC_BYTES", str(24 * S.grid.ncell))  # the FP64 tensor, not its FP32 copy
+    with pytest.raises(pkg.FDFDError) as ei:
+        A.set_eps(S.eps_diag, S.eps_off)
+    assert ei.value.code == FDFD_ERR_NOMEM
+    monkeypatch.delenv("FDFD_FAIL_ALLOC_BYTES")
+    for y, p in zip(y0, ("c128", "c64")):
+        assert np.array_equal(A.matvec(x, p), y)
+    A.set_eps(S.eps_diag, S.eps_off)
+    ref = S.A @ x
+    for p, tol in (("c128", 1e-12), ("c64", 1e-5)):
+        assert np.linalg.norm(A.matvec(x, p) - ref) <= tol * np.linalg.norm(ref)
+    A.close()
