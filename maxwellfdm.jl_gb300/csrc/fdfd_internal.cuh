@@ -140,7 +140,7 @@ struct fdfd_handle {
   double *eoff64 = nullptr;
   float *eoff32 = nullptr;
   uint8_t *oflag = nullptr;
-  uint8_t *oflag_rows[2] = {nullptr, nullptr};  // the same per x tile, group of 1 / 2 rows and plane
+  uint8_t *oflag_rows[2] = {nullptr, nullptr};  // the same per x tile, group of 1 / 2 rows and plane (strips)
   bool has_off = false;
   // the non-zero off-diagonal corners per (32×16 tile, plane), for complex64 on PEC walls (stencil3.cu)
   int2 *corner_list = nullptr;

@@ -25,9 +25,10 @@
 
 namespace fdfd {
 
-// The two kernels below are bound by the FP64 pipe (measured 0.53·10¹² lane
-// FMAs/s on the chip: a warp's FP64 instruction holds its scheduler's pipe
-// for 64 cycles however few lanes are active), so they are laid out to issue
+// The two kernels below are bound by the FP64 pipe (a warp's FP64
+// instruction holds its scheduler's pipe for 64 cycles however few lanes are
+// active: 0.63·10¹² lane FMAs/s on the chip at its top clock, 0.53 to 0.63
+// measured), so they are laid out to issue
 // few FP64 instructions:
 //   * threads run over the flattened cells of an x-y plane, so ragged Nx
 //     leaves no idle lanes, and march along z keeping what the next plane

@@ -73,17 +73,6 @@ template <bool RC>
 __device__ __forceinline__ double2 wsum(double2 a, double2 u, double2 b, double2 v) {
   return cadd(mulc<RC>(a, u), mulc<RC>(b, v));
 }
-// u·s + v·t for real s, t
-__device__ __forceinline__ float2 pmix(float2 u, float s, float2 v, float t) {
-  return __ffma2_rn(u, f2(s), __fmul2_rn(v, f2(t)));
-}
-__device__ __forceinline__ double2 pmix(double2 u, double s, double2 v, double t) {
-  return cadd(cscale(u, s), cscale(v, t));
-}
-// (u + v)·s for real s
-__device__ __forceinline__ float2 psums(float2 u, float2 v, float s) { return __fmul2_rn(__fadd2_rn(u, v), f2(s)); }
-__device__ __forceinline__ double2 psums(double2 u, double2 v, double s) { return cscale(cadd(u, v), s); }
-
 // A complex64 curl coefficient as csum takes it: its real part twice (the
 // operand of a paired multiply; 16 bytes, one shared-memory load).
 template <typename R> struct Coef;

@@ -12,8 +12,10 @@
 //     (cp.async.bulk.tensor.3d, one elected thread, mbarrier completion with
 //     bounded waits), two planes ahead of the plane being computed; the
 //     out-of-bounds zero fill of TMA realises the PEC ghost planes;
-//   * k_apply (general: Bloch phases, Aᵀ): a 3-slot ring filled by plain
-//     loads that apply the boundary rules element by element;
+//   * k_apply (Aᵀ, the allocation-free residual, and what neither k_apply_tma
+//     nor the second and third kernels of stencil2.cuh and stencil3.cu serve:
+//     COCG on periodic axes or odd Nx): a 3-slot ring filled by plain loads
+//     that apply the boundary rules element by element;
 //   * H = Cₑ E is computed once per plane for the tile plus its low halo and
 //     kept for two planes (H(k−1), H(k)) in shared memory;
 //   * y(k) = Cₘ H − ω² Pε E is formed from shared memory with the per-axis

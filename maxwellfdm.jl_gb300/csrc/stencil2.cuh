@@ -27,13 +27,14 @@
 //   * pinned DOFs (tangential E on the low PEC walls, kept in the vector
 //     but outside Cₑ) are zeroed as they are loaded, so no fix-up pass
 //     touches the ring; the diagonal ε term uses their true values;
-//   * off-diagonal ε (only where the 32×8 tile-plane flag is set): each
-//     thread forms the corner terms at its own corner from registers and
+//   * off-diagonal ε (only where the flag of the warp's strip and plane is
+//     set): each thread forms the corner terms at its own corner from registers and
 //     shuffles and averages the two corners around each output.
 // It serves the forward operator; where TMA cannot (odd Nx in complex64,
 // periodic axes) k_apply_cp runs the same march on a ring filled by cp.async;
 // the first TMA kernel (stencil.cu) keeps the S-weighted COCG epilogue and
-// the plain-load kernel Aᵀ.
+// the plain-load kernel Aᵀ.  complex64 on PEC walls may go to the third kernel
+// instead (stencil3.cu), as the autotuner measures.
 #pragma once
 
 #include <cuda.h>

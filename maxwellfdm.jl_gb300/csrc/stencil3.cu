@@ -120,7 +120,8 @@ __device__ __forceinline__ bool bar_any(bool p) {
   return r != 0;
 }
 
-// CPA: the ring is filled by cp.async (odd Nx), else by TMA.
+// CPA: the ring is filled by cp.async (odd Nx), else by TMA.  OFF: ε has
+// off-diagonal entries.
 template <int EPI, bool CPA, bool OFF>
 __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<float> &a, const Extra<float> &ex,
                                          const float2 *__restrict__ x, float2 *__restrict__ y,
@@ -164,7 +165,6 @@ __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<f
   const int i0 = bx * TX, j0 = by * TYT, kfirst = k0 - 1;
   const int gi = i0 + lane, jw = RW * w;
   const int cx = 6 * (i0 - G::XOFF), cy = j0 - 1;
-  // OFF: ε has off-diagonal entries
 
   if (!CPA && (smem_u32(sm) & 127u) != 0u) {  // TMA destinations (the declared alignment gives it)
     if (tid == 0) atomicExch(errflag, 2);
@@ -484,7 +484,6 @@ __device__ __forceinline__ void apply_v3(const CUtensorMap &tmap, const OpArgs<f
     // rounds of corners beyond the helpers': one per warp
     if (OFF && run) {
       C ax, ay;
-      
 #pragma unroll 1
       for (int n = G::NH + w; n < rounds(1); n += NW) z_terms(entry(k0, n), 1, k0, ax, ay);
     }
