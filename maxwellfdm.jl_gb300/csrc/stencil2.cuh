@@ -241,12 +241,13 @@ __device__ __forceinline__ void apply_v2(const CUtensorMap &tmap, const CUtensor
       // one flag per warp strip (RW rows): its outputs at plane q read a
       // non-zero off-diagonal ε
       unsigned char any = 0;
-      if constexpr (CPA) {
+      if (bx_ || by_ || bz_) {
         // eight lines of memory, all on their way before the first is used:
-        // 64×64×96 periodic in x and y 11.7 → 11.1 µs.  (Left out of the TMA
-        // form: with it layout 4 ties with the third kernel at 96³ in the
-        // tuner's 2 µs clock, which then keeps it, although it is the slower
-        // one where launches overlap — 13.1 µs against 11.6.)
+        // 64×64×96 periodic in x and y 11.7 → 11.2 to 11.6 µs.  (On PEC walls it is
+        // left out: with it layout 4 ties with the third kernel in the tuner's
+        // 2 µs clock, which then keeps it, although it is the slower one
+        // where launches overlap — 96³ 13.1 µs against 11.6, 81×122×47 up to
+        // 14.3 against 12.9.)
         unsigned char f[NW];
 #pragma unroll
         for (int s = 0; s < NW; ++s) {
